@@ -1,6 +1,6 @@
 // BF16 x BF16 mat-mul on the tensor cores for many activation rows: y[m][n] = act(w[n][k] x[m][k] + bias) + addend, F32 sums.
 //
-// Output tiles of 128 weight rows x NC activation rows (64, 128 or 256), walked by persistent CTAs, one per SM, the column blocks of a
+// Output tiles of 128 weight rows x NC activation rows (64 or 128), or of 256 x 256 by pairs of CTAs (further down), walked by persistent CTAs, one per SM, the column blocks of a
 // weight row block next to each other so that the weights cross HBM once.  Per tile a pipeline of K = 64 steps: one thread moves the
 // two operand boxes with TMA (128-byte swizzle; the hardware fills what lies outside either matrix with zeros), one thread issues four
 // M 128 x N NC x K 16 MMAs per step into one of two tensor-memory stages, four warps drain the other stage: lane = weight row, so a
@@ -22,7 +22,7 @@ constexpr int GB_ERR_WAIT = 4;
 template <int NC>
 struct GbCfg {
     static constexpr int A_BYTES = GB_ROWS * GB_K * 2, B_BYTES = NC * GB_K * 2, STAGE = A_BYTES + B_BYTES;
-    static constexpr int STAGES = NC == 256 ? 4 : NC == 128 ? 6 : 8;
+    static constexpr int STAGES = NC == 128 ? 6 : 8;
     static constexpr int SMEM = STAGES * STAGE + 1024;
     // kind::f16 instruction descriptor: F32 accumulator, BF16 x BF16, both operands K-major, N = NC, M = 128
     static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(GB_ROWS >> 4) << 24);
@@ -89,6 +89,58 @@ __device__ __forceinline__ void gb_tmem_ld32(uint32_t (&r)[32], uint32_t taddr) 
           "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr)
         : "memory");
+}
+
+// columns [c_begin, c_end) (multiples of 32) of this thread's tensor-memory lane: weight row `row` against activation rows col0 + c.
+// read() is called by the whole warp once all of them are in registers
+template <typename Read>
+__device__ __forceinline__ void gb_drain(const GbOut &o, uint32_t trow, int row, int col0, int c_begin, int c_end, Read read) {
+    const int lane = threadIdx.x & 31;
+    const bool row_ok = row < o.n;
+    const float bias = o.bias && row_ok ? o.bias[row] : 0.0f;
+#pragma unroll 1
+    for (int c0 = c_begin; c0 < c_end; c0 += 32) {
+        uint32_t v[32];
+        float ad[32];
+        gb_tmem_ld32(v, trow + (uint32_t)c0);
+        if (o.addend) {
+#pragma unroll
+            for (int c = 0; c < 32; c++) {
+                const int col = col0 + c0 + c;
+                ad[c] = row_ok && col < o.m ? o.addend[(int64_t)col * o.ld_addend + row] : 0.0f;
+            }
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (c0 + 32 >= c_end) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            read();
+        }
+        if (o.act == ACT_CLAMPED_GATE) {
+            const int odd = lane & 1;
+#pragma unroll
+            for (int c = 0; c < 32; c += 2) {
+                const float x0 = __uint_as_float(v[c]) + bias, x1 = __uint_as_float(v[c + 1]) + bias;
+                const float other = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
+                const float r = clamped_gate(odd ? other : x0, odd ? x1 : other, o.act_limit, o.act_alpha);
+                const int col = col0 + c0 + c + odd;
+                if (!row_ok || col >= o.m) continue;
+                if (o.y_type == B200_TYPE_F32) ((float *)o.y)[(int64_t)col * o.ldy + (row >> 1)] = r;
+                else ((__nv_bfloat16 *)o.y)[(int64_t)col * o.ldy + (row >> 1)] = __float2bfloat16_rn(r);
+            }
+            continue;
+        }
+        if (!row_ok) continue;
+#pragma unroll
+        for (int c = 0; c < 32; c++) {
+            const int col = col0 + c0 + c;
+            if (col >= o.m) break;
+            float r = dense_act(o.act, __uint_as_float(v[c]) + bias);
+            if (o.addend) r += ad[c];
+            if (o.y_type == B200_TYPE_F32) ((float *)o.y)[(int64_t)col * o.ldy + row] = r;
+            else ((__nv_bfloat16 *)o.y)[(int64_t)col * o.ldy + row] = __float2bfloat16_rn(r);
+        }
+    }
 }
 
 template <int NC>
@@ -189,52 +241,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
             if (!__all_sync(0xffffffffu, gb_bar_wait(gb_smem(&bars.tfull[ts]), (uint32_t)(j / GB_TSTAGES) & 1u, abort_flag))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = rb * GB_ROWS + 32 * q + lane, col0 = cb * NC;
-            const bool row_ok = row < o.n;
-            const float bias = o.bias && row_ok ? o.bias[row] : 0.0f;
             const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(ts * NC);
-#pragma unroll 1
-            for (int c0 = 0; c0 < NC; c0 += 32) {
-                uint32_t v[32];
-                float ad[32];
-                gb_tmem_ld32(v, trow + (uint32_t)c0);
-                if (o.addend) {
-#pragma unroll
-                    for (int c = 0; c < 32; c++) {
-                        const int col = col0 + c0 + c;
-                        ad[c] = row_ok && col < o.m ? o.addend[(int64_t)col * o.ld_addend + row] : 0.0f;
-                    }
-                }
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (c0 + 32 == NC) {
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) gb_bar_arrive(gb_smem(&bars.tempty[ts]));
-                }
-                if (o.act == ACT_CLAMPED_GATE) {
-                    const int odd = lane & 1;
-#pragma unroll
-                    for (int c = 0; c < 32; c += 2) {
-                        const float x0 = __uint_as_float(v[c]) + bias, x1 = __uint_as_float(v[c + 1]) + bias;
-                        const float other = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
-                        const float r = clamped_gate(odd ? other : x0, odd ? x1 : other, o.act_limit, o.act_alpha);
-                        const int col = col0 + c0 + c + odd;
-                        if (!row_ok || col >= o.m) continue;
-                        if (o.y_type == B200_TYPE_F32) ((float *)o.y)[(int64_t)col * o.ldy + (row >> 1)] = r;
-                        else ((__nv_bfloat16 *)o.y)[(int64_t)col * o.ldy + (row >> 1)] = __float2bfloat16_rn(r);
-                    }
-                    continue;
-                }
-                if (!row_ok) continue;
-#pragma unroll
-                for (int c = 0; c < 32; c++) {
-                    const int col = col0 + c0 + c;
-                    if (col >= o.m) break;
-                    float r = dense_act(o.act, __uint_as_float(v[c]) + bias);
-                    if (o.addend) r += ad[c];
-                    if (o.y_type == B200_TYPE_F32) ((float *)o.y)[(int64_t)col * o.ldy + row] = r;
-                    else ((__nv_bfloat16 *)o.y)[(int64_t)col * o.ldy + row] = __float2bfloat16_rn(r);
-                }
-            }
+gb_drain(o, trow, row, col0, 0, NC, [&] {
+                if (lane == 0) gb_bar_arrive(gb_smem(&bars.tempty[ts]));
+            });
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -242,6 +252,163 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
     if (warp == 2) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(GB_TSTAGES * NC) : "memory");
+    }
+    if (threadIdx.x == 0 && bars.abort_flag) atomicExch(err, GB_ERR_WAIT);
+}
+
+// ---- pairs of SMs: more than 128 activation rows -----------------------------------------------------------------------------------------
+// A tile of 256 weight rows x 256 activation rows is computed by the two CTAs of a cluster with one MMA per K = 16 (cta_group::2, M 256,
+// N 256): each holds 128 of the weight rows and half of the activation rows in its shared memory and the sums of its weight rows in its
+// tensor memory.  The even CTA's MMA thread issues for both.  Its `full` barrier counts the bytes of both CTAs' copies, its `tempty`
+// barrier the epilogue warps of both; commits are multicast to both CTAs' `empty` and `tfull` barriers.
+// What bounds it: shared memory, then power.  Per K = 16 an SM's tensor core takes 128 cycles; a CTA alone on its 128 x 256 tile reads
+// 12 KB and copies 12 KB in per MMA, 192 cycles at 128 bytes a cycle; a pair reads and copies 8 KB each, 128 cycles.  Against the
+// 128 x 256 tiles of single CTAs that it took the place of (us, a mat-mul alone): 8192 x 2048 x 2048 rows 62.0 -> 55.6, 14336 x 4096 x
+// 2048 188.9 -> 170.5 (1.41 PFLOP/s), 22016 x 4096 x 2048 278 -> 256.  A tile takes the same time with fewer columns (N 192, 128: no faster),
+// so 256 it is.  Two epilogue warps share a quarter of the lanes: with K = 1024 one alone would take longer than the tile's MMAs.
+constexpr int GP_EPI_WARPS = 8, GP_THREADS = 128 + GP_EPI_WARPS * 32, GP_STAGES = 6;
+constexpr int GP_A_BYTES = GB_ROWS * GB_K * 2, GP_STAGE = 2 * GP_A_BYTES, GP_SMEM = GP_STAGES * GP_STAGE + 1024;
+constexpr int GP_NC = 256;   // activation rows of a tile, tensor-memory columns of an accumulator stage
+constexpr int GP_HALF = GP_NC / 2;
+// kind::f16 instruction descriptor: F32 accumulator, BF16 x BF16, both operands K-major, N = 256, M = 256
+constexpr uint32_t GP_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GP_NC >> 3) << 17) | ((uint32_t)(2 * GB_ROWS >> 4) << 24);
+
+__device__ __forceinline__ uint32_t gp_of_rank(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void gp_tma_load(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {   // bar: the leader's, a cluster address
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map),
+                 "r"(x), "r"(y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void gp_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, int accumulate) {
+    asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p; }" ::"r"(d_tmem), "l"(adesc), "l"(bdesc),
+                 "r"(idesc), "r"(accumulate)
+                 : "memory");
+}
+__device__ __forceinline__ void gp_commit(uint32_t bar) {   // on this barrier of both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void gp_arrive(uint32_t bar) {   // a cluster address
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void gp_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(GP_THREADS, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, GbOut o, int ksteps, int col_blocks, int tiles, int *err) {
+    constexpr int S = GP_STAGES;
+    extern __shared__ uint8_t gb_raw[];
+    __shared__ GbBars bars;
+    pdl_trigger();
+    const uint32_t smem = (gb_smem(gb_raw) + 1023u) & ~1023u;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rank = (int)(blockIdx.x & 1), pair = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);   // clusters of two along x
+    volatile int *abort_flag = &bars.abort_flag;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < S; i++) {
+            gb_bar_init(gb_smem(&bars.full[i]), 1);
+            gb_bar_init(gb_smem(&bars.empty[i]), 1);
+        }
+        for (int i = 0; i < GB_TSTAGES; i++) {
+            gb_bar_init(gb_smem(&bars.tfull[i]), 1);
+            gb_bar_init(gb_smem(&bars.tempty[i]), 2 * GP_EPI_WARPS);
+        }
+        bars.abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 2) {
+        // all columns of both SMs: the operand stages fill their shared memory, so no other CTA is waiting for some
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gb_smem(&bars.tmem_base)), "r"(GB_TSTAGES * GP_NC) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    gp_cluster_sync();   // both CTAs' barriers stand
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = bars.tmem_base;
+    pdl_wait();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int step = 0;
+            for (int t = pair; t < tiles; t += pairs) {
+                const int rb = t / col_blocks, cb = t - rb * col_blocks;
+                const int arow = rb * 2 * GB_ROWS + rank * GB_ROWS, brow = cb * GP_NC + rank * GP_HALF;
+                bool ok = true;
+                for (int ks = 0; ks < ksteps; ks++, step++) {
+                    const int s = step % S;
+                    if (!gb_bar_wait(gb_smem(&bars.empty[s]), ((uint32_t)(step / S) & 1u) ^ 1u, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t own = gb_smem(&bars.full[s]), bar = gp_of_rank(own, 0), stage = smem + (uint32_t)(s * GP_STAGE);
+                    if (rank == 0) gb_bar_expect(own, 2 * GP_STAGE);
+                    gp_tma_load(stage, &wmap, ks * GB_K, arow, bar);
+                    gp_tma_load(stage + GP_A_BYTES, &xmap, ks * GB_K, brow, bar);
+                }
+                if (!ok) break;
+            }
+            // the copies in flight, also when this CTA gave up: the stages they fill come free (bounded) only after they have landed
+            for (int p = step; p < step + S; p++) {
+                for (uint32_t it = 0; it < GB_WAIT_LIMIT; it++) {
+                    uint32_t ok;
+                    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                                 : "=r"(ok) : "r"(gb_smem(&bars.empty[p % S])), "r"(((uint32_t)(p / S) & 1u) ^ 1u) : "memory");
+                    if (ok) break;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            int step = 0, j = 0;
+            bool ok = true;
+            for (int t = pair; t < tiles && ok; t += pairs, j++) {
+                const int ts = j % GB_TSTAGES;
+                if (!gb_bar_wait(gb_smem(&bars.tempty[ts]), ((uint32_t)(j / GB_TSTAGES) & 1u) ^ 1u, abort_flag)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t d_acc = tmem + (uint32_t)(ts * GP_NC);
+                for (int ks = 0; ks < ksteps; ks++, step++) {
+                    const int s = step % S;
+                    if (!gb_bar_wait(gb_smem(&bars.full[s]), (uint32_t)(step / S) & 1u, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t stage = smem + (uint32_t)(s * GP_STAGE);
+                    const uint64_t ad = gb_desc(stage), bd = gb_desc(stage + GP_A_BYTES);
+#pragma unroll
+                    for (int i = 0; i < GB_K / 16; i++) gp_mma(d_acc, ad + 2 * i, bd + 2 * i, GP_IDESC, (ks | i) != 0);   // 32 bytes on per K = 16
+                    gp_commit(gb_smem(&bars.empty[s]));
+                }
+                if (ok) gp_commit(gb_smem(&bars.tfull[ts]));
+            }
+        }
+    } else if (warp >= GB_EPI_WARP0) {
+        const int q = warp & 3, h = (warp - GB_EPI_WARP0) >> 2;   // tensor-memory lanes 32 q .., first or second half of the columns
+        int j = 0;
+        for (int t = pair; t < tiles; t += pairs, j++) {
+            const int rb = t / col_blocks, cb = t - rb * col_blocks, ts = j % GB_TSTAGES;
+            if (!__all_sync(0xffffffffu, gb_bar_wait(gb_smem(&bars.tfull[ts]), (uint32_t)(j / GB_TSTAGES) & 1u, abort_flag))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int row = rb * 2 * GB_ROWS + rank * GB_ROWS + 32 * q + lane, col0 = cb * GP_NC;
+            const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(ts * GP_NC);
+            const uint32_t free_bar = gp_of_rank(gb_smem(&bars.tempty[ts]), 0);
+            gb_drain(o, trow, row, col0, GP_HALF * h, GP_HALF * h + GP_HALF, [&] {
+                if (lane == 0) gp_arrive(free_bar);
+            });
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    gp_cluster_sync();   // nothing of either CTA reaches into the other any more
+    if (warp == 2) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(GB_TSTAGES * GP_NC) : "memory");
     }
     if (threadIdx.x == 0 && bars.abort_flag) atomicExch(err, GB_ERR_WAIT);
 }
@@ -297,6 +464,30 @@ int launch_nc(const DenseMm &d, int sms, cudaStream_t s) {
                       (int)((d.k + GB_K - 1) / GB_K), (int)cb, tiles, err);
 }
 
+int launch_pair(const DenseMm &d, int sms, cudaStream_t s) {
+    static bool attr_done[64] = {false};
+    int dev = 0;
+    B200_CUDA(cudaGetDevice(&dev));
+    B200_REQUIRE(dev >= 0 && dev < 64, "gemm: device index %d out of range", dev);
+    if (!attr_done[dev]) {
+        B200_CUDA(cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM));
+        attr_done[dev] = true;
+    }
+    CUtensorMap wmap, xmap;
+    int rc = rows_map(&wmap, d.w, d.k, d.n, d.ldw, GB_ROWS);
+    if (rc == B200_STATUS_SUCCESS) rc = rows_map(&xmap, d.x, d.k, d.m, d.ldx, GP_HALF);
+    if (rc != B200_STATUS_SUCCESS) return rc;
+    int *err = nullptr;
+    rc = device_error_word(&err);
+    if (rc != B200_STATUS_SUCCESS) return rc;
+    const int64_t rb = (d.n + 2 * GB_ROWS - 1) / (2 * GB_ROWS), cb = (d.m + GP_NC - 1) / GP_NC;
+    B200_REQUIRE(rb * cb < (1ll << 30), "gemm: too many tiles");
+    const GbOut o = {d.y, d.y_type, d.ldy, d.addend, d.ld_addend, d.bias, d.act, d.act_limit, d.act_alpha, (int)d.n, (int)d.m};
+    const int tiles = (int)(rb * cb), pairs = tiles < sms / 2 ? tiles : sms / 2;
+    return launch_pdl_cluster(gemm_bf16_pair_kernel, dim3((unsigned)(2 * pairs)), dim3(GP_THREADS), 2u, (size_t)GP_SMEM, s, wmap, xmap, o,
+                              (int)((d.k + GB_K - 1) / GB_K), (int)cb, tiles, err);
+}
+
 }  // namespace
 
 // what the tensor maps can describe: 16-byte aligned bases and row strides
@@ -309,11 +500,11 @@ int launch_gemm_bf16(const DenseMm &d, cudaStream_t s) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     if (d.m <= 64) return launch_nc<64>(d, sms, s);
-    const int64_t rb = (d.n + GB_ROWS - 1) / GB_ROWS;
-    const auto waves = [&](int nc) { return (rb * ((d.m + nc - 1) / nc) + sms - 1) / sms; };
-    // a 256-wide tile takes about 1.8 times a 128-wide one
-    if (d.m <= 128 || 10 * waves(128) <= 18 * waves(256)) return launch_nc<128>(d, sms, s);
-    return launch_nc<256>(d, sms, s);
+    // A 128 x 128 tile of one CTA takes about as long as a 256 x 256 tile of a pair (the MMA's time hardly depends on N), so the pairs pay
+    // once the small tiles would need a second wave: 6144 x 4096 x 512 rows (192 small tiles) 46.5 -> 30.7 us, 2048 x 2048 x 2048 (256) 28.2 ->
+    // 19.3; in one wave they only add their start: 4096 x 4096 x 512 (128) 27.3 -> 28.3, 300 x 264 x 300 (9) 7.8 -> 9.6
+    const int64_t small = (d.n + GB_ROWS - 1) / GB_ROWS * ((d.m + 127) / 128);
+    return d.m <= 128 || small <= sms ? launch_nc<128>(d, sms, s) : launch_pair(d, sms, s);
 }
 
 }  // namespace b200

@@ -88,6 +88,28 @@ def test_wide_tiles(sess, m):
     assert np.abs(get(sess, y) - want).max() < 1e-4
 
 
+@pytest.mark.parametrize("n,k,m", [(1290, 8, 1920), (20 * 256, 64, 897), (38 * 128 + 2, 200, 513), (149 * 128, 1032, 129)])
+def test_tiles_of_pairs(sess, n, k, m):
+    """more 128 x 128 tiles than SMs: two CTAs share a tile of 256 x 256; every epilogue, ragged on all sides"""
+    rng = np.random.default_rng(n)
+    w, x, add, bias = M.bf16(rng.standard_normal((n, k))), M.bf16(rng.standard_normal((m, k))), rng.standard_normal((m, n)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    tw, tx, ta, tb = put(sess, w, gp.BF16), put(sess, x, gp.BF16), put(sess, add), put(sess, bias)
+    plain = x.astype(np.float64) @ w.T.astype(np.float64)
+    scale = np.abs(x.astype(np.float64)) @ np.abs(w.T.astype(np.float64)) + 1.0
+    for act, addend, yt in ((0, None, gp.F32), (1, ta, gp.F32), (0, None, gp.BF16)):
+        y = node(sess, DENSE_MM, yt, [n, m], [tw, tx, addend], ints=[(0, act)])
+        assert sess.compute([y]) == 0, sess.last_error()
+        want = (P.gelu_tanh(plain) if act else plain) + (add if addend is not None else 0.0)
+        got = get(sess, y)
+        # exact products, sums in F32; BF16 results keep 8 bits
+        assert (np.abs(got - want) <= (2 ** -8 * np.abs(want) if yt == gp.BF16 else 0) + 2e-6 * scale).all()
+    y = node(sess, DENSE_MM, gp.F32, [n // 2, m], [tw, tx, None, None, tb], ints=[(0, 2)], floats=[(2, 3.0), (3, 1.702)])
+    assert sess.compute([y]) == 0, sess.last_error()
+    z = plain + bias
+    g, u = np.minimum(z[:, ::2], 3.0), np.clip(z[:, 1::2], -3.0, 3.0)
+    assert np.allclose(get(sess, y), g * P.sigmoid(1.702 * g) * (u + 1.0), rtol=1e-4, atol=2e-4 * max(1.0, np.sqrt(k) / 8))
+
+
 @pytest.mark.parametrize("wt", [gp.BF16, gp.F32])
 @pytest.mark.parametrize("n,k,m", [(50, 48, 1), (7, 37, 2), (300, 512, 5), (64, 1028, 16)])
 def test_norm_inside_the_mat_mul(sess, n, k, m, wt):
