@@ -1,3 +1,5 @@
+// Few waves of 32-row tiles of the 32-element-block types (gemm_b32_tcgen05.cu takes over beyond), MUL_MAT_ID, calls without scratch memory, and
+// Q6_K on request.
 // Prompt-shaped mat-mul for Q8_0, Q4_0, MXFP4 and Q6_K weights on the fifth-generation tensor cores: tcgen05.mma
 // kind::i8 with the block dots accumulated in tensor memory.  Same pipeline as the Q4_K kernel of gemm_tcgen05.cu
 // (one CTA = 128 weight rows x 32 activation rows, one 256-element group of K per step, producer warps that unpack
@@ -92,24 +94,33 @@ __device__ __forceinline__ void tmem_ld16(int (&v)[16], uint32_t taddr) {
                  : "memory");
 }
 
-// four 4-bit codes (one per byte of x) -> four signed bytes of 2 * E2M1: crates/ggml/src/quants.rs:660
-__device__ __forceinline__ uint32_t mxfp4_lut4(uint32_t x) {
-    const uint32_t lo = x & 0x07070707u;
-    const uint32_t t = lo | (lo >> 4);
-    const uint32_t sel = (t & 0xffu) | ((t >> 8) & 0xff00u);
-    const uint32_t pos = __byte_perm(0x03020100u, 0x0c080604u, sel);
-    const uint32_t neg = __byte_perm(0xfdfeff00u, 0xf4f8fafcu, sel);
-    const uint32_t m = ((x & 0x08080808u) >> 3) * 0xffu;
-    return (pos & ~m) | (neg & m);
+// every byte's sign bit in all its bits (the selector mode that __byte_perm leaves out)
+__device__ __forceinline__ uint32_t sign_bytes(uint32_t x) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %1, 0xba98;" : "=r"(r) : "r"(x));
+    return r;
+}
+// eight 4-bit codes -> eight signed bytes of 2 * E2M1 (crates/ggml/src/quants.rs:660): of the low nibbles and of the high ones.  Byte permutes look
+// up the values of three bits, four nibbles at a time, in a positive and a negative table; a permute that spreads sign bits makes the masks between
+// them.  15 instructions where a look-up per four separated codes took 27: 4096 x 4096 on 128 rows 46 -> 39 us (Q4_0 31), the experts above as
+// MXFP4 211 -> 176 with the work items
+__device__ __forceinline__ void mxfp4_values(uint32_t x, uint32_t *lo, uint32_t *hi) {
+    const uint32_t s0 = x & 0x77777777u, s1 = s0 >> 16;
+    const uint32_t p0 = __byte_perm(0x03020100u, 0x0c080604u, s0), p1 = __byte_perm(0x03020100u, 0x0c080604u, s1);   // nibbles 0 .. 3 and 4 .. 7
+    const uint32_t n0 = __byte_perm(0xfdfeff00u, 0xf4f8fafcu, s0), n1 = __byte_perm(0xfdfeff00u, 0xf4f8fafcu, s1);
+    const uint32_t ml = sign_bytes(x << 4), mh = sign_bytes(x);   // 0xff where the code's sign bit is set
+    *lo = (__byte_perm(p0, p1, 0x6420) & ~ml) | (__byte_perm(n0, n1, 0x6420) & ml);
+    *hi = (__byte_perm(p0, p1, 0x7531) & ~mh) | (__byte_perm(n0, n1, 0x7531) & mh);
 }
 // four nibbles (one per byte) minus 8, as signed bytes: no borrow between bytes ((n | 0x80) - 8 keeps bit 7 set, then flip it)
 __device__ __forceinline__ uint32_t nibbles_minus8(uint32_t x) { return ((x | 0x80808080u) - 0x08080808u) ^ 0x80808080u; }
 
 // MUL_MAT_ID, grouped by expert: CTA column blockIdx.x is work item w = up to 32 (token, slot) pairs routed to one
-// expert.  work_expert[w] names the expert (-1: an unused item, the CTA leaves at once), col_act[32 w + c] the
+// expert.  *n_items items are in use (the other CTAs leave at once); work_expert[w] names the expert, col_act[32 w + c] the
 // quantized activation row of column c and col_out[32 w + c] the output row (pair index), -1 for the unused columns
 // of a short item.  Null work_expert: a plain mat-mul.
 struct GroupMap {
+    const int *n_items;
     const int *work_expert;
     const int *col_act;
     const int *col_out;
@@ -166,8 +177,8 @@ gemm_i8_tcgen05_kernel(const uint8_t *__restrict__ tiles, ActView acts, float *d
     const bool grouped = gm.work_expert != nullptr;
     if (grouped) {
         pdl_wait();   // the work list is a previous kernel's output
+        if ((int)blockIdx.x >= *gm.n_items) return;   // every thread of the CTA: nothing has been allocated yet
         const int e = gm.work_expert[blockIdx.x];
-        if (e < 0) return;   // every thread of the CTA: nothing has been allocated yet
         tiles += (int64_t)e * gm.expert_bytes;
         if (threadIdx.x < TI_COLS) {
             col_act_s[threadIdx.x] = gm.col_act[(int64_t)blockIdx.x * TI_COLS + threadIdx.x];
@@ -342,15 +353,16 @@ gemm_i8_tcgen05_kernel(const uint8_t *__restrict__ tiles, ActView acts, float *d
                 for (int c = 0; c < 8; c++) {
                     // piece c = block c: low nibbles = elements 0..15 of the block, high nibbles = elements 16..31
                     uint4 lo, hi;
-                    lo.x = w[c].x & 0x0f0f0f0fu; lo.y = w[c].y & 0x0f0f0f0fu; lo.z = w[c].z & 0x0f0f0f0fu; lo.w = w[c].w & 0x0f0f0f0fu;
-                    hi.x = (w[c].x >> 4) & 0x0f0f0f0fu; hi.y = (w[c].y >> 4) & 0x0f0f0f0fu;
-                    hi.z = (w[c].z >> 4) & 0x0f0f0f0fu; hi.w = (w[c].w >> 4) & 0x0f0f0f0fu;
                     if (TYPE == B200_TYPE_MXFP4) {
-                        lo.x = mxfp4_lut4(lo.x); lo.y = mxfp4_lut4(lo.y); lo.z = mxfp4_lut4(lo.z); lo.w = mxfp4_lut4(lo.w);
-                        hi.x = mxfp4_lut4(hi.x); hi.y = mxfp4_lut4(hi.y); hi.z = mxfp4_lut4(hi.z); hi.w = mxfp4_lut4(hi.w);
+                        mxfp4_values(w[c].x, &lo.x, &hi.x);
+                        mxfp4_values(w[c].y, &lo.y, &hi.y);
+                        mxfp4_values(w[c].z, &lo.z, &hi.z);
+                        mxfp4_values(w[c].w, &lo.w, &hi.w);
                     } else {
-                        lo.x = nibbles_minus8(lo.x); lo.y = nibbles_minus8(lo.y); lo.z = nibbles_minus8(lo.z); lo.w = nibbles_minus8(lo.w);
-                        hi.x = nibbles_minus8(hi.x); hi.y = nibbles_minus8(hi.y); hi.z = nibbles_minus8(hi.z); hi.w = nibbles_minus8(hi.w);
+                        lo.x = nibbles_minus8(w[c].x & 0x0f0f0f0fu); lo.y = nibbles_minus8(w[c].y & 0x0f0f0f0fu);
+                        lo.z = nibbles_minus8(w[c].z & 0x0f0f0f0fu); lo.w = nibbles_minus8(w[c].w & 0x0f0f0f0fu);
+                        hi.x = nibbles_minus8((w[c].x >> 4) & 0x0f0f0f0fu); hi.y = nibbles_minus8((w[c].y >> 4) & 0x0f0f0f0fu);
+                        hi.z = nibbles_minus8((w[c].z >> 4) & 0x0f0f0f0fu); hi.w = nibbles_minus8((w[c].w >> 4) & 0x0f0f0f0fu);
                     }
                     *(uint4 *)(A + (2 * c) * 128) = lo;
                     *(uint4 *)(A + (2 * c + 1) * 128) = hi;
@@ -443,7 +455,7 @@ gemm_i8_tcgen05_kernel(const uint8_t *__restrict__ tiles, ActView acts, float *d
 
 template <int TYPE>
 int launch_i8(int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst, cudaStream_t s,
-              GroupMap gm = GroupMap{nullptr, nullptr, nullptr, 0}, int64_t work_items = 0) {
+              GroupMap gm = GroupMap{nullptr, nullptr, nullptr, nullptr, 0}, int64_t work_items = 0) {
     static bool attr_done[64] = {false};
     int dev = 0;
     B200_CUDA(cudaGetDevice(&dev));
@@ -462,55 +474,76 @@ int launch_i8(int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView act
                       dst, lddst, n, nb, m, err, gm);
 }
 
-// ---- MUL_MAT_ID: (token, slot) pairs grouped by expert ---------------------------------------------------------
-// counts[e] = pairs routed to expert e (the ids outside [0, n_expert) are skipped, as the per-pair kernels skip them)
-__global__ void mmid_count_kernel(const int32_t *ids, int n_pairs, int n_expert, int *counts) {
+// MUL_MAT_ID's work items, by one CTA: the (token, slot) pairs counted per expert, the experts' items (nc pairs each) laid out one after the other,
+// and every pair put in the next free column of its expert's items (which one does not matter: an output depends on its own pair only).  Pairs
+// whose id is out of range are skipped, as the per-pair kernels skip them.  Counters in shared memory, or (many experts) in global memory.
+// Latency is all there is to it: in place of a memset and three launches (27 us of kernels, one thread planning) the whole MUL_MAT_ID of 128 Q4_0
+// experts (768 x 2048) went 153 -> 138 us on 512 tokens of 8 experts, 29 -> 20 on 40 tokens of 2 (256 x 512)
+constexpr int MP_THREADS = 1024, MP_SHARED_EXPERTS = 5120;
+__global__ void __launch_bounds__(MP_THREADS) mmid_items_kernel(const int32_t *ids, int n_pairs, int n_ids, int ne11, int n_expert, int nc, int *global_counts, int *n_items,
+                                                                int *work_expert, int *col_act, int *col_out) {
+    extern __shared__ int mp_counts[];
+    __shared__ int part[MP_THREADS / 32];
     pdl_trigger();
     pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_pairs) return;
-    const int e = ids[i];
-    if (e >= 0 && e < n_expert) atomicAdd(&counts[e], 1);
-}
-// one CTA: work items per expert (32 pairs each) laid out expert after expert; first_item[e] = the expert's first item
-__global__ void mmid_plan_kernel(const int *counts, int n_expert, int max_items, int *first_item, int *cursor, int *work_expert, int *col_act,
-                                 int *col_out) {
-    pdl_trigger();
-    pdl_wait();
-    __shared__ int total;
-    if (threadIdx.x == 0) {
-        int at = 0;
-        for (int e = 0; e < n_expert; e++) {
-            first_item[e] = at;
-            cursor[e] = 0;
-            const int items = (counts[e] + TI_COLS - 1) / TI_COLS;
-            for (int i = 0; i < items && at + i < max_items; i++) work_expert[at + i] = e;
-            at += items;
-        }
-        total = at < max_items ? at : max_items;
-        for (int w = total; w < max_items; w++) work_expert[w] = -1;
+    int *first = global_counts ? global_counts : mp_counts, *cursor = first + n_expert;   // cursor: pairs counted, then columns given out
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int e = tid; e < n_expert; e += MP_THREADS) cursor[e] = 0;
+    __syncthreads();
+    for (int i = tid; i < n_pairs; i += MP_THREADS) {
+        const int e = ids[i];
+        if (e >= 0 && e < n_expert) atomicAdd(&cursor[e], 1);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < max_items * TI_COLS; i += blockDim.x) {
-        col_act[i] = -1;
-        col_out[i] = -1;
+    // a thread's run of experts, then the runs' first items
+    const int per = (n_expert + MP_THREADS - 1) / MP_THREADS, e0 = min(tid * per, n_expert), e1 = min(e0 + per, n_expert);
+    int mine = 0;
+    for (int e = e0; e < e1; e++) mine += (cursor[e] + nc - 1) / nc;
+    int at = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += v;
     }
-}
-// pair i takes the next free column of its expert's items (the order inside an expert does not matter: every output
-// element depends on its own pair only)
-__global__ void mmid_scatter_kernel(const int32_t *ids, int n_pairs, int n_ids, int ne11, int n_expert, const int *first_item, int *cursor,
-                                    int *col_act, int *col_out) {
-    pdl_trigger();
-    pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_pairs) return;
-    const int e = ids[i];
-    if (e < 0 || e >= n_expert) return;
-    const int at = atomicAdd(&cursor[e], 1);
-    const int tok = i / n_ids, slot = i % n_ids;
-    const int64_t col = (int64_t)first_item[e] * TI_COLS + at;
-    col_act[col] = tok * ne11 + slot % ne11;   // crates/ggml/src/compute.rs:2124: the activation row of a slot
-    col_out[col] = i;
+    if (lane == 31) part[warp] = at;
+    __syncthreads();
+    if (warp == 0) {
+        int v = part[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        part[lane] = v;
+    }
+    __syncthreads();
+    at += (warp ? part[warp - 1] : 0) - mine;
+    for (int e = e0; e < e1; e++) {
+        first[e] = at;
+        at += (cursor[e] + nc - 1) / nc;
+    }
+    if (tid == 0) *n_items = part[MP_THREADS / 32 - 1];
+    __syncthreads();
+    // the items' experts, the unused columns of each expert's last item
+    for (int e = warp; e < n_expert; e += MP_THREADS / 32) {
+        const int c = cursor[e], items = (c + nc - 1) / nc, base = first[e];
+        for (int i = lane; i < items; i += 32) work_expert[base + i] = e;
+        for (int i = c + lane; i < items * nc; i += 32) {
+            col_act[(int64_t)base * nc + i] = -1;
+            col_out[(int64_t)base * nc + i] = -1;
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < n_expert; e += MP_THREADS) cursor[e] = 0;
+    __syncthreads();
+    for (int i = tid; i < n_pairs; i += MP_THREADS) {
+        const int e = ids[i];
+        if (e < 0 || e >= n_expert) continue;
+        const int64_t col = (int64_t)first[e] * nc + atomicAdd(&cursor[e], 1);
+        const int tok = i / n_ids, slot = i - tok * n_ids;
+        col_act[col] = tok * ne11 + slot % ne11;   // crates/ggml/src/compute.rs:2124: the activation row of a slot
+        col_out[col] = i;
+    }
 }
 
 }  // namespace
@@ -519,28 +552,23 @@ __global__ void mmid_scatter_kernel(const int32_t *ids, int n_pairs, int n_ids, 
 // crates/ggml/src/compute.rs:2131-2151, repack.rs:1048-1068, is the per-block fma of this kernel): the pairs are counted
 // and grouped by expert on the device, and every expert's weights meet all the rows routed to it in tensor-core tiles
 // of 32 pairs.  lists: scratch of mmid_grouped_scratch_bytes(n_expert, pairs) bytes.
+static int64_t mmid_max_items(int64_t n_expert, int64_t n_pairs) { return n_pairs / TI_COLS + (n_expert < n_pairs ? n_expert : n_pairs); }
 size_t mmid_grouped_scratch_bytes(int64_t n_expert, int64_t n_pairs) {
-    const int64_t max_items = n_pairs / TI_COLS + n_expert;
-    return (size_t)(3 * n_expert + max_items + 2 * max_items * TI_COLS) * sizeof(int) + 256;
+    return (size_t)(2 * n_expert + 1 + mmid_max_items(n_expert, n_pairs) * (1 + 2 * TI_COLS)) * sizeof(int) + 256;
 }
 int launch_mul_mat_id_grouped(int type, int64_t n, int64_t k, int64_t n_expert, int64_t ne11, int64_t n_tok, int64_t n_ids, const uint8_t *tiles,
                               ActView acts, const int32_t *ids, float *dst, void *lists, cudaStream_t s) {
     B200_REQUIRE(type == B200_TYPE_MXFP4 || type == B200_TYPE_Q4_0, "mul_mat_id grouped: type %d is not a 32-element-block type on the 8x8 route", type);
     const int64_t n_pairs = n_tok * n_ids;
     B200_REQUIRE(n_pairs < 0x7fffffffLL / TI_COLS && n_expert < (1 << 20), "mul_mat_id grouped: too many pairs or experts");
-    const int64_t max_items = n_pairs / TI_COLS + n_expert;
-    int *counts = (int *)lists, *first_item = counts + n_expert, *cursor = first_item + n_expert, *work_expert = cursor + n_expert;
-    int *col_act = work_expert + max_items, *col_out = col_act + max_items * TI_COLS;
-    B200_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)n_expert, s));
-    int rc = launch_pdl(mmid_count_kernel, dim3((unsigned)((n_pairs + 255) / 256)), dim3(256), 0, s, ids, (int)n_pairs, (int)n_expert, counts);
-    if (rc != B200_STATUS_SUCCESS) return rc;
-    rc = launch_pdl(mmid_plan_kernel, dim3(1), dim3(256), 0, s, (const int *)counts, (int)n_expert, (int)max_items, first_item, cursor, work_expert,
-                    col_act, col_out);
-    if (rc != B200_STATUS_SUCCESS) return rc;
-    rc = launch_pdl(mmid_scatter_kernel, dim3((unsigned)((n_pairs + 255) / 256)), dim3(256), 0, s, ids, (int)n_pairs, (int)n_ids, (int)ne11, (int)n_expert,
-                    (const int *)first_item, cursor, col_act, col_out);
+    const int64_t max_items = mmid_max_items(n_expert, n_pairs);
+    int *counts = (int *)lists, *n_items = counts + 2 * n_expert, *work_expert = n_items + 1, *col_act = work_expert + max_items, *col_out = col_act + max_items * TI_COLS;
+    const bool shared = n_expert <= MP_SHARED_EXPERTS;   // two words each: 40 KB, within what a kernel may use unasked
+    int rc = launch_pdl(mmid_items_kernel, dim3(1), dim3(MP_THREADS), shared ? (size_t)n_expert * 8 : (size_t)0, s, ids, (int)n_pairs, (int)n_ids, (int)ne11, (int)n_expert,
+                        TI_COLS, shared ? (int *)nullptr : counts, n_items, work_expert, col_act, col_out);
     if (rc != B200_STATUS_SUCCESS) return rc;
     GroupMap gm;
+    gm.n_items = n_items;
     gm.work_expert = work_expert;
     gm.col_act = col_act;
     gm.col_out = col_out;

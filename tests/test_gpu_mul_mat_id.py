@@ -89,3 +89,30 @@ def test_grouped_by_expert_with_ragged_counts(dev, ty):
     got = dev.mul_mat_id(dev.ExpertWeights(ty, W, n, k), B, ids)
     assert dev.kernel_error() == 0
     assert bits_equal(got, want)
+
+
+@pytest.mark.parametrize("ty", [orc.MXFP4, orc.Q4_0], ids=lambda t: orc.TYPE_NAMES[t])
+def test_grouped_by_expert_with_many_pairs_each(dev, ty):
+    """hundreds of pairs an expert, many work items"""
+    E, n, k, n_tok, top = 8, 1016, 256, 603, 4
+    W = synth.weights(ty, E * n, k, seed=84, period=512).reshape(E, n, -1)
+    B = synth.activations(n_tok, k, seed=85).reshape(n_tok, 1, k)
+    rng = np.random.default_rng(86)
+    ids = np.argsort(rng.random((n_tok, E)), axis=1)[:, :top].astype(np.int32)
+    want, _ = orc.mul_mat_id(ty, W, B, ids)
+    got = dev.mul_mat_id(dev.ExpertWeights(ty, W, n, k), B, ids)
+    assert dev.kernel_error() == 0
+    assert bits_equal(got, want)
+
+
+def test_grouping_with_more_experts_than_shared_counters(dev):
+    """more experts than the grouping kernel keeps in shared memory; most have no pair"""
+    E, n, k, n_tok, top = 5200, 8, 256, 40, 2
+    W = synth.weights(orc.Q4_0, E * n, k, seed=87, period=512).reshape(E, n, -1)
+    B = synth.activations(n_tok, k, seed=88).reshape(n_tok, 1, k)
+    ids = np.random.default_rng(89).integers(0, E, (n_tok, top)).astype(np.int32)
+    ids[3] = (0, E - 1)
+    want, _ = orc.mul_mat_id(orc.Q4_0, W, B, ids)
+    got = dev.mul_mat_id(dev.ExpertWeights(orc.Q4_0, W, n, k), B, ids)
+    assert dev.kernel_error() == 0
+    assert bits_equal(got, want)
