@@ -7,11 +7,34 @@
 // store of one activation row's 32 outputs is one contiguous piece.  The activation function and the residual add are done there;
 // a gated one takes neighbouring weight rows (gate, up), which neighbouring lanes exchange, each keeping every other activation row.
 // Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device error word.
-#include <cuda.h>
-
 #include "dense.cuh"
+#include "tensor_map.h"
 
 namespace b200 {
+
+typedef CUresult (*encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                              const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static encode_fn tensor_map_encoder() {
+    static encode_fn fn = nullptr;
+    if (!fn) {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = (encode_fn)p;
+        else cudaGetLastError();
+    }
+    return fn;
+}
+int rows_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64_t k, int64_t rows, int64_t ld, int box_rows) {
+    encode_fn enc = tensor_map_encoder();
+    B200_REQUIRE(enc != nullptr, "gemm: the driver has no tensor-map encoder");
+    const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * 2};
+    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, es[2] = {1, 1};
+    const CUresult r = enc(map, type, 2, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    B200_REQUIRE(r == CUDA_SUCCESS, "gemm: tensor map of %lld x %lld (stride %lld) refused (%d)", (long long)rows, (long long)k, (long long)ld, (int)r);
+    return B200_STATUS_SUCCESS;
+}
 
 namespace {
 
@@ -262,10 +285,10 @@ gb_drain(o, trow, row, col0, 0, NC, [&] {
 // tensor memory.  The even CTA's MMA thread issues for both.  Its `full` barrier counts the bytes of both CTAs' copies, its `tempty`
 // barrier the epilogue warps of both; commits are multicast to both CTAs' `empty` and `tfull` barriers.
 // What bounds it: shared memory, then power.  Per K = 16 an SM's tensor core takes 128 cycles; a CTA alone on its 128 x 256 tile reads
-// 12 KB and copies 12 KB in per MMA, 192 cycles at 128 bytes a cycle; a pair reads and copies 8 KB each, 128 cycles.  Against the
+// 12 KB and copies 12 KB in for it, 192 cycles at 128 bytes a cycle; a pair reads and copies 8 KB each, 128 cycles.  Against the
 // 128 x 256 tiles of single CTAs that it took the place of (us, a mat-mul alone): 8192 x 2048 x 2048 rows 62.0 -> 55.6, 14336 x 4096 x
-// 2048 188.9 -> 170.5 (1.41 PFLOP/s), 22016 x 4096 x 2048 278 -> 256.  A tile takes the same time with fewer columns (N 192, 128: no faster),
-// so 256 it is.  Two epilogue warps share a quarter of the lanes: with K = 1024 one alone would take longer than the tile's MMAs.
+// 2048 188.9 -> 170.5 (1.41 PFLOP/s), 22016 x 4096 x 2048 278 -> 256.  Narrower pair tiles (N 224, 192, 160,
+// 128) took longer from 1024 x 4096 x 2048 rows up.  Two epilogue warps share a quarter of the lanes: with K = 1024 one alone would take longer than the tile's MMAs.
 constexpr int GP_EPI_WARPS = 8, GP_THREADS = 128 + GP_EPI_WARPS * 32, GP_STAGES = 6;
 constexpr int GP_A_BYTES = GB_ROWS * GB_K * 2, GP_STAGE = 2 * GP_A_BYTES, GP_SMEM = GP_STAGES * GP_STAGE + 1024;
 constexpr int GP_NC = 256;   // activation rows of a tile, tensor-memory columns of an accumulator stage
@@ -413,31 +436,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_con
     if (threadIdx.x == 0 && bars.abort_flag) atomicExch(err, GB_ERR_WAIT);
 }
 
-typedef CUresult (*encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                              const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-encode_fn tensor_map_encoder() {
-    static encode_fn fn = nullptr;
-    if (!fn) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = (encode_fn)p;
-        else cudaGetLastError();
-    }
-    return fn;
-}
-// rows of k BF16 elements ld apart, in boxes of 64 elements x box_rows
-int rows_map(CUtensorMap *map, const void *base, int64_t k, int64_t rows, int64_t ld, int box_rows) {
-    encode_fn enc = tensor_map_encoder();
-    B200_REQUIRE(enc != nullptr, "gemm: the driver has no tensor-map encoder");
-    const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)GB_K, (cuuint32_t)box_rows}, es[2] = {1, 1};
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    B200_REQUIRE(r == CUDA_SUCCESS, "gemm: tensor map of %lld x %lld (stride %lld) refused (%d)", (long long)rows, (long long)k, (long long)ld, (int)r);
-    return B200_STATUS_SUCCESS;
-}
-
 template <int NC>
 int launch_nc(const DenseMm &d, int sms, cudaStream_t s) {
     using C = GbCfg<NC>;
@@ -450,8 +448,8 @@ int launch_nc(const DenseMm &d, int sms, cudaStream_t s) {
         attr_done[dev] = true;
     }
     CUtensorMap wmap, xmap;
-    int rc = rows_map(&wmap, d.w, d.k, d.n, d.ldw, GB_ROWS);
-    if (rc == B200_STATUS_SUCCESS) rc = rows_map(&xmap, d.x, d.k, d.m, d.ldx, NC);
+    int rc = rows_map(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.w, d.k, d.n, d.ldw, GB_ROWS);
+    if (rc == B200_STATUS_SUCCESS) rc = rows_map(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.x, d.k, d.m, d.ldx, NC);
     if (rc != B200_STATUS_SUCCESS) return rc;
     int *err = nullptr;
     rc = device_error_word(&err);
@@ -474,8 +472,8 @@ int launch_pair(const DenseMm &d, int sms, cudaStream_t s) {
         attr_done[dev] = true;
     }
     CUtensorMap wmap, xmap;
-    int rc = rows_map(&wmap, d.w, d.k, d.n, d.ldw, GB_ROWS);
-    if (rc == B200_STATUS_SUCCESS) rc = rows_map(&xmap, d.x, d.k, d.m, d.ldx, GP_HALF);
+    int rc = rows_map(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.w, d.k, d.n, d.ldw, GB_ROWS);
+    if (rc == B200_STATUS_SUCCESS) rc = rows_map(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.x, d.k, d.m, d.ldx, GP_HALF);
     if (rc != B200_STATUS_SUCCESS) return rc;
     int *err = nullptr;
     rc = device_error_word(&err);
@@ -500,7 +498,7 @@ int launch_gemm_bf16(const DenseMm &d, cudaStream_t s) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     if (d.m <= 64) return launch_nc<64>(d, sms, s);
-    // A 128 x 128 tile of one CTA takes about as long as a 256 x 256 tile of a pair (the MMA's time hardly depends on N), so the pairs pay
+    // A 128 x 128 tile of one CTA takes nearly as long as a 256 x 256 tile of a pair (half the MMA time, but as many copies), so the pairs pay
     // once the small tiles would need a second wave: 6144 x 4096 x 512 rows (192 small tiles) 46.5 -> 30.7 us, 2048 x 2048 x 2048 (256) 28.2 ->
     // 19.3; in one wave they only add their start: 4096 x 4096 x 512 (128) 27.3 -> 28.3, 300 x 264 x 300 (9) 7.8 -> 9.6
     const int64_t small = (d.n + GB_ROWS - 1) / GB_ROWS * ((d.m + 127) / 128);

@@ -984,10 +984,9 @@ int launch_gemv(int type, int route, int64_t n, int64_t k, int64_t m, const uint
             const char *e = getenv("B200_Q6K_TCGEN05");
             if (e && e[0] == '1') return launch_gemm_tcgen05_i8(type, n, k, m, tiles, acts, dst, lddst, s);
         }
-        if ((type == B200_TYPE_Q4_0 || type == B200_TYPE_MXFP4) && route == B200_ROUTE_REPACK && m >= GEMM_MMA_MIN_COLS)
-            return launch_gemm_tcgen05_i8(type, n, k, m, tiles, acts, dst, lddst, s);
-        if (type == B200_TYPE_Q8_0 && route == B200_ROUTE_ROWDOT && m >= GEMM_MMA_MIN_COLS && numerics_mode() == 1)
-            return launch_gemm_tcgen05_i8(type, n, k, m, tiles, acts, dst, lddst, s);
+        const bool b32 = ((type == B200_TYPE_Q4_0 || type == B200_TYPE_MXFP4) && route == B200_ROUTE_REPACK) || (type == B200_TYPE_Q8_0 && route == B200_ROUTE_ROWDOT && numerics_mode() == 1);
+        if (b32 && m >= GEMM_MMA_MIN_COLS)
+            return !no_scratch_mode() && gemm_b32_wins(type, n, k, m) ? launch_gemm_b32(type, n, k, m, tiles, acts, dst, lddst, s) : launch_gemm_tcgen05_i8(type, n, k, m, tiles, acts, dst, lddst, s);
     }
     if (type == B200_TYPE_Q6_K && route == B200_ROUTE_TILED && m >= GEMM_MMA_MIN_COLS && gemm_mma_enabled())
         return launch_gemm_mma(6, n, k, m, tiles, acts, dst, lddst, s);

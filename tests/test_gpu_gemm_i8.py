@@ -42,6 +42,27 @@ def test_bit_exact_types(dev, ty, shape, monkeypatch):
     assert bits_equal(got, want), f"max |d| = {np.abs(got - want).max()}"
 
 
+# more waves of 32-row tiles than the f16 kernel needs of 64- (the first) and 128-row ones; ragged on both sides
+@pytest.mark.parametrize("shape", [(2056, 4096, 300), (2000, 2048, 705), (4728, 2816, 193)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("ty", [orc.Q4_0, orc.MXFP4, orc.Q8_0], ids=lambda t: orc.TYPE_NAMES[t])
+def test_many_rows(dev, ty, shape):
+    n, k, m = shape
+    W = synth.weights(ty, n, k, seed=420 + ty, period=512)
+    x = synth.activations(m, k, seed=421 + m)
+    want, _ = orc.mul_mat(ty, W, x)
+    dev.set_numerics(dev.FAST)
+    try:
+        got = dev.mul_mat(dev.Weight(ty, W, k), x)
+    finally:
+        dev.set_numerics(dev.EXACT)
+    assert dev.kernel_error() == 0
+    if ty != orc.Q8_0:
+        assert bits_equal(got, want)
+        return
+    bound = 1e-5 * (np.abs(x).astype(np.float64) @ np.abs(orc.dequantize(ty, W, k)).astype(np.float64).T)
+    assert (np.abs(got.astype(np.float64) - want.astype(np.float64)) <= bound).all()
+
+
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
 def test_q8_0_fast_mode_within_the_mat_mul_tolerance(dev, shape):
     n, k, m = shape
