@@ -119,6 +119,9 @@ void b200_debug_decode_step_wait(int spin_limit, int skip_cta, int skip_barrier)
  * per CTA.  Pure host arithmetic (CTA waves times measured time per wave, plus the expansion); no CUDA call.
  * (The reference's own choice among its gemm kernels by shape: crates/ggml/src/compute.rs:1420-1841.) */
 int b200_prompt_kernel_choice(int64_t n, int64_t m, int sm_count);
+/* The same for Q4_0, Q8_0 (fast numerics) and MXFP4 mat-muls of 8 and more activation rows: 0 = integer tcgen05 kernel, 64 / 128 = the f16
+ * tcgen05 kernel with that many activation rows per tile (both give the same bits); -1 = bad arguments. */
+int b200_block32_kernel_choice(int type, int64_t n, int64_t k, int64_t m, int sm_count);
 
 /* ---- device memory (cudaMalloc-backed; buffers of the backend use the same) */
 int b200_malloc(void **dev_ptr, size_t bytes);

@@ -162,6 +162,7 @@ int launch_gemm_tcgen05(int mode, int64_t n, int64_t k, int64_t m, const uint8_t
 int launch_gemm_tcgen05_i8(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst,
                            cudaStream_t s);
 // Q8_0 / Q4_0 / MXFP4 mat-muls of many rows on tcgen05 kind::f16, scratch for the expanded activations (gemm_b32_tcgen05.cu)
+int gemm_b32_pick_for(int type, int64_t n, int64_t k, int64_t m, int sms);
 bool gemm_b32_wins(int type, int64_t n, int64_t k, int64_t m);
 int launch_gemm_b32(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst, cudaStream_t s);
 // MUL_MAT_ID with the pairs grouped by expert on the device (MXFP4 / Q4_0 experts on the 8x8 route): gemm_tcgen05_i8.cu

@@ -15,7 +15,8 @@
 //   warps 0 .. 7    drain: warp w owns weight rows 32 (w % 4) .. and columns NC / 2 (w / 4) ..; per block d_w d_x, then the fma, two columns
 //                   per instruction
 //   warp 8          one thread issues two K = 16 MMAs per block into one of TS tensor-memory stages of NC columns
-//   warp 9          (one thread) copies the step's activations, 64 f16 of NC rows, by TMA, and their scales
+//   warp 9          (one thread) copies the step's activations, 64 f16 of NC rows, by TMA, and their scales, which have slots and barriers of
+//                   their own: the MMAs take the ones, the drain waits for the others
 //   warps 12 .. 19  produce the weights' operand: a thread per row and block of the step
 // The activations are expanded to f16 once per mat-mul (expand_q8_0_acts_kernel): rows of K values, the elements of each 8 in the order
 // 0 2 1 3 4 6 5 7 in which the producers' unpacking yields them.
@@ -56,7 +57,7 @@ struct BqCfg {
 };
 template <int NC>
 struct alignas(16) BqBars {
-    uint64_t afull[8], bfull[8], empty[8], tfull[4], tempty[4];
+    uint64_t afull[8], bfull[8], empty[8], tfull[4], tempty[4], dfull[BqCfg<NC>::DSLOTS];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -70,6 +71,9 @@ __device__ __forceinline__ void bq_init(uint64_t *bar, uint32_t count) {
 }
 __device__ __forceinline__ void bq_arrive(uint64_t *bar) {
     asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(bq_smem(bar)) : "memory");
+}
+__device__ __forceinline__ void bq_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ bool bq_poll(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
@@ -184,6 +188,7 @@ gemm_b32_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t 
             bq_init(&bars.tfull[i], 1);
             bq_init(&bars.tempty[i], BQ_EPI_WARPS);
         }
+        for (int i = 0; i < C::DSLOTS; i++) bq_init(&bars.dfull[i], 1);
         bars.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -233,6 +238,12 @@ gemm_b32_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t 
             for (int ks = 0; ks < ksteps; ks++, step++) {
                 const uint32_t ws = ws_next;
                 if (ks + 1 < ksteps) ws_next = load_scales(ks + 1);
+                // the step's activation scales, a copy of their own: the dots being there says nothing of it.  The slot is not filled again before
+                // this warp has left the step, so its phase cannot run ahead
+                if (!(ok = __all_sync(0xffffffffu, bq_wait(&bars.dfull[step % C::DSLOTS], (uint32_t)(step / C::DSLOTS) & 1u, abort_flag)))) {
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");   // the first round's loads are on their way
+                    break;
+                }
                 const float4 *das = reinterpret_cast<const float4 *>(da + (size_t)(step % C::DSLOTS) * 2 * NC + CPT * h);
                 const uint32_t trow = trow0 + (uint32_t)((step % TS) * C::TCOLS);
 #pragma unroll
@@ -392,8 +403,9 @@ gemm_b32_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t 
                         ok = false;
                         break;
                     }
-                    const uint32_t bar = bq_smem(&bars.bfull[s]), ds = bq_smem(da + (size_t)(step % C::DSLOTS) * 2 * NC);
-                    asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(C::B_STEP + C::DSLOT) : "memory");
+                    const uint32_t bar = bq_smem(&bars.bfull[s]), ds = bq_smem(da + (size_t)(step % C::DSLOTS) * 2 * NC), dbar = bq_smem(&bars.dfull[step % C::DSLOTS]);
+                    bq_expect(bar, C::B_STEP);
+                    bq_expect(dbar, C::DSLOT);
                     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
                                      smem + (uint32_t)(s * C::STAGE + BQ_A_STEP)),
                                  "l"(&xmap), "r"(ks * 64), "r"(cb * NC), "r"(bar)
@@ -401,14 +413,14 @@ gemm_b32_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t 
 #pragma unroll
                     for (int i = 0; i < 2; i++)
                         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(ds + (uint32_t)(i * NC * 4)),
-                                     "l"(scales + (int64_t)(2 * ks + i) * ld_scale + (int64_t)cb * NC), "r"(NC * 4), "r"(bar)
+                                     "l"(scales + (int64_t)(2 * ks + i) * ld_scale + (int64_t)cb * NC), "r"(NC * 4), "r"(dbar)
                                      : "memory");
                 }
             }
             // the copies in flight, also when this CTA gave up
             for (int p = step < S ? 0 : step - S; p < step; p++)
                 for (uint32_t it = 0; it < BQ_WAIT_LIMIT; it++)
-                    if (bq_poll(&bars.bfull[p % S], (uint32_t)(p / S) & 1u)) break;
+                    if (bq_poll(&bars.bfull[p % S], (uint32_t)(p / S) & 1u) && bq_poll(&bars.dfull[p % C::DSLOTS], (uint32_t)(p / C::DSLOTS) & 1u)) break;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -470,16 +482,17 @@ int b32_columns(int64_t row_blocks, int64_t m, int sms) {
 
 }  // namespace
 
-// whether launch_gemm_b32 is the quicker one: the int8 kernel (gemm_tcgen05_i8.cu) has tiles of 32 columns and no expanded activations, which pays
+// the columns of launch_gemm_b32's tiles where it is the quicker one, else 0: the int8 kernel (gemm_tcgen05_i8.cu) has tiles of 32 columns and no expanded activations, which pays
 // while they make few waves.  Same results.  us with the int8 kernel and with this one, Q8_0: 14336 x 4096 on 512 rows 364, 263 (MXFP4 512, 279);
 // 2000 x 2048 on 705 54, 44; 8000 x 2048 on 90 33, 30; and the other way 4096 x 4096 on 128 32, 51; 1024 x 2048 on 300 20, 30; 11000 x 8192 on
 // 200 243, 255
-bool gemm_b32_wins(int type, int64_t n, int64_t k, int64_t m) {
+int gemm_b32_pick_for(int type, int64_t n, int64_t k, int64_t m, int sms) {
     const int64_t row_blocks = (n + BQ_ROWS - 1) / BQ_ROWS;
-    const int sms = sm_count(), nc = b32_columns(row_blocks, m, sms);
+    const int nc = b32_columns(row_blocks, m, sms);
     const double here = b32_waves(row_blocks, m, nc, sms) * (nc == 128 ? BQ_WAVE_128 : BQ_WAVE_64) * (double)(k / 32) + BQ_EXPAND;
-    return here < b32_waves(row_blocks, m, 32, sms) * (type == B200_TYPE_MXFP4 ? BQ_WAVE_I8_MXFP4 : BQ_WAVE_I8) * (double)(k / 32);
+    return here < b32_waves(row_blocks, m, 32, sms) * (type == B200_TYPE_MXFP4 ? BQ_WAVE_I8_MXFP4 : BQ_WAVE_I8) * (double)(k / 32) ? nc : 0;
 }
+bool gemm_b32_wins(int type, int64_t n, int64_t k, int64_t m) { return gemm_b32_pick_for(type, n, k, m, sm_count()) != 0; }
 
 // Q8_0 (fast numerics), Q4_0 and MXFP4 (8x8 gemm chain) mat-muls
 int launch_gemm_b32(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst, cudaStream_t s) {

@@ -5,6 +5,8 @@ exact integer block dots and run the same f32 chain.  Q8_0's tensor-core form be
 numerics mode: it adds whole 32-element block dots where the CPU route adds eight lanes of four, so it is held to
 the mat-mul tolerance instead, defined as the reference defines it (crates/ggml/src/compute.rs:7467-7577):
 |got - ref| <= 1e-5 * sum_k |w_k x_k| per output element."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -42,24 +44,41 @@ def test_bit_exact_types(dev, ty, shape, monkeypatch):
     assert bits_equal(got, want), f"max |d| = {np.abs(got - want).max()}"
 
 
-# more waves of 32-row tiles than the f16 kernel needs of 64- (the first) and 128-row ones; ragged on both sides
-@pytest.mark.parametrize("shape", [(2056, 4096, 300), (2000, 2048, 705), (4728, 2816, 193)], ids=lambda s: "x".join(map(str, s)))
+# the f16 kernel's tiles of 64 and of 128 columns, ragged on both sides: one tile a CTA, then three and more (its stages, scale slots and sums
+# carried from tile to tile), the last ones with only one 256-element group a tile
+MANY_ROWS = [(2056, 4096, 300, 64), (2000, 2048, 705, 128), (4728, 2816, 193, 64), (56296, 1024, 61, 64), (14344, 1024, 509, 128), (14344, 256, 509, 128)]
+
+
+@pytest.mark.parametrize("shape", MANY_ROWS, ids=lambda s: "x".join(map(str, s[:3])))
 @pytest.mark.parametrize("ty", [orc.Q4_0, orc.MXFP4, orc.Q8_0], ids=lambda t: orc.TYPE_NAMES[t])
 def test_many_rows(dev, ty, shape):
-    n, k, m = shape
-    W = synth.weights(ty, n, k, seed=420 + ty, period=512)
+    n, k, m, columns = shape
+    assert dev.lib.b200_block32_kernel_choice(ty, C.c_int64(n), C.c_int64(k), C.c_int64(m), 148) == columns
+    period, ld = 504, n + 8   # rows of the result farther apart than its length
+    W = synth.weights(ty, n, k, seed=420 + ty, period=period)
     x = synth.activations(m, k, seed=421 + m)
-    want, _ = orc.mul_mat(ty, W, x)
+    want, _ = orc.mul_mat(ty, W[:period], x)   # a multiple of 8 rows: the same route
+    want = np.tile(want, (1, (n + period - 1) // period))[:, :n]
+    w, dx, out = dev.Weight(ty, W, k), dev.device_array(x), dev.device_array(np.full((m, ld), 7.0, np.float32))
+
+    def run(entry):
+        dev.check(entry(ty, n, k, m, w.ptr, dx.ptr, k, out.ptr, ld, 0, None), "mul_mat")
+        assert dev.kernel_error() == 0
+        got = out.download(np.float32, m * ld).reshape(m, ld)
+        assert (got[:, n:] == 7.0).all()
+        return got[:, :n]
+
     dev.set_numerics(dev.FAST)
     try:
-        got = dev.mul_mat(dev.Weight(ty, W, k), x)
+        got = run(dev.lib.b200_mul_mat)
+        if ty != orc.Q8_0:
+            assert bits_equal(got, want)
+        elif dev.lib.b200_act_scratch_nbytes(m, k) <= dev.lib.b200_static_scratch_nbytes():
+            assert bits_equal(got, run(dev.lib.b200_mul_mat_static_scratch))   # the int8 kernel: the same chain
     finally:
         dev.set_numerics(dev.EXACT)
-    assert dev.kernel_error() == 0
-    if ty != orc.Q8_0:
-        assert bits_equal(got, want)
-        return
-    bound = 1e-5 * (np.abs(x).astype(np.float64) @ np.abs(orc.dequantize(ty, W, k)).astype(np.float64).T)
+    bound = 1e-5 * (np.abs(x).astype(np.float64) @ np.abs(orc.dequantize(ty, W[:period], k)).astype(np.float64).T)
+    bound = np.tile(bound, (1, (n + period - 1) // period))[:, :n]
     assert (np.abs(got.astype(np.float64) - want.astype(np.float64)) <= bound).all()
 
 
