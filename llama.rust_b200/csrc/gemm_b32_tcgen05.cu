@@ -47,8 +47,9 @@ struct BqCfg {
     static constexpr int STAGES = NC == 128 ? 6 : 8;
     static constexpr int TS = 256 / NC, TCOLS = 2 * NC;   // tensor-memory stages: the two blocks of a step next to each other
     // scale slots: when a stage comes free (its MMAs are done) the drain may still be in the step TS steps behind it
-    static constexpr int DSLOTS = STAGES + TS + 1, DSLOT = 2 * NC * 4;
-    static constexpr int SMEM = STAGES * STAGE + DSLOTS * DSLOT + 1024;   // 206848, 204288
+    static constexpr int DSLOTS = 16, DSLOT = 2 * NC * 4;
+    static_assert(DSLOTS > STAGES + TS, "scale slots");
+    static constexpr int SMEM = STAGES * STAGE + DSLOTS * DSLOT + 1024;   // 214016, 205824
     // two warpgroups drain, one holds the single-thread roles, two produce: the sum stays within the 5 x 96 registers of the launch
     static constexpr int REGS_EPI = NC == 128 ? 152 : 144, REGS_CTL = 40, REGS_PROD = NC == 128 ? 64 : 72;
     static_assert(2 * REGS_EPI + REGS_CTL + 2 * REGS_PROD <= 5 * 96, "register split");
@@ -213,8 +214,11 @@ gemm_b32_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t 
         float2 acc[CPT / 2];
         int step = 0;   // steps done by this CTA
         bool ok = true;
-        const auto ready = [&](int p) {   // step p's dots are in tensor memory
-            const bool r = __all_sync(0xffffffffu, bq_wait(&bars.tfull[p % TS], (uint32_t)(p / TS) & 1u, abort_flag));
+        // step p's dots are in tensor memory, and its activation scales in their slot: a copy of their own, of which the dots being there says
+        // nothing.  The slot is not filled again before this warp has left the step, so its phase cannot run ahead
+        const auto ready = [&](int p) {
+            const bool r = __all_sync(0xffffffffu, bq_wait(&bars.tfull[p % TS], (uint32_t)(p / TS) & 1u, abort_flag) &&
+                                                       bq_wait(&bars.dfull[p % C::DSLOTS], (uint32_t)(p / C::DSLOTS) & 1u, abort_flag));
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             return r;
         };
@@ -238,12 +242,6 @@ gemm_b32_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t 
             for (int ks = 0; ks < ksteps; ks++, step++) {
                 const uint32_t ws = ws_next;
                 if (ks + 1 < ksteps) ws_next = load_scales(ks + 1);
-                // the step's activation scales, a copy of their own: the dots being there says nothing of it.  The slot is not filled again before
-                // this warp has left the step, so its phase cannot run ahead
-                if (!(ok = __all_sync(0xffffffffu, bq_wait(&bars.dfull[step % C::DSLOTS], (uint32_t)(step / C::DSLOTS) & 1u, abort_flag)))) {
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");   // the first round's loads are on their way
-                    break;
-                }
                 const float4 *das = reinterpret_cast<const float4 *>(da + (size_t)(step % C::DSLOTS) * 2 * NC + CPT * h);
                 const uint32_t trow = trow0 + (uint32_t)((step % TS) * C::TCOLS);
 #pragma unroll
@@ -257,8 +255,13 @@ gemm_b32_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t 
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
                         if (lane == 0) bq_arrive(&bars.tempty[step % TS]);
-                        // the next step's first round, if its dots are there already
-                        early = ks + 1 == ksteps || __all_sync(0xffffffffu, bq_poll(&bars.tfull[(step + 1) % TS], (uint32_t)((step + 1) / TS) & 1u));
+                        // the next step's first round, if its dots (and scales) are there already
+                        early = ks + 1 == ksteps;
+                        if (!early) {
+                            const bool dots = bq_poll(&bars.tfull[(step + 1) % TS], (uint32_t)((step + 1) / TS) & 1u);
+                            const bool scales_in = bq_poll(&bars.dfull[(step + 1) % C::DSLOTS], (uint32_t)((step + 1) / C::DSLOTS) & 1u);
+                            early = __all_sync(0xffffffffu, dots && scales_in);
+                        }
                         if (early && ks + 1 < ksteps) {
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                             bq_ld32(v[0], trow0 + (uint32_t)(((step + 1) % TS) * C::TCOLS));
