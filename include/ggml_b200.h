@@ -121,7 +121,7 @@ void b200_debug_decode_step_wait(int spin_limit, int skip_cta, int skip_barrier)
 int b200_prompt_kernel_choice(int64_t n, int64_t m, int sm_count);
 /* The same for Q4_0, Q8_0 (fast numerics) and MXFP4 mat-muls of 8 and more activation rows: 0 = integer tcgen05 kernel, 64 / 128 = the f16
  * tcgen05 kernel with that many activation rows per tile (both give the same bits); -1 = bad arguments. */
-int b200_block32_kernel_choice(int type, int64_t n, int64_t k, int64_t m, int sm_count);
+int b200_block32_kernel_choice(int type, int64_t n, int64_t m, int sm_count);
 
 /* ---- device memory (cudaMalloc-backed; buffers of the backend use the same) */
 int b200_malloc(void **dev_ptr, size_t bytes);
@@ -157,7 +157,11 @@ int b200_quantize_activations(int kind, int64_t m, int64_t k, const float *dev_x
 
 /* Device-side form of the same quantizers for callers that own the scratch:
  * dev_act must hold b200_act_scratch_nbytes(m, k) bytes (256-byte aligned). One
- * quantized activation can feed several mat-muls (wq/wk/wv read the same row). */
+ * quantized activation can feed several mat-muls (wq/wk/wv read the same row).
+ * Of more than 32 rows the block also has room for Q8_0 values as f16 (2 bytes an
+ * element), which the quantizer writes for the tensor-core kernels: Q8_0, Q4_0 and
+ * MXFP4 mat-muls on such blocks use no memory of the library's, so that calls with
+ * blocks of their own may run in several streams and be captured. */
 size_t b200_act_scratch_nbytes(int64_t m, int64_t k);
 int b200_quantize_activations_device(int kind, int64_t m, int64_t k, const float *dev_x, int64_t ldx,
                                      void *dev_act, void *stream);

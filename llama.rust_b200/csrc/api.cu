@@ -64,7 +64,7 @@ unsigned long long library_alloc_count() {
     std::lock_guard<std::mutex> lk(g_scratch_mu);
     return g_alloc_count;
 }
-static Scratch g_scratch[4][64];   // [0] general scratch, [1] the K-split exchange of the decode mat-mul (lives across the other's users)
+static Scratch g_scratch[5][64];   // [0] general scratch, [1] the K-split exchange of the decode mat-mul (lives across the other's users)
 static unsigned long long g_scratch_gen = 0;
 
 // bumped whenever a scratch block is replaced: a captured CUDA graph that baked the old address in is stale
@@ -78,6 +78,19 @@ int scratch_get(size_t bytes, void **ptr) { return scratch_get_slot(0, bytes, pt
 int scratch_get_kx(size_t bytes, void **ptr) { return scratch_get_slot(1, bytes, ptr); }
 int scratch_get_lists(size_t bytes, void **ptr) { return scratch_get_slot(2, bytes, ptr); }   // attention's visible-position lists
 int scratch_get_images(size_t bytes, void **ptr) { return scratch_get_slot(3, bytes, ptr); }  // the prompt mat-mul's f16 operand images
+// b200_mul_mat's f16 activations, where their kernel is the quicker one and a block for them can be had.  In a block of their own, and never of a
+// call that is being captured: a graph of b200_mul_mat keeps only the address of the general block, as with the kernels that do without
+static ActF16 scratch_f16_acts(int type, int route, int64_t n, int64_t k, int64_t m, cudaStream_t s) {
+    ActF16 none;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (!gemv_wants_f16_acts(type, route, n, m) || act_f16_bytes(m, k) == 0) return none;
+    void *p = nullptr;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess || (st == cudaStreamCaptureStatusNone && scratch_get_slot(4, act_f16_bytes(m, k), &p) != B200_STATUS_SUCCESS)) {
+        cudaGetLastError();
+        return none;
+    }
+    return act_f16_carve(p, m, k);
+}
 static int scratch_get_slot(int slot, size_t bytes, void **ptr) {
     int dev = 0;
     B200_CUDA(cudaGetDevice(&dev));
@@ -198,9 +211,9 @@ int b200_debug_decode_step_times(unsigned long long *out, int n) { return decode
 void b200_debug_decode_step_wait(int spin_limit, int skip_cta, int skip_barrier) { decode_persistent_debug(spin_limit, skip_cta, skip_barrier); }
 
 int b200_prompt_kernel_choice(int64_t n, int64_t m, int sm_count) { return gemm_chain_pick_for(n, m, sm_count); }
-int b200_block32_kernel_choice(int type, int64_t n, int64_t k, int64_t m, int sm_count) {
-    if ((type != B200_TYPE_Q4_0 && type != B200_TYPE_Q8_0 && type != B200_TYPE_MXFP4) || n <= 0 || k <= 0 || k % GROUP_K != 0 || m <= 0 || sm_count <= 0) return -1;
-    return gemm_b32_pick_for(type, n, k, m, sm_count);
+int b200_block32_kernel_choice(int type, int64_t n, int64_t m, int sm_count) {
+    if ((type != B200_TYPE_Q4_0 && type != B200_TYPE_Q8_0 && type != B200_TYPE_MXFP4) || n <= 0 || m <= 0 || sm_count <= 0) return -1;
+    return gemm_b32_pick_for(type, n, m, sm_count);
 }
 
 int b200_malloc(void **dev_ptr, size_t bytes) {
@@ -374,7 +387,12 @@ int b200_quantize_activations(int kind, int64_t m, int64_t k, const float *dev_x
 
 size_t b200_act_scratch_nbytes(int64_t m, int64_t k) {
     if (m < 0 || k <= 0 || k % 32 != 0) return 0;
-    return act_scratch_bytes(m, k);
+    return act_scratch_bytes(m, k) + act_f16_bytes(m, k);
+}
+
+// the f16 rows in a caller's block: behind the quantized ones
+static ActF16 callers_f16_acts(const void *dev_act, int kind, int64_t m, int64_t k) {
+    return kind == B200_ACT_Q8_0 ? act_f16_carve((uint8_t *)const_cast<void *>(dev_act) + act_scratch_bytes(m, k), m, k) : ActF16{};
 }
 
 int b200_quantize_activations_device(int kind, int64_t m, int64_t k, const float *dev_x, int64_t ldx, void *dev_act,
@@ -383,7 +401,7 @@ int b200_quantize_activations_device(int kind, int64_t m, int64_t k, const float
     if (m == 0) return B200_STATUS_SUCCESS;
     B200_REQUIRE(dev_x && dev_act, "quantize_activations_device: null pointer");
     B200_REQUIRE(((uintptr_t)dev_act & 255) == 0, "quantize_activations_device: scratch must be 256-byte aligned");
-    return launch_quantize_acts(kind, m, k, dev_x, ldx, act_carve(dev_act, m, k), (cudaStream_t)stream);
+    return launch_quantize_acts(kind, m, k, dev_x, ldx, act_carve(dev_act, m, k), (cudaStream_t)stream, callers_f16_acts(dev_act, kind, m, k));
 }
 
 int b200_event_create(void **event) {
@@ -429,7 +447,7 @@ int b200_mul_mat_q8(int type, int64_t n, int64_t k, int64_t m, const void *dev_w
     B200_REQUIRE(act_kind == act_kind_for(type, route, m), "mul_mat_q8: activation kind %d does not fit type %d", act_kind,
                  type);
     ActBuf a = act_carve(const_cast<void *>(dev_act), m, k);
-    return launch_gemv(type, route, n, k, m, (const uint8_t *)dev_w, a.view(), dev_dst, lddst, (cudaStream_t)stream);
+    return launch_gemv(type, route, n, k, m, (const uint8_t *)dev_w, a.view(), dev_dst, lddst, (cudaStream_t)stream, callers_f16_acts(dev_act, act_kind, m, k));
 }
 
 // Times `reps` back-to-back launches of b200_mul_mat_q8 that rotate over n_w copies of the weights, as one replayed
@@ -506,7 +524,7 @@ int b200_mul_mat_q8_rows_multi(int type, int64_t k, int64_t m, int count, const 
     }
     B200_REQUIRE(act_kind == act_kind_for(type, route, m), "mul_mat_q8_rows_multi: activation kind %d does not fit type %d", act_kind, type);
     ActBuf a = act_carve(const_cast<void *>(dev_act), m, k);
-    return launch_gemv_rows_multi(type, route, count, n, k, m, (const uint8_t *const *)dev_w, a.view(), dev_dst, lddst, (cudaStream_t)stream);
+    return launch_gemv_rows_multi(type, route, count, n, k, m, (const uint8_t *const *)dev_w, a.view(), dev_dst, lddst, (cudaStream_t)stream, callers_f16_acts(dev_act, act_kind, m, k));
 }
 
 int b200_mul_mat_row_fused(int type, int64_t k, int count, const int64_t *n, const void *const *dev_w, float *const *dev_dst,
@@ -596,9 +614,10 @@ int b200_mul_mat(int type, int64_t n, int64_t k, int64_t m, const void *dev_w, c
     if (rc != B200_STATUS_SUCCESS) return rc;
     ActBuf a = act_carve(scratch, m, k);
     const int kind = act_kind_for(type, route, m);
-    rc = launch_quantize_acts(kind, m, k, dev_x, ldx, a, s);
+    const ActF16 f16 = scratch_f16_acts(type, route, n, k, m, s);
+    rc = launch_quantize_acts(kind, m, k, dev_x, ldx, a, s, f16);
     if (rc != B200_STATUS_SUCCESS) return rc;
-    return launch_gemv(type, route, n, k, m, (const uint8_t *)dev_w, a.view(), dev_dst, lddst, s);
+    return launch_gemv(type, route, n, k, m, (const uint8_t *)dev_w, a.view(), dev_dst, lddst, s, f16);
 }
 
 int b200_mul_mat_host(int type, int64_t n, int64_t k, int64_t m, const void *dev_w, const float *host_x,

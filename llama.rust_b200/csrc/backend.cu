@@ -581,7 +581,7 @@ static int mul_mat_2d(BackendCtx *bc, const ggml_tensor *w, const float *x, int6
 // the quantized copy of activation rows x in bc->act, made now unless the previous mat-mul left the same one
 static int quantized_acts(BackendCtx *bc, const float *x, int64_t ldx, int64_t m, int64_t k, int kind) {
     if (!(bc->act_src == x && bc->act_m == m && bc->act_k == k && bc->act_ld == ldx && bc->act_kind == kind)) {
-        const size_t need = b200_act_scratch_nbytes(m, k);
+        const size_t need = kind == B200_ACT_Q8_0 ? b200_act_scratch_nbytes(m, k) : act_scratch_bytes(m, k);   // only Q8_0 rows have an f16 form
         if (need > bc->act_bytes) {
             if (bc->act) B200_CUDA(cudaFree(bc->act));
             bc->act = nullptr;
@@ -784,7 +784,7 @@ static int upcoming_q8_K_kind(const ggml_cgraph *g, int from, const ggml_tensor 
     return 0;
 }
 static int act_reserve(BackendCtx *bc, int64_t m, int64_t k) {
-    const size_t need = b200_act_scratch_nbytes(m, k);
+    const size_t need = act_scratch_bytes(m, k);   // Q8_K kinds
     if (need > bc->act_bytes) {
         B200_CUDA(cudaStreamSynchronize(bc->stream));
         if (bc->act) B200_CUDA(cudaFree(bc->act));

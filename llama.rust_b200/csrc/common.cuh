@@ -138,14 +138,25 @@ struct ActPrologue {
 };
 size_t act_scratch_bytes(int64_t m, int64_t k);
 ActBuf act_carve(void *scratch, int64_t m, int64_t k);
+// Q8_0 rows once more as the f16 tensor-core kernel reads them (gemm_b32_tcgen05.cu), for batches that it can take: f16 values, the elements of
+// each 8 in the order 0 2 1 3 4 6 5 7, and the scales as f32, [block][row], zero from row m up to ld.  x null: absent
+struct ActF16 {
+    uint16_t *x = nullptr;
+    float *scales = nullptr;
+    int64_t ld = 0;
+};
+constexpr int ACT_F16_MIN_ROWS = 33;   // up to 32 rows the int8 kernel, with tiles of 32, needs no more of them
+size_t act_f16_bytes(int64_t m, int64_t k);   // 0: too few rows, or no mat-mul has rows of this length
+ActF16 act_f16_carve(void *block, int64_t m, int64_t k);
 
 // ---- kernels' host launchers (each returns a b200_status) -------------------
-int launch_quantize_acts(int kind, int64_t m, int64_t k, const float *x, int64_t ldx, ActBuf out, cudaStream_t s);
+int launch_quantize_acts(int kind, int64_t m, int64_t k, const float *x, int64_t ldx, ActBuf out, cudaStream_t s, ActF16 f16 = ActF16{});   // f16: Q8_0 only
 int launch_repack(int type, int64_t n_rows, int64_t k, const uint8_t *src_blocks, uint8_t *tiles, bool inverse,
                   cudaStream_t s);
 int launch_dequantize(int type, int64_t n_rows, int64_t k, const uint8_t *tiles, float *out, cudaStream_t s);
 int launch_gemv(int type, int route, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts,
-                float *dst, int64_t lddst, cudaStream_t s);
+                float *dst, int64_t lddst, cudaStream_t s, ActF16 f16 = ActF16{});
+bool gemv_wants_f16_acts(int type, int route, int64_t n, int64_t m);   // whether launch_gemv reads them where it is given them
 
 int launch_gemm_mma(int mode, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst,
                     cudaStream_t s);
@@ -161,10 +172,10 @@ int launch_gemm_tcgen05(int mode, int64_t n, int64_t k, int64_t m, const uint8_t
 // Q8_0 / Q4_0 / MXFP4 / Q6_K prompt mat-muls on tcgen05 kind::i8 (gemm_tcgen05_i8.cu)
 int launch_gemm_tcgen05_i8(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst,
                            cudaStream_t s);
-// Q8_0 / Q4_0 / MXFP4 mat-muls of many rows on tcgen05 kind::f16, scratch for the expanded activations (gemm_b32_tcgen05.cu)
-int gemm_b32_pick_for(int type, int64_t n, int64_t k, int64_t m, int sms);
-bool gemm_b32_wins(int type, int64_t n, int64_t k, int64_t m);
-int launch_gemm_b32(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst, cudaStream_t s);
+// Q8_0 / Q4_0 / MXFP4 mat-muls of many rows on tcgen05 kind::f16 (gemm_b32_tcgen05.cu)
+int gemm_b32_pick_for(int type, int64_t n, int64_t m, int sms);
+bool gemm_b32_wins(int type, int64_t n, int64_t m);
+int launch_gemm_b32(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActF16 acts, float *dst, int64_t lddst, cudaStream_t s);
 // MUL_MAT_ID with the pairs grouped by expert on the device (MXFP4 / Q4_0 experts on the 8x8 route): gemm_tcgen05_i8.cu
 size_t mmid_grouped_scratch_bytes(int64_t n_expert, int64_t n_pairs);
 int launch_mul_mat_id_grouped(int type, int64_t n, int64_t k, int64_t n_expert, int64_t ne11, int64_t n_tok, int64_t n_ids, const uint8_t *tiles,
@@ -177,7 +188,7 @@ int launch_gemm_tcgen05_f16x64(int64_t n, int64_t k, int64_t m, const uint8_t *t
 constexpr int GEMM_FAST_MIN_COLS = 64;   // activation rows from which the fast-numerics Q4_K prompt kernel takes the mat-mul
 int gemm_tcgen05_f16_choice();   // gemm_tcgen05.cu: B200_GEMM_TCGEN05_F16 (-1 = unset: the library picks)
 int launch_gemv_rows_multi(int type, int route, int count, const int64_t *n, int64_t k, int64_t m, const uint8_t *const *tiles, ActView acts, float *const *dst,
-                           const int64_t *lddst, cudaStream_t s);   // gemv.cu
+                           const int64_t *lddst, cudaStream_t s, ActF16 f16 = ActF16{});   // gemv.cu
 int launch_gemm_kq_fast_multi(int type, int count, const int64_t *n, int64_t k, int64_t m, const uint8_t *const *tiles, ActView acts, float *const *dst,
                               const int64_t *lddst, cudaStream_t s);   // up to three matrices over the same activations
 int launch_gemm_kq_fast(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst, cudaStream_t s);   // Q4_K / Q6_K

@@ -18,8 +18,8 @@
 //   warp 9          (one thread) copies the step's activations, 64 f16 of NC rows, by TMA, and their scales, which have slots and barriers of
 //                   their own: the MMAs take the ones, the drain waits for the others
 //   warps 12 .. 19  produce the weights' operand: a thread per row and block of the step
-// The activations are expanded to f16 once per mat-mul (expand_q8_0_acts_kernel): rows of K values, the elements of each 8 in the order
-// 0 2 1 3 4 6 5 7 in which the producers' unpacking yields them.
+// The activations come as f16 from their quantizer (ActF16): rows of K values, the elements of each 8 in the order 0 2 1 3 4 6 5 7 in which the
+// producers' unpacking yields them, in the block that holds the quantized rows: calls with blocks of their own share nothing.
 //
 // What bounds it: the handing over of blocks and shared memory.  A block of a 128 x 128 tile takes 820 cycles; its MMAs take 128, the drain's lanes 256
 // (a multiply and an fma per output, half of the issue slots with the producers), shared memory about 670 wavefronts (scales 290, operands of
@@ -140,28 +140,6 @@ __device__ __forceinline__ uint32_t bq_nibbles(uint32_t x) {
         return bq_h2(__hmul2(bq_as_h2(em | s), __float2half2_rn(32768.0f)));
     }
 }
-
-}  // namespace
-
-// Q8_0 activations -> f16 rows (see above) and their scales as f32, [block][ld_scale], zero past row m.  A CTA takes 32 rows x
-// 128 elements.
-__global__ void __launch_bounds__(256) expand_q8_0_acts_kernel(ActView acts, __half *x, float *scales, int64_t ld_scale, int64_t m) {
-    pdl_trigger();
-    pdl_wait();
-    const int64_t K = acts.k, r0 = (int64_t)blockIdx.x * 32, row = r0 + (threadIdx.x >> 3), at = (int64_t)blockIdx.y * 128 + (threadIdx.x & 7) * 16;
-    if (row < m) {
-        const uint4 y = *(const uint4 *)(acts.qs + row * K + at);
-        uint4 *o = (uint4 *)(x + row * K + at);
-        o[0] = make_uint4(bq_signed(y.x, 0), bq_signed(y.x, 8), bq_signed(y.y, 0), bq_signed(y.y, 8));
-        o[1] = make_uint4(bq_signed(y.z, 0), bq_signed(y.z, 8), bq_signed(y.w, 0), bq_signed(y.w, 8));
-    }
-    if (threadIdx.x < 128) {
-        const int64_t blk = (int64_t)blockIdx.y * 4 + (threadIdx.x >> 5), r = r0 + (threadIdx.x & 31);
-        if (r < ld_scale) scales[blk * ld_scale + r] = r < m ? f16_bits_to_f32(acts.dh[r * (K / 32) + blk]) : 0.0f;
-    }
-}
-
-namespace {
 
 template <int TYPE, int NC>
 __global__ void __launch_bounds__(BQ_THREADS, 1)
@@ -440,8 +418,7 @@ struct BqCall {
     const uint8_t *tiles;
     float *dst;
     int64_t lddst;
-    const __half *x;
-    const float *scales;
+    ActF16 acts;
     int64_t row_blocks, col_blocks;
 };
 
@@ -459,11 +436,11 @@ int launch_b32(const BqCall &c, int sms, cudaStream_t s) {
     int rc = device_error_word(&err);
     if (rc != B200_STATUS_SUCCESS) return rc;
     CUtensorMap xmap;
-    rc = rows_map(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, c.x, c.k, c.m, c.k, NC);
+    rc = rows_map(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, c.acts.x, c.k, c.m, c.k, NC);
     if (rc != B200_STATUS_SUCCESS) return rc;
     const int64_t tiles = c.row_blocks * c.col_blocks;
-    return launch_pdl(gemm_b32_tcgen05_kernel<TYPE, NC>, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(BQ_THREADS), (size_t)BqCfg<NC>::SMEM, s, xmap, c.tiles, c.scales,
-                      c.col_blocks * NC, c.dst, c.lddst, c.n, (int)(c.k / GROUP_K), c.m, (int)c.row_blocks, (int)c.col_blocks, err);
+    return launch_pdl(gemm_b32_tcgen05_kernel<TYPE, NC>, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(BQ_THREADS), (size_t)BqCfg<NC>::SMEM, s, xmap, c.tiles, (const float *)c.acts.scales,
+                      c.acts.ld, c.dst, c.lddst, c.n, (int)(c.k / GROUP_K), c.m, (int)c.row_blocks, (int)c.col_blocks, err);
 }
 template <int TYPE>
 int launch_b32_nc(int nc, const BqCall &c, int sms, cudaStream_t s) {
@@ -475,50 +452,40 @@ int sm_count() {
     return sms;
 }
 
-// ns of a wave of tiles per 32-element block, with 64 and 128 columns (4096 x 4096 on 64 rows 50 us, on 512 rows 75 us), of the int8 kernel's 32
-// columns (4096 x 4096 on 64 rows 31 us), and ns of the expansion
-constexpr double BQ_WAVE_64 = 350, BQ_WAVE_128 = 500, BQ_WAVE_I8 = 200, BQ_WAVE_I8_MXFP4 = 260, BQ_EXPAND = 3000;
-double b32_waves(int64_t row_blocks, int64_t m, int nc, int sms) { return (double)((row_blocks * ((m + nc - 1) / nc) + sms - 1) / sms); }
+// ns of a wave of tiles per 32-element block, with 64 and 128 columns (4096 x 4096 on 256 rows 48 us, on 512 rows 72 us), and of the int8
+// kernel's 32 columns (4096 x 4096 on 64 rows 31 us; MXFP4 38)
+constexpr int BQ_WAVE_64 = 350, BQ_WAVE_128 = 500, BQ_WAVE_I8 = 200, BQ_WAVE_I8_MXFP4 = 260;
+int64_t b32_waves(int64_t row_blocks, int64_t m, int nc, int sms) { return (row_blocks * ((m + nc - 1) / nc) + sms - 1) / sms; }
 int b32_columns(int64_t row_blocks, int64_t m, int sms) {
     return b32_waves(row_blocks, m, 128, sms) * BQ_WAVE_128 < b32_waves(row_blocks, m, 64, sms) * BQ_WAVE_64 ? 128 : 64;
 }
 
 }  // namespace
 
-// the columns of launch_gemm_b32's tiles where it is the quicker one, else 0: the int8 kernel (gemm_tcgen05_i8.cu) has tiles of 32 columns and no expanded activations, which pays
-// while they make few waves.  Same results.  us with the int8 kernel and with this one, Q8_0: 14336 x 4096 on 512 rows 364, 263 (MXFP4 512, 279);
-// 2000 x 2048 on 705 54, 44; 8000 x 2048 on 90 33, 30; and the other way 4096 x 4096 on 128 32, 51; 1024 x 2048 on 300 20, 30; 11000 x 8192 on
-// 200 243, 255
-int gemm_b32_pick_for(int type, int64_t n, int64_t k, int64_t m, int sms) {
+// the columns of launch_gemm_b32's tiles where it is the quicker one, else 0: the int8 kernel (gemm_tcgen05_i8.cu) has tiles of 32 columns, which
+// pays while they make few waves.  Same results.  us of a call with the int8 kernel and with this one, Q8_0: 14336 x 4096 on 512 rows
+// 367, 262 (MXFP4 442, 239); 8816 x 2304 on 107 37, 33; 2488 x 1024 on 307 22, 18; and the other way 4096 x 4096 on 128 32, 50; 23288 x 11520 on
+// 134 466, 487
+int gemm_b32_pick_for(int type, int64_t n, int64_t m, int sms) {
     const int64_t row_blocks = (n + BQ_ROWS - 1) / BQ_ROWS;
     const int nc = b32_columns(row_blocks, m, sms);
-    const double here = b32_waves(row_blocks, m, nc, sms) * (nc == 128 ? BQ_WAVE_128 : BQ_WAVE_64) * (double)(k / 32) + BQ_EXPAND;
-    return here < b32_waves(row_blocks, m, 32, sms) * (type == B200_TYPE_MXFP4 ? BQ_WAVE_I8_MXFP4 : BQ_WAVE_I8) * (double)(k / 32) ? nc : 0;
+    const int64_t here = b32_waves(row_blocks, m, nc, sms) * (nc == 128 ? BQ_WAVE_128 : BQ_WAVE_64);
+    return here < b32_waves(row_blocks, m, 32, sms) * (type == B200_TYPE_MXFP4 ? BQ_WAVE_I8_MXFP4 : BQ_WAVE_I8) ? nc : 0;
 }
-bool gemm_b32_wins(int type, int64_t n, int64_t k, int64_t m) { return gemm_b32_pick_for(type, n, k, m, sm_count()) != 0; }
+bool gemm_b32_wins(int type, int64_t n, int64_t m) { return gemm_b32_pick_for(type, n, m, sm_count()) != 0; }
 
 // Q8_0 (fast numerics), Q4_0 and MXFP4 (8x8 gemm chain) mat-muls
-int launch_gemm_b32(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst, cudaStream_t s) {
+int launch_gemm_b32(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActF16 acts, float *dst, int64_t lddst, cudaStream_t s) {
     B200_REQUIRE(k % GROUP_K == 0, "gemm: k = %lld must be a multiple of 256", (long long)k);
     if (n == 0 || m == 0) return B200_STATUS_SUCCESS;
     const int64_t row_blocks = (n + BQ_ROWS - 1) / BQ_ROWS;
     const int sms = sm_count(), nc = b32_columns(row_blocks, m, sms);
     BqCall c = {};
-    c.n = n; c.k = k; c.m = m; c.tiles = tiles; c.dst = dst; c.lddst = lddst;
+    c.n = n; c.k = k; c.m = m; c.tiles = tiles; c.dst = dst; c.lddst = lddst; c.acts = acts;
     c.row_blocks = row_blocks;
     c.col_blocks = (m + nc - 1) / nc;
-    B200_REQUIRE(c.row_blocks * c.col_blocks < (1ll << 31) - (1 << 20) && k / 128 <= 65535, "gemm: %lld x %lld is too large for one launch", (long long)n, (long long)m);
-    const int64_t ld_scale = c.col_blocks * nc;
-    const size_t x_bytes = ((size_t)m * k * 2 + 255) / 256 * 256;
-    void *block = nullptr;
-    int rc = scratch_get_images(x_bytes + (size_t)(k / 32) * ld_scale * 4, &block);
-    if (rc != B200_STATUS_SUCCESS) return rc;
-    __half *x = (__half *)block;
-    float *scales = (float *)((uint8_t *)block + x_bytes);
-    c.x = x;
-    c.scales = scales;
-    rc = launch_pdl(expand_q8_0_acts_kernel, dim3((unsigned)((ld_scale + 31) / 32), (unsigned)(k / 128)), dim3(256), (size_t)0, s, acts, x, scales, ld_scale, m);
-    if (rc != B200_STATUS_SUCCESS) return rc;
+    B200_REQUIRE(c.row_blocks * c.col_blocks < (1ll << 31) - (1 << 20), "gemm: %lld x %lld is too large for one launch", (long long)n, (long long)m);
+    B200_REQUIRE(acts.x && acts.ld >= c.col_blocks * nc, "gemm: no f16 activations for %lld rows", (long long)m);
     switch (type) {
         case B200_TYPE_Q8_0: return launch_b32_nc<B200_TYPE_Q8_0>(nc, c, sms, s);
         case B200_TYPE_Q4_0: return launch_b32_nc<B200_TYPE_Q4_0>(nc, c, sms, s);

@@ -1,4 +1,4 @@
-// Few waves of 32-row tiles of the 32-element-block types (gemm_b32_tcgen05.cu takes over beyond), MUL_MAT_ID, calls without scratch memory, and
+// Few waves of 32-row tiles of the 32-element-block types (gemm_b32_tcgen05.cu takes over beyond), MUL_MAT_ID, calls without f16 activations, and
 // Q6_K on request.
 // Prompt-shaped mat-mul for Q8_0, Q4_0, MXFP4 and Q6_K weights on the fifth-generation tensor cores: tcgen05.mma
 // kind::i8 with the block dots accumulated in tensor memory.  Same pipeline as the Q4_K kernel of gemm_tcgen05.cu

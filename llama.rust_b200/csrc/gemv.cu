@@ -884,7 +884,7 @@ bool gemv_rows_add_fusable(int type, int route, int64_t m) {
 // where each of them would take it by itself (the same kernel and tolerance; its CTAs cut the tiles' f32 sums in other
 // places than separate launches would), separate launches otherwise.
 int launch_gemv_rows_multi(int type, int route, int count, const int64_t *n, int64_t k, int64_t m, const uint8_t *const *tiles, ActView acts, float *const *dst,
-                           const int64_t *lddst, cudaStream_t s) {
+                           const int64_t *lddst, cudaStream_t s, ActF16 f16) {
     const char *fe = getenv("B200_GEMM_FAST");
     const bool whole = route == B200_ROUTE_TILED || (route == B200_ROUTE_REPACK && m % 4 == 0);   // no tail rows on another chain
     int64_t rows = 0;
@@ -898,14 +898,21 @@ int launch_gemv_rows_multi(int type, int route, int count, const int64_t *n, int
         gemm_small_multi_enabled())
         return launch_gemm_small_multi(count, n, k, m, tiles, acts, dst, lddst, s);
     for (int e = 0; e < count; e++) {
-        int rc = launch_gemv(type, route, n[e], k, m, tiles[e], acts, dst[e], lddst[e], s);
+        int rc = launch_gemv(type, route, n[e], k, m, tiles[e], acts, dst[e], lddst[e], s, f16);
         if (rc != B200_STATUS_SUCCESS) return rc;
     }
     return B200_STATUS_SUCCESS;
 }
 
+// 32-element-block types on a route whose chain (Q8_0: whose tolerance) the tcgen05 kernels keep
+static bool block32_on_tcgen05(int type, int route, int64_t m) {
+    return m >= GEMM_MMA_MIN_COLS && gemm_tcgen05_enabled() && gemm_mma_enabled() &&
+           (((type == B200_TYPE_Q4_0 || type == B200_TYPE_MXFP4) && route == B200_ROUTE_REPACK) || (type == B200_TYPE_Q8_0 && route == B200_ROUTE_ROWDOT && numerics_mode() == 1));
+}
+bool gemv_wants_f16_acts(int type, int route, int64_t n, int64_t m) { return block32_on_tcgen05(type, route, m) && gemm_b32_wins(type, n, m); }
+
 int launch_gemv(int type, int route, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst,
-                int64_t lddst, cudaStream_t s) {
+                int64_t lddst, cudaStream_t s, ActF16 f16) {
     B200_REQUIRE(k % GROUP_K == 0, "gemv: k = %lld must be a multiple of 256", (long long)k);
     const int nb = (int)(k / GROUP_K);
     // the bulk-copy streaming kernel wins while every CTA has at most one row tile (no second wave to
@@ -984,9 +991,8 @@ int launch_gemv(int type, int route, int64_t n, int64_t k, int64_t m, const uint
             const char *e = getenv("B200_Q6K_TCGEN05");
             if (e && e[0] == '1') return launch_gemm_tcgen05_i8(type, n, k, m, tiles, acts, dst, lddst, s);
         }
-        const bool b32 = ((type == B200_TYPE_Q4_0 || type == B200_TYPE_MXFP4) && route == B200_ROUTE_REPACK) || (type == B200_TYPE_Q8_0 && route == B200_ROUTE_ROWDOT && numerics_mode() == 1);
-        if (b32 && m >= GEMM_MMA_MIN_COLS)
-            return !no_scratch_mode() && gemm_b32_wins(type, n, k, m) ? launch_gemm_b32(type, n, k, m, tiles, acts, dst, lddst, s) : launch_gemm_tcgen05_i8(type, n, k, m, tiles, acts, dst, lddst, s);
+        if (block32_on_tcgen05(type, route, m))
+            return f16.x && gemm_b32_wins(type, n, m) ? launch_gemm_b32(type, n, k, m, tiles, f16, dst, lddst, s) : launch_gemm_tcgen05_i8(type, n, k, m, tiles, acts, dst, lddst, s);
     }
     if (type == B200_TYPE_Q6_K && route == B200_ROUTE_TILED && m >= GEMM_MMA_MIN_COLS && gemm_mma_enabled())
         return launch_gemm_mma(6, n, k, m, tiles, acts, dst, lddst, s);

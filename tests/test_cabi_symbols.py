@@ -69,12 +69,12 @@ def test_block32_kernel_choice_follows_waves():
     lib = ctypes.CDLL(b200.load().LIB_PATH)
     f = lib.b200_block32_kernel_choice
     f.restype = ctypes.c_int
-    f.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_int]
+    f.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int]
     q8_0, q4_0, mxfp4 = 8, 2, 39
     for ty in (q8_0, q4_0, mxfp4):
-        assert f(ty, 4096, 4096, 32, 148) == 0 and f(ty, 1024, 2048, 300, 148) == 0    # one wave of the integer kernel
-        assert f(ty, 14336, 4096, 512, 148) == 128 and f(ty, 2056, 4096, 300, 148) == 64
-    assert f(12, 4096, 4096, 512, 148) == -1 and f(q8_0, 4096, 100, 512, 148) == -1 and f(q8_0, 4096, 4096, 512, 0) == -1
+        assert f(ty, 4096, 32, 148) == 0 and f(ty, 1024, 300, 148) == 0    # one wave of the integer kernel
+        assert f(ty, 14336, 512, 148) == 128 and f(ty, 2056, 300, 148) == 64
+    assert f(12, 4096, 512, 148) == -1 and f(q8_0, 4096, 512, 0) == -1
 
 
 def test_rows_add_fusable_is_host_arithmetic():

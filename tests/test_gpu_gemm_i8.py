@@ -6,6 +6,9 @@ numerics mode: it adds whole 32-element block dots where the CPU route adds eigh
 the mat-mul tolerance instead, defined as the reference defines it (crates/ggml/src/compute.rs:7467-7577):
 |got - ref| <= 1e-5 * sum_k |w_k x_k| per output element."""
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -53,7 +56,7 @@ MANY_ROWS = [(2056, 4096, 300, 64), (2000, 2048, 705, 128), (4728, 2816, 193, 64
 @pytest.mark.parametrize("ty", [orc.Q4_0, orc.MXFP4, orc.Q8_0], ids=lambda t: orc.TYPE_NAMES[t])
 def test_many_rows(dev, ty, shape):
     n, k, m, columns = shape
-    assert dev.lib.b200_block32_kernel_choice(ty, C.c_int64(n), C.c_int64(k), C.c_int64(m), 148) == columns
+    assert dev.lib.b200_block32_kernel_choice(ty, C.c_int64(n), C.c_int64(m), 148) == columns
     period, ld = 504, n + 8   # rows of the result farther apart than its length
     W = synth.weights(ty, n, k, seed=420 + ty, period=period)
     x = synth.activations(m, k, seed=421 + m)
@@ -80,6 +83,116 @@ def test_many_rows(dev, ty, shape):
     bound = 1e-5 * (np.abs(x).astype(np.float64) @ np.abs(orc.dequantize(ty, W[:period], k)).astype(np.float64).T)
     bound = np.tile(bound, (1, (n + period - 1) // period))[:, :n]
     assert (np.abs(got.astype(np.float64) - want.astype(np.float64)) <= bound).all()
+
+
+def own_block(dev, m, k):
+    """a caller's activation block, 256-byte aligned"""
+    buf = dev.DeviceBuffer(dev.lib.b200_act_scratch_nbytes(m, k) + 256)
+    return buf, (buf.ptr + 255) // 256 * 256
+
+
+@pytest.mark.parametrize("ty", [orc.MXFP4, orc.Q8_0], ids=lambda t: orc.TYPE_NAMES[t])
+def test_callers_with_blocks_of_their_own_share_nothing(dev, ty):
+    """two streams, each with its activation block, mat-muls side by side; a captured call replayed after larger ones"""
+    import torch
+    n, k, m, rounds = 14344, 1024, 509, 12
+    assert dev.lib.b200_block32_kernel_choice(ty, C.c_int64(n), C.c_int64(m), 148) == 128
+    w = dev.Weight(ty, synth.weights(ty, n, k, seed=440, period=504), k)
+    dev.set_numerics(dev.FAST)
+    try:
+        jobs = []
+        for i in range(2):
+            x = synth.activations(m, k, seed=441 + i)
+            buf, act = own_block(dev, m, k)
+            jobs.append((dev.device_array(x), buf, act, dev.DeviceBuffer(4 * m * n), torch.cuda.Stream()))
+
+        def call(job, stream):
+            dx, _, act, out, _ = job
+            dev.check(dev.lib.b200_quantize_activations_device(dev.ACT_Q8_0, m, k, dx.ptr, k, act, stream), "quantize")
+            dev.check(dev.lib.b200_mul_mat_q8(ty, n, k, m, w.ptr, act, dev.ACT_Q8_0, out.ptr, n, 0, stream), "mul_mat_q8")
+
+        want = []
+        for job in jobs:
+            call(job, None)
+            want.append(job[3].download(np.uint32, m * n))
+        torch.cuda.synchronize()
+        before = int(dev.lib.b200_debug_alloc_count())
+        for _ in range(rounds):
+            for job in jobs:
+                call(job, job[4].cuda_stream)
+        torch.cuda.synchronize()
+        assert int(dev.lib.b200_debug_alloc_count()) == before
+        for job, bits in zip(jobs, want):
+            assert np.array_equal(job[3].download(np.uint32, m * n), bits)
+
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=jobs[0][4]):
+            call(jobs[0], jobs[0][4].cuda_stream)
+        big = dev.device_array(synth.activations(4 * m, k, seed=443))
+        out = dev.DeviceBuffer(4 * 4 * m * n)
+        dev.check(dev.lib.b200_mul_mat(ty, n, k, 4 * m, w.ptr, big.ptr, k, out.ptr, n, 0, None), "mul_mat")
+        torch.cuda.synchronize()
+        dev.check(dev.lib.b200_memset(jobs[0][3].ptr, 0, 4 * m * n, None), "memset")
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(jobs[0][3].download(np.uint32, m * n), want[0])
+        assert dev.kernel_error() == 0
+    finally:
+        dev.set_numerics(dev.EXACT)
+
+
+OWNED_CHILD = r"""
+import b200, orc, synth
+dev = b200.load()
+dev.set_device(0)
+dev.set_numerics(dev.FAST)
+n, k, m = 14344, 1024, 509
+for ty in (orc.Q8_0, orc.Q4_0, orc.MXFP4):
+    w, x = dev.Weight(ty, synth.weights(ty, n, k, seed=440, period=504), k), dev.device_array(synth.activations(m, k, seed=441))
+    buf, out = dev.DeviceBuffer(dev.lib.b200_act_scratch_nbytes(m, k) + 256), dev.DeviceBuffer(4 * m * n)
+    act = (buf.ptr + 255) // 256 * 256
+    dev.check(dev.lib.b200_quantize_activations_device(dev.ACT_Q8_0, m, k, x.ptr, k, act, None), "quantize")
+    dev.check(dev.lib.b200_mul_mat_q8(ty, n, k, m, w.ptr, act, dev.ACT_Q8_0, out.ptr, n, 0, None), "mul_mat_q8")
+    dev.synchronize()
+print("ALLOCATED", int(dev.lib.b200_debug_alloc_count()), dev.kernel_error())
+"""
+
+
+def test_callers_blocks_are_all_the_memory_there_is(dev):
+    """in a process whose first mat-muls these are, the library allocates nothing of its own"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    r = subprocess.run([sys.executable, "-c", OWNED_CHILD], capture_output=True, text=True, cwd=here, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert r.stdout.split()[-3:] == ["ALLOCATED", "0", "0"], r.stdout
+
+
+@pytest.mark.parametrize("kind_rows", [33, 64, 130])
+@pytest.mark.parametrize("ldx_extra", [0, 3])
+def test_quantized_rows_and_their_f16_form(dev, kind_rows, ldx_extra):
+    """what the f16 kernel reads: the quantizer's values (held to the oracle's elsewhere) as f16 in the order 0 2 1 3 4 6 5 7 of each 8, scales by block, zero past the last row"""
+    m, k = kind_rows, 768
+    x = synth.activations(m, k + ldx_extra, seed=450 + m)
+    x[1] = 0.0
+    x[2, :64] *= 1e30
+    x[3, 7] = np.nan
+    x[4, 5] = np.inf
+    buf, act = own_block(dev, m, k)
+    dx = dev.device_array(x)
+    dev.check(dev.lib.b200_quantize_activations_device(dev.ACT_Q8_0, m, k, dx.ptr, k + ldx_extra, act, None), "quantize")
+    raw = buf.download(np.uint8, buf.nbytes)[act - buf.ptr:]
+    blocks = np.frombuffer(dev.quantize_activations(dev.ACT_Q8_0, np.ascontiguousarray(x[:, :k])).tobytes(), np.uint8).reshape(m, k // 32, 34)
+    quants = blocks[..., 2:].copy().view(np.int8).reshape(m, k)
+    scales = blocks[..., :2].copy().view(np.float16).reshape(m, k // 32).astype(np.float32)
+    assert np.array_equal(raw[:m * k].view(np.int8).reshape(m, k), quants)
+    up = lambda v: (v + 255) // 256 * 256
+    at = up(m * k) + up(m * (k // 256) * 4) + up(m * (k // 16) * 2) + up(m * (k // 32) * 2)
+    order = np.array([0, 2, 1, 3, 4, 6, 5, 7])
+    assert np.array_equal(raw[at:at + 2 * m * k].view(np.float16).reshape(m, k // 8, 8), quants.reshape(m, k // 8, 8)[..., order].astype(np.float16))
+    at += up(2 * m * k)
+    ld = (m + 127) // 128 * 128
+    got = raw[at:at + 4 * ld * (k // 32)].view(np.float32).reshape(k // 32, ld)
+    assert np.array_equal(got[:, :m].view(np.uint32), np.ascontiguousarray(scales.T).view(np.uint32)) and not got[:, m:].any()
 
 
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
