@@ -122,6 +122,9 @@ int b200_prompt_kernel_choice(int64_t n, int64_t m, int sm_count);
 /* The same for Q4_0, Q8_0 (fast numerics) and MXFP4 mat-muls of 8 and more activation rows: 0 = integer tcgen05 kernel, 64 / 128 = the f16
  * tcgen05 kernel with that many activation rows per tile (both give the same bits); -1 = bad arguments. */
 int b200_block32_kernel_choice(int type, int64_t n, int64_t m, int sm_count);
+/* The same for BF16 mat-muls of more than 16 activation rows: 64 / 128 / 256 = tiles of 128 weight rows and that many activation rows, 2 = tiles
+ * of 256 x 256 by pairs of SMs; -1 = bad arguments. */
+int b200_bf16_kernel_choice(int64_t n, int64_t k, int64_t m, int sm_count);
 
 /* ---- device memory (cudaMalloc-backed; buffers of the backend use the same) */
 int b200_malloc(void **dev_ptr, size_t bytes);

@@ -280,6 +280,7 @@ struct DenseMm {
 };
 int launch_dense_mm(const DenseMm &d, cudaStream_t s);
 bool gemm_bf16_takes(const DenseMm &d);                         // gemm_bf16_tcgen05.cu
+int gemm_bf16_pick_for(int64_t n, int64_t k, int64_t m, int sms);
 int launch_gemm_bf16(const DenseMm &d, cudaStream_t s);
 // weighted RMS norm of F32 rows into F32 or BF16 rows; rows of a table by index times a factor (dense_mm.cu)
 int launch_rms_norm_w(const float *x, int64_t ldx, const float *w, void *y, int y_type, int64_t ldy, int64_t ne0, int64_t nrows, float eps, cudaStream_t s);

@@ -1,7 +1,7 @@
 // BF16 x BF16 mat-mul on the tensor cores for many activation rows: y[m][n] = act(w[n][k] x[m][k] + bias) + addend, F32 sums.
 //
-// Output tiles of 128 weight rows x NC activation rows (64 or 128), or of 256 x 256 by pairs of CTAs (further down), walked by persistent CTAs, one per SM, the column blocks of a
-// weight row block next to each other so that the weights cross HBM once.  Per tile a pipeline of K = 64 steps: one thread moves the
+// Output tiles of 128 weight rows x NC activation rows (64, 128 or 256), or of 256 x 256 by pairs of CTAs (further down), walked by persistent
+// CTAs, one per SM, the column blocks of a weight row block next to each other so that the weights cross HBM once.  Per tile a pipeline of K = 64 steps: one thread moves the
 // two operand boxes with TMA (128-byte swizzle; the hardware fills what lies outside either matrix with zeros), one thread issues four
 // M 128 x N NC x K 16 MMAs per step into one of two tensor-memory stages, four warps drain the other stage: lane = weight row, so a
 // store of one activation row's 32 outputs is one contiguous piece.  The activation function and the residual add are done there;
@@ -45,7 +45,7 @@ constexpr int GB_ERR_WAIT = 4;
 template <int NC>
 struct GbCfg {
     static constexpr int A_BYTES = GB_ROWS * GB_K * 2, B_BYTES = NC * GB_K * 2, STAGE = A_BYTES + B_BYTES;
-    static constexpr int STAGES = NC == 128 ? 6 : 8;
+    static constexpr int STAGES = NC == 256 ? 4 : NC == 128 ? 6 : 8;
     static constexpr int SMEM = STAGES * STAGE + 1024;
     // kind::f16 instruction descriptor: F32 accumulator, BF16 x BF16, both operands K-major, N = NC, M = 128
     static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(GB_ROWS >> 4) << 24);
@@ -265,7 +265,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = rb * GB_ROWS + 32 * q + lane, col0 = cb * NC;
             const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(ts * NC);
-gb_drain(o, trow, row, col0, 0, NC, [&] {
+            gb_drain(o, trow, row, col0, 0, NC, [&] {
                 if (lane == 0) gb_bar_arrive(gb_smem(&bars.tempty[ts]));
             });
         }
@@ -494,15 +494,32 @@ bool gemm_bf16_takes(const DenseMm &d) {
            d.n < (1ll << 31) - 256 && d.m < (1ll << 31) - 256 && d.norm_w == nullptr;
 }
 
+// Which form takes n weight rows x m activation rows: the activation rows of a CTA's tile (64, 128, 256), or 2 for pairs.  Each form by its waves
+// times what one takes: a 128 x 128 tile as 5 per element of K, a pair's 256 x 256 one 6 (half the MMA time of its four quarters and as many
+// copies as one of them), a 128 x 256 one 7; with short rows the drain (800 elements' worth; four warps over 256 columns 1100).  us as 128 x 128,
+// 128 x 256 and pairs, waves in brackets, K 4096: 11008 x 300 rows 45 (2), 54 (2), 48 (2); 4096 x 2048 85 (4), 55 (2), 50 (2); K 2048: 6272 x 700 27 (2),
+// 20 (1), 28 (2); 8192 x 2048 77 (7), 61 (4), 55 (4); K 512: 6272 x 3000 37 (8), 35 (4), 32 (5).
+// A pair also starts a microsecond later (cluster, tensor memory of both SMs), which one wave of short rows and a column block filled to
+// 160 of its 256 rows at most does not make up: 12288 x 2048 on 140 rows 16.7, 17.3 as pairs; on 192 17.9, 17.7; 12288 x 4096 on 140 31.1, 28.8
+int gemm_bf16_pick_for(int64_t n, int64_t k, int64_t m, int sms) {
+    if (m <= 64) return 64;
+    if (m <= 128) return 128;
+    const auto waves = [&](int64_t rows, int64_t cols, int64_t at_once) { return (((n + rows - 1) / rows) * ((m + cols - 1) / cols) + at_once - 1) / at_once; };
+    const int64_t w128 = waves(GB_ROWS, 128, sms), w256 = waves(GB_ROWS, 256, sms), wp = sms > 1 ? waves(2 * GB_ROWS, GP_NC, sms / 2) : INT32_MAX;
+    if (w128 > 1 && w256 == 1 && wp == 1 && m <= 160 && k <= 2048) return 256;
+    const int64_t short_k = k < 800 ? 800 : k, t128 = 5 * w128 * short_k, t256 = 7 * w256 * (k < 1100 ? 1100 : k), tp = 6 * wp * short_k;
+    return t128 <= t256 && t128 <= tp ? 128 : tp <= t256 ? 2 : 256;
+}
+
 int launch_gemm_bf16(const DenseMm &d, cudaStream_t s) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    if (d.m <= 64) return launch_nc<64>(d, sms, s);
-    // A 128 x 128 tile of one CTA takes nearly as long as a 256 x 256 tile of a pair (half the MMA time, but as many copies), so the pairs pay
-    // once the small tiles would need a second wave: 6144 x 4096 x 512 rows (192 small tiles) 46.5 -> 30.7 us, 2048 x 2048 x 2048 (256) 28.2 ->
-    // 19.3; in one wave they only add their start: 4096 x 4096 x 512 (128) 27.3 -> 28.3, 300 x 264 x 300 (9) 7.8 -> 9.6
-    const int64_t small = (d.n + GB_ROWS - 1) / GB_ROWS * ((d.m + 127) / 128);
-    return d.m <= 128 || small <= sms ? launch_nc<128>(d, sms, s) : launch_pair(d, sms, s);
+    switch (gemm_bf16_pick_for(d.n, d.k, d.m, sms)) {
+        case 64: return launch_nc<64>(d, sms, s);
+        case 128: return launch_nc<128>(d, sms, s);
+        case 256: return launch_nc<256>(d, sms, s);
+        default: return launch_pair(d, sms, s);
+    }
 }
 
 }  // namespace b200

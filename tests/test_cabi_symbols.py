@@ -77,6 +77,23 @@ def test_block32_kernel_choice_follows_waves():
     assert f(12, 4096, 512, 148) == -1 and f(q8_0, 4096, 512, 0) == -1
 
 
+def test_bf16_kernel_choice_counts_every_forms_waves():
+    """host arithmetic only: which form a BF16 mat-mul takes on 148 SMs.  Pairs need twice the SMs of a tile, so that their waves have
+    to be counted like the others': with as many waves as 128 x 128 tiles they lose, and where 128 x 256 tiles save one these win"""
+    lib = ctypes.CDLL(b200.load().LIB_PATH)
+    f = lib.b200_bf16_kernel_choice
+    f.restype = ctypes.c_int
+    f.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_int]
+    assert f(4096, 4096, 64, 148) == 64 and f(32000, 4096, 128, 148) == 128
+    for n, k, m in ((4096, 4096, 1100), (11008, 4096, 300), (10240, 4096, 300), (5120, 5120, 800), (4096, 4096, 512), (300, 264, 300)):
+        assert f(n, k, m, 148) == 128, (n, k, m)
+    for n, k, m in ((6272, 2048, 700), (4736, 2048, 1000), (14336, 1024, 129), (12288, 2048, 160)):
+        assert f(n, k, m, 148) == 256, (n, k, m)
+    for n, k, m in ((8192, 2048, 2048), (14336, 4096, 2048), (6144, 4096, 512), (22016, 4096, 2048), (12288, 4096, 140), (14336, 1024, 192), (6272, 512, 3000)):
+        assert f(n, k, m, 148) == 2, (n, k, m)
+    assert f(4096, 4096, 4096, 1) in (128, 256) and f(0, 64, 64, 148) == -1 and f(64, 64, 64, 0) == -1
+
+
 def test_rows_add_fusable_is_host_arithmetic():
     """which (weight type, weight rows, activation rows) the few-rows kernels take with the residual add inside: 8 to 31 rows,
     Q4_K on the 8x8 route with whole groups of four rows, or Q6_K on the tiled route; answered without a device"""

@@ -29,6 +29,13 @@ def sess(lib):
     s.close()
 
 
+@pytest.fixture
+def big_sess(lib):
+    s = gp.Session(*lib, buffer_bytes=1 << 30)
+    yield s
+    s.close()
+
+
 def put(s, arr, ty=gp.F32):
     """rows of arr (last dimension first in ne) as a tensor of the type"""
     arr = np.ascontiguousarray(arr)
@@ -78,7 +85,7 @@ def test_dense_mat_mul(sess, n, k, m, wt, xt, yt):
 
 @pytest.mark.parametrize("m", [255, 513, 2048])
 def test_wide_tiles(sess, m):
-    """enough tiles that the 256-column form is taken, ragged on both sides"""
+    """one CTA's 128 x 128 tiles in one wave (255), pairs in one wave and in two; ragged on both sides"""
     n, k = 4096 + 60, 264
     rng = np.random.default_rng(m)
     w, x = M.bf16(rng.standard_normal((n, k))), M.bf16(rng.standard_normal((m, k)))
@@ -88,12 +95,22 @@ def test_wide_tiles(sess, m):
     assert np.abs(get(sess, y) - want).max() < 1e-4
 
 
-@pytest.mark.parametrize("n,k,m", [(1290, 8, 1920), (20 * 256, 64, 897), (38 * 128 + 2, 200, 513), (149 * 128, 1032, 129)])
-def test_tiles_of_pairs(sess, n, k, m):
-    """more 128 x 128 tiles than SMs: two CTAs share a tile of 256 x 256; every epilogue, ragged on all sides"""
+# (weight rows, K, activation rows, form: 2 = pairs of CTAs with tiles of 256 x 256, else a CTA's activation rows, elements between one row's
+# end and the next row).  From three tiles on a CTA or pair reuses its accumulators: 369 tiles for 74 pairs, 441 for 148 CTAs
+TILES = [(1290, 8, 1920, 2, 0), (20 * 256, 64, 897, 2, 8), (38 * 128 + 2, 200, 513, 2, 0), (149 * 128, 1032, 129, 2, 0), (10250, 72, 2049, 2, 0), (10250, 1032, 2049, 2, 24),
+         (4090, 1208, 1100, 128, 0), (6266, 1208, 2293, 256, 8), (12290, 264, 131, 256, 0)]
+
+
+@pytest.mark.parametrize("n,k,m,form,pad", TILES)
+def test_tiles_of_pairs(big_sess, n, k, m, form, pad):
+    """more 128 x 128 tiles than SMs: two CTAs share a tile of 256 x 256, or a CTA takes several; every epilogue, ragged on all sides"""
+    sess = big_sess
+    assert b200.load().lib.b200_bf16_kernel_choice(C.c_int64(n), C.c_int64(k), C.c_int64(m), 148) == form
     rng = np.random.default_rng(n)
     w, x, add, bias = M.bf16(rng.standard_normal((n, k))), M.bf16(rng.standard_normal((m, k))), rng.standard_normal((m, n)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
-    tw, tx, ta, tb = put(sess, w, gp.BF16), put(sess, x, gp.BF16), put(sess, add), put(sess, bias)
+    tw, tx = (put(sess, np.pad(a, ((0, 0), (0, pad)), constant_values=1e30), gp.BF16) for a in (w, x))
+    ta, tb = put(sess, add), put(sess, bias)
+    tw.ne[0] = tx.ne[0] = k   # rows farther apart than they are long: nothing reads what lies between
     plain = x.astype(np.float64) @ w.T.astype(np.float64)
     scale = np.abs(x.astype(np.float64)) @ np.abs(w.T.astype(np.float64)) + 1.0
     for act, addend, yt in ((0, None, gp.F32), (1, ta, gp.F32), (0, None, gp.BF16)):
