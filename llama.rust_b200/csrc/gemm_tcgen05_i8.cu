@@ -474,26 +474,36 @@ int launch_i8(int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView act
                       dst, lddst, n, nb, m, err, gm);
 }
 
-// MUL_MAT_ID's work items, by one CTA: the (token, slot) pairs counted per expert, the experts' items (nc pairs each) laid out one after the other,
+// MUL_MAT_ID's work items, by one CTA: the (token, slot) pairs counted per expert, the experts' items (TI_COLS pairs each) laid out one after the other,
 // and every pair put in the next free column of its expert's items (which one does not matter: an output depends on its own pair only).  Pairs
 // whose id is out of range are skipped, as the per-pair kernels skip them.  Counters in shared memory, or (many experts) in global memory.
 // Latency is all there is to it: in place of a memset and three launches (27 us of kernels, one thread planning) the whole MUL_MAT_ID of 128 Q4_0
-// experts (768 x 2048) went 153 -> 138 us on 512 tokens of 8 experts, 29 -> 20 on 40 tokens of 2 (256 x 512)
-constexpr int MP_THREADS = 1024, MP_SHARED_EXPERTS = 5120;
-__global__ void __launch_bounds__(MP_THREADS) mmid_items_kernel(const int32_t *ids, int n_pairs, int n_ids, int ne11, int n_expert, int nc, int *global_counts, int *n_items,
+// experts (768 x 2048) went 153 -> 138 us on 512 tokens of 8 experts, 29 -> 20 on 40 tokens of 2 (256 x 512).  A thread has MP_BATCH ids on their
+// way: with one at a time, many pairs took longer than by those launches (Q4_0, 8192 tokens of 8 among 128 experts, 256 x 512: 290 us by launches,
+// 304, now 282; 65535 tokens of 8 among 32, 64 x 256: 1185, 1288, 1114)
+constexpr int MP_THREADS = 1024, MP_SHARED_EXPERTS = 5120, MP_BATCH = 8;
+__global__ void __launch_bounds__(MP_THREADS) mmid_items_kernel(const int32_t *ids, int n_pairs, int n_ids, int ne11, int n_expert, int *global_counts, int *n_items,
                                                                 int *work_expert, int *col_act, int *col_out) {
+    constexpr int nc = TI_COLS;
     extern __shared__ int mp_counts[];
     __shared__ int part[MP_THREADS / 32];
     pdl_trigger();
     pdl_wait();
     int *first = global_counts ? global_counts : mp_counts, *cursor = first + n_expert;   // cursor: pairs counted, then columns given out
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const auto each_pair = [&](auto &&take) {   // take(pair, expert), in no order
+        for (int i0 = tid; i0 < n_pairs; i0 += MP_BATCH * MP_THREADS) {
+            int e[MP_BATCH];
+#pragma unroll
+            for (int j = 0; j < MP_BATCH; j++) e[j] = i0 + j * MP_THREADS < n_pairs ? ids[i0 + j * MP_THREADS] : -1;
+#pragma unroll
+            for (int j = 0; j < MP_BATCH; j++)
+                if (e[j] >= 0 && e[j] < n_expert) take(i0 + j * MP_THREADS, e[j]);
+        }
+    };
     for (int e = tid; e < n_expert; e += MP_THREADS) cursor[e] = 0;
     __syncthreads();
-    for (int i = tid; i < n_pairs; i += MP_THREADS) {
-        const int e = ids[i];
-        if (e >= 0 && e < n_expert) atomicAdd(&cursor[e], 1);
-    }
+    each_pair([&](int, int e) { atomicAdd(&cursor[e], 1); });
     __syncthreads();
     // a thread's run of experts, then the runs' first items
     const int per = (n_expert + MP_THREADS - 1) / MP_THREADS, e0 = min(tid * per, n_expert), e1 = min(e0 + per, n_expert);
@@ -536,14 +546,12 @@ __global__ void __launch_bounds__(MP_THREADS) mmid_items_kernel(const int32_t *i
     __syncthreads();
     for (int e = tid; e < n_expert; e += MP_THREADS) cursor[e] = 0;
     __syncthreads();
-    for (int i = tid; i < n_pairs; i += MP_THREADS) {
-        const int e = ids[i];
-        if (e < 0 || e >= n_expert) continue;
+    each_pair([&](int i, int e) {
         const int64_t col = (int64_t)first[e] * nc + atomicAdd(&cursor[e], 1);
         const int tok = i / n_ids, slot = i - tok * n_ids;
         col_act[col] = tok * ne11 + slot % ne11;   // crates/ggml/src/compute.rs:2124: the activation row of a slot
         col_out[col] = i;
-    }
+    });
 }
 
 }  // namespace
@@ -565,7 +573,7 @@ int launch_mul_mat_id_grouped(int type, int64_t n, int64_t k, int64_t n_expert, 
     int *counts = (int *)lists, *n_items = counts + 2 * n_expert, *work_expert = n_items + 1, *col_act = work_expert + max_items, *col_out = col_act + max_items * TI_COLS;
     const bool shared = n_expert <= MP_SHARED_EXPERTS;   // two words each: 40 KB, within what a kernel may use unasked
     int rc = launch_pdl(mmid_items_kernel, dim3(1), dim3(MP_THREADS), shared ? (size_t)n_expert * 8 : (size_t)0, s, ids, (int)n_pairs, (int)n_ids, (int)ne11, (int)n_expert,
-                        TI_COLS, shared ? (int *)nullptr : counts, n_items, work_expert, col_act, col_out);
+                        shared ? (int *)nullptr : counts, n_items, work_expert, col_act, col_out);
     if (rc != B200_STATUS_SUCCESS) return rc;
     GroupMap gm;
     gm.n_items = n_items;
