@@ -21,9 +21,11 @@
 // The activations come as f16 from their quantizer (ActF16): rows of K values, the elements of each 8 in the order 0 2 1 3 4 6 5 7 in which the
 // producers' unpacking yields them, in the block that holds the quantized rows: calls with blocks of their own share nothing.
 //
-// What bounds it: the handing over of blocks and shared memory.  A block of a 128 x 128 tile takes 820 cycles; its MMAs take 128, the drain's lanes 256
-// (a multiply and an fma per output, half of the issue slots with the producers), shared memory about 670 wavefronts (scales 290, operands of
-// the MMAs 128, weights 115, copies 64).  Tried and slower: 16 draining warps (spills at 128 columns; 64 columns 50 -> 53 us), the scales
+// What bounds it: the handing over of blocks and shared memory.  A block of a 128 x 128 tile takes 900 cycles (Q8_0, 14336 x 4096 on 512 rows); its
+// MMAs take 128, the drain's lanes 256 (a multiply and an fma per output; 53 % of the issue slots are used in all), shared memory about 610
+// wavefronts: 290 of loads (activation scales, barriers) and 120 of stores (weights) as counted, 128 for the MMAs' operands and 70 for the
+// copies as worked out.  The 128-column instances of Q8_0 and MXFP4 spill 40 and 28 bytes.  Tried and slower: 16 draining warps (far more
+// spills at 128 columns; 64 columns 50 -> 53 us), the scales
 // brought to tensor memory by an MMA with a row of ones (4096 x 4096 on 64 rows 50 -> 66 us, 14336 x 4096 on 512 263 -> 271).
 // Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device error word.
 #include <cuda_fp16.h>

@@ -284,11 +284,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
 // N 256): each holds 128 of the weight rows and half of the activation rows in its shared memory and the sums of its weight rows in its
 // tensor memory.  The even CTA's MMA thread issues for both.  Its `full` barrier counts the bytes of both CTAs' copies, its `tempty`
 // barrier the epilogue warps of both; commits are multicast to both CTAs' `empty` and `tfull` barriers.
-// What bounds it: shared memory, then power.  Per K = 16 an SM's tensor core takes 128 cycles; a CTA alone on its 128 x 256 tile reads
-// 12 KB and copies 12 KB in for it, 192 cycles at 128 bytes a cycle; a pair reads and copies 8 KB each, 128 cycles.  Against the
-// 128 x 256 tiles of single CTAs that it took the place of (us, a mat-mul alone): 8192 x 2048 x 2048 rows 62.0 -> 55.6, 14336 x 4096 x
-// 2048 188.9 -> 170.5 (1.41 PFLOP/s), 22016 x 4096 x 2048 278 -> 256.  Narrower pair tiles (N 224, 192, 160,
-// 128) took longer from 1024 x 4096 x 2048 rows up.  Two epilogue warps share a quarter of the lanes: with K = 1024 one alone would take longer than the tile's MMAs.
+// What bounds it: the tensor cores (86 % of the active cycles on 14336 x 4096 x 2048 rows) at the clock that power leaves them (1.56 of
+// 1.965 GHz there).  Why pairs: per K = 16 an SM's tensor core takes 128 cycles; a CTA alone on its 128 x 256 tile reads
+// 12 KB and copies 12 KB in for it, 192 cycles at 128 bytes a cycle; a pair reads and copies 8 KB each, 128 cycles.  Against
+// 128 x 256 tiles of single CTAs (us, a mat-mul alone): 8192 x 2048 x 2048 rows 62.0 -> 55.6, 14336 x 4096 x 2048 188.9 -> 170.5
+// (1.41 PFLOP/s), 22016 x 4096 x 2048 278 -> 256.  Narrower pair tiles (N 224, 192, 160, 128) took longer from 1024 x 4096 x 2048 rows
+// up.  Two epilogue warps share a quarter of the lanes: with K = 1024 one alone would take longer than the tile's MMAs.
 constexpr int GP_EPI_WARPS = 8, GP_THREADS = 128 + GP_EPI_WARPS * 32, GP_STAGES = 6;
 constexpr int GP_A_BYTES = GB_ROWS * GB_K * 2, GP_STAGE = 2 * GP_A_BYTES, GP_SMEM = GP_STAGES * GP_STAGE + 1024;
 constexpr int GP_NC = 256;   // activation rows of a tile, tensor-memory columns of an accumulator stage

@@ -102,8 +102,8 @@ __device__ __forceinline__ uint32_t sign_bytes(uint32_t x) {
 }
 // eight 4-bit codes -> eight signed bytes of 2 * E2M1 (crates/ggml/src/quants.rs:660): of the low nibbles and of the high ones.  Byte permutes look
 // up the values of three bits, four nibbles at a time, in a positive and a negative table; a permute that spreads sign bits makes the masks between
-// them.  15 instructions where a look-up per four separated codes took 27: 4096 x 4096 on 128 rows 46 -> 39 us (Q4_0 31), the experts above as
-// MXFP4 211 -> 176 with the work items
+// them.  15 instructions where a look-up per four separated codes took 27: 4096 x 4096 on 128 rows 46 -> 39 us (Q4_0 31); MUL_MAT_ID
+// of 128 experts (768 x 2048, 512 tokens of 8) 211 -> 176 with mmid_items_kernel
 __device__ __forceinline__ void mxfp4_values(uint32_t x, uint32_t *lo, uint32_t *hi) {
     const uint32_t s0 = x & 0x77777777u, s1 = s0 >> 16;
     const uint32_t p0 = __byte_perm(0x03020100u, 0x0c080604u, s0), p1 = __byte_perm(0x03020100u, 0x0c080604u, s1);   // nibbles 0 .. 3 and 4 .. 7
@@ -585,7 +585,7 @@ int launch_mul_mat_id_grouped(int type, int64_t n, int64_t k, int64_t n_expert, 
     return launch_i8<B200_TYPE_Q4_0>(n, k, TI_COLS, tiles, acts, dst, n, s, gm, max_items);
 }
 
-// Q8_0 (fast numerics), Q4_0, MXFP4 (8x8 gemm chain) and Q6_K (tiled chain) prompt mat-muls, 32 activation rows and up
+// Q8_0 (fast numerics), Q4_0, MXFP4 (8x8 gemm chain) and Q6_K (tiled chain) mat-muls, any number of activation rows (launch_gemv comes here from 8)
 int launch_gemm_tcgen05_i8(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst,
                            cudaStream_t s) {
     B200_REQUIRE(k % GROUP_K == 0, "gemm: k = %lld must be a multiple of 256", (long long)k);

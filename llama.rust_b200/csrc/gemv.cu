@@ -970,10 +970,10 @@ int launch_gemv(int type, int route, int64_t n, int64_t k, int64_t m, const uint
         }
         return B200_STATUS_SUCCESS;
     }
-    // 32 activation rows and up: tcgen05 int8 kernels.  Q6_K (tiled chain, on request), Q4_0 and MXFP4 (8x8 gemm chain) keep the CPU
-    // routes' bits; Q8_0's tensor-core form adds whole 32-element dots where the CPU adds eight 4-element lanes, so it
-    // serves the fast numerics mode only.  The 32-element-block types take it from 8 rows on (their only alternative
-    // re-reads the weights once per two activation rows).
+    // tcgen05 kernels.  Q4_0 and MXFP4 (8x8 gemm chain) keep the CPU route's bits; Q8_0's tensor-core form adds whole 32-element dots where
+    // the CPU adds eight 4-element lanes, so it serves the fast numerics mode only.  These types take them from 8 activation rows on (their only
+    // alternative re-reads the weights once per two rows): int8 in few tiles, f16 in many (gemm_b32_pick_for).  Q6_K: from GEMM_FAST_MIN_COLS rows
+    // under fast numerics; its int8 form (tiled chain, the CPU's bits) from GEMM_TCGEN05_MIN_COLS rows on request.
     if (gemm_tcgen05_enabled() && gemm_mma_enabled()) {
         // fast numerics: Q6_K prompt batches on the f16 tensor-core kernel with one accumulator per super-block (within 1e-5
         // of sum |w x|), from 2048 weight rows (measured with 512 activation rows: 4096 x 14336 424 -> 218 us, 14336 x 4096
