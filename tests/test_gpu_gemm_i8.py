@@ -85,6 +85,34 @@ def test_many_rows(dev, ty, shape):
     assert (np.abs(got.astype(np.float64) - want.astype(np.float64)) <= bound).all()
 
 
+@pytest.mark.parametrize("ty", [orc.Q4_0, orc.MXFP4], ids=lambda t: orc.TYPE_NAMES[t])
+def test_many_rows_of_every_code_and_far_scales(dev, ty):
+    """random codes (both zeros of E2M1 among them, rows of nothing else), scales from subnormal to near the largest, activations at the ends
+    of their range: the CPU route's bits"""
+    n, k, m, period = 14344, 256, 509, 504
+    assert dev.lib.b200_block32_kernel_choice(ty, C.c_int64(n), C.c_int64(m), 148) == 128
+    rng = np.random.default_rng(460 + ty)
+    if ty == orc.Q4_0:
+        b = rng.integers(0, 256, (period, k // 32, 18), dtype=np.uint8)
+        b[..., :2] = rng.choice(np.array([6e-8, -1e-5, 0.0, -0.0, 0.01, -0.02, 60000.0, -65504.0], np.float16), (period, k // 32)).view(np.uint8).reshape(period, k // 32, 2)
+        b[5, :, 2:], b[6, :, 2:] = 0x88, 0x00
+    else:
+        b = rng.integers(0, 256, (period, k // 32, 17), dtype=np.uint8)
+        b[..., 0] = rng.choice(np.array([0, 1, 2, 20, 118, 121, 127, 200], np.uint8), (period, k // 32))
+        b[5, :, 1:], b[6, :, 1:], b[7, :, 1:] = 0x88, 0x80, 0x08
+    W = b.reshape(period, -1)
+    x = synth.activations(m, k, seed=461)
+    x[0], x[1] = 3.0, -3.0                       # every quant 127, -127
+    x[2, ::2], x[2, 1::2] = 1e-30, -1e-30
+    x[3] *= 1e4
+    want, _ = orc.mul_mat(ty, W, x)
+    assert np.isfinite(want).all()
+    W = np.tile(W, ((n + period - 1) // period, 1))[:n]
+    got = dev.mul_mat(dev.Weight(ty, W, k), x)
+    assert dev.kernel_error() == 0
+    assert bits_equal(got, np.tile(want, (1, (n + period - 1) // period))[:, :n])
+
+
 def own_block(dev, m, k):
     """a caller's activation block, 256-byte aligned"""
     buf = dev.DeviceBuffer(dev.lib.b200_act_scratch_nbytes(m, k) + 256)
