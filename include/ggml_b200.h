@@ -97,8 +97,7 @@ unsigned long long b200_debug_decode_step_launches(void);
 /* profiling aid: the device clock (ns) at which CTA 0 of the last persistent step started and passed each of its grid
  * barriers; call after synchronizing; returns how many stamps were copied (0 where there is nothing to read) */
 int b200_debug_decode_step_times(unsigned long long *out, int n);
-/* profiling aid: with B200_FA_PREFILL_PROFILE=1 in the environment the tcgen05 prompt-attention kernel sums, for one thread
- * of each role of its first CTA, the SM clocks spent at each barrier and at work (24 counters); this reads them back */
+/* formerly a profiling aid; the prompt-attention kernel keeps no such counters: fills out[0 .. n - 1] with zeros */
 int b200_debug_fa_prefill_profile(unsigned long long *out, int n);
 /* profiling aid: with B200_GEMM_FAST_PROFILE=1 the fast-numerics Q4_K prompt mat-mul sums, for one thread of each role of its
  * first CTA, the SM clocks spent at each barrier and at work (10 counters); this reads them back and clears them */

@@ -438,7 +438,6 @@ int decode_persistent_times(unsigned long long *out, int n);
 int gemm_fast_profile(unsigned long long *out, int n);            // gemm_tcgen05_fast.cu
 void gemm_fast_debug_wait(int spin_limit, int mute_cta);          // gemm_tcgen05_fast.cu: test hook
 int gemm_fast_reset_flags();                                      // gemm_tcgen05_fast.cu: the partial-tile flags of the current device, all down
-int flash_attn_prefill_profile(unsigned long long *out, int n);   // flash_attn_prefill_tc.cu
 
 // route the reference takes for (type, n, m), and the activation quantizer that route reads
 int pick_route(int type, int64_t n, int64_t m);

@@ -589,8 +589,7 @@ int flash_attn_faithful_tiled(const b200_flash_attn_args *a, cudaStream_t s);   
 bool flash_attn_decode_head(const b200_flash_attn_args *a, int n_chunks, int64_t chunk, cudaStream_t s, int *rc);   // flash_attn_head.cu
 bool flash_attn_rows_visible(const b200_flash_attn_args *a, cudaStream_t s, int *rc);                               // flash_attn_vis.cu
 bool flash_attn_fast_rows(const b200_flash_attn_args *a, cudaStream_t s, int *rc);                                  // flash_attn_fast.cu
-bool flash_attn_fast_prefill(const b200_flash_attn_args *a, cudaStream_t s, int *rc);                               // flash_attn_prefill.cu
-bool flash_attn_fast_prefill_tc(const b200_flash_attn_args *a, cudaStream_t s, int *rc);                            // flash_attn_prefill_tc.cu
+bool flash_attn_fast_prompt(const b200_flash_attn_args *a, cudaStream_t s, int *rc);                                // flash_attn_prompt.cu
 bool flash_attn_decode_mma(const b200_flash_attn_args *a, cudaStream_t s, int *rc);                                 // flash_attn_decode_mma.cu
 
 // B200_FA_DECODE_MMA=0 keeps fast-mode attention of fewer than 64 query rows off the tensor-core flash-decoding kernel: single
@@ -599,16 +598,6 @@ bool flash_attn_decode_mma(const b200_flash_attn_args *a, cudaStream_t s, int *r
 static bool fa_decode_mma_enabled() {
     const char *e = getenv("B200_FA_DECODE_MMA");
     return !(e && e[0] == '0');
-}
-
-// B200_FA_PREFILL_TC=1 sends fast-mode prompt attention with head size 128 to the tcgen05 kernel (read per call).  It gives
-// the same values as the mma.sync kernel and, measured on 512 query rows over 32768 cached positions, the same speed
-// (1.33 against 1.31 ms): with unswizzled core-matrix operands an M 128 x N 64 x K 16 MMA takes about 127 cycles and the
-// 16-byte cp.async copies that build those operands cost their warps about 90 cycles each, so the mma.sync kernel stays
-// the default until the operands come in through tensor-map copies in the 128-byte swizzle.
-static bool fa_prefill_tc_enabled() {
-    const char *e = getenv("B200_FA_PREFILL_TC");
-    return e && e[0] == '1';
 }
 
 // B200_FA_DECODE_FUSED=0 keeps single-row attention on the three-kernel path (for side-by-side measurements)
@@ -678,14 +667,23 @@ extern "C" int b200_flash_attn_ext(const struct b200_flash_attn_args *args, void
     // than it (measured on 16 sequences over 10240 cells).
     const bool policy = args->mode == 0 && numerics_mode() == 1;
     if ((args->mode == 1 || policy) && args->n_tok < 64) {
-        if (fa_decode_mma_enabled() && flash_attn_decode_mma(args, (cudaStream_t)stream, &rc)) return rc;
+        if (fa_decode_mma_enabled()) {
+            // Two to 63 rows.  The prompt kernel computes 128 rows at a time with its positions over a cluster, the decode kernel 16 rows (whole
+            // tokens) that skip what none of them sees.  32 heads of 128 on 8 KV heads, us decode / prompt kernel: a causal batch of 16 rows
+            // over 2048 positions 22.8 / 13.1, 8192 36 / 19, 32768 95 / 44 (63 rows 344 / 60); sequences that see a 16th each 19.1 / 12.6,
+            // 22.7 / 21.9, 46 / 60 (of 63 sequences 66 / 52).  Above 8192 positions so few rows are more likely sequences than a prompt's.
+            // What the decode kernel does not take (mask rows of an odd length) is the prompt kernel's as well.
+            const bool wide = args->n_tok > 1 && (args->n_kv <= 8192 || args->n_tok >= 32);
+            if (wide && flash_attn_fast_prompt(args, (cudaStream_t)stream, &rc)) return rc;
+            if (flash_attn_decode_mma(args, (cudaStream_t)stream, &rc)) return rc;
+            if (args->n_tok > 1 && flash_attn_fast_prompt(args, (cudaStream_t)stream, &rc)) return rc;
+        }
         if ((args->mode == 1 || args->n_tok == 1) && flash_attn_fast_rows(args, (cudaStream_t)stream, &rc)) return rc;
     }
     if (args->n_tok < 64) return flash_attn_faithful_rows(args, (cudaStream_t)stream);
     // prompt batches: the tensor-core kernel under mode 1 or the fast numerics policy, the bit-exact tiled kernel otherwise
     if (args->mode == 1 || (args->mode == 0 && numerics_mode() == 1)) {
-        if (fa_prefill_tc_enabled() && flash_attn_fast_prefill_tc(args, (cudaStream_t)stream, &rc)) return rc;   // head size 128, tcgen05
-        if (flash_attn_fast_prefill(args, (cudaStream_t)stream, &rc)) return rc;
+        if (flash_attn_fast_prompt(args, (cudaStream_t)stream, &rc)) return rc;
     }
     return flash_attn_faithful_tiled(args, (cudaStream_t)stream);
 }

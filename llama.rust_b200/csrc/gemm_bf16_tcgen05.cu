@@ -35,6 +35,14 @@ int rows_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64
     B200_REQUIRE(r == CUDA_SUCCESS, "gemm: tensor map of %lld x %lld (stride %lld) refused (%d)", (long long)rows, (long long)k, (long long)ld, (int)r);
     return B200_STATUS_SUCCESS;
 }
+bool cache_tile_map(CUtensorMap *map, const void *base, int64_t d, int64_t heads, int64_t n_pos, int64_t nb1, int64_t nb2, int box_pos) {
+    encode_fn enc = tensor_map_encoder();
+    if (!enc) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)d, (cuuint64_t)heads, (cuuint64_t)n_pos}, strides[2] = {(cuuint64_t)nb2, (cuuint64_t)nb1};
+    const cuuint32_t box[3] = {64, 1, (cuuint32_t)box_pos}, es[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 namespace {
 

@@ -1,0 +1,126 @@
+"""The fast prompt-attention kernel (csrc/flash_attn_prompt.cu) where it can go wrong: edges of its 128-row blocks and 128-position tiles, positions
+over one to eight CTAs, mask rows on and off 16-byte boundaries, tiles that are clear, hidden or mixed, running maxima that grow (-m gpu).
+
+Tolerance, per output row relative to the row's largest magnitude, against float64 with q rounded to f16 (as the operation rounds it): the weights
+are rounded to f16 before the second product and in the sum alike, 2^-11 of each weight, which over a row gives at most 2 * 2^-11 = 9.8e-4
+of the largest |v|; 1e-3 as asked of F16-KV attention."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import b200
+from test_gpu_flash_attn import synth_case
+from test_gpu_flash_attn_fast import ref64, row_rel
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-3
+
+
+@pytest.fixture(scope="module")
+def dev():
+    mod = b200.load()
+    assert mod.device_count() > 0
+    mod.set_device(0)
+    return mod
+
+
+def check(dev, q, k, v, mask, scale, got=None, coarse=()):
+    """coarse: rows whose scores carry a bias of -65504 everywhere: in log2 units an F32 step there is 2^-7, so that every weight is off by up to
+    2^-8 ln 2 = 2.7e-3 of itself; 1e-2 for an output that is smaller than the values it is made of"""
+    if got is None:
+        got = dev.flash_attn(q, dev.KvCacheView(k, v), mask, scale, mode=1)
+    assert dev.kernel_error() == 0
+    live = np.ones(q.shape[1], bool) if mask is None else (mask != 0xFC00).any(axis=1)
+    assert not got[~live].any()
+    with np.errstate(invalid="ignore"):
+        want = ref64(q.astype(np.float16).astype(np.float32), k, v, mask, scale)
+    fine = live.copy()
+    fine[list(coarse)] = False
+    assert row_rel(got[fine], want[fine]) <= TOL
+    for t in coarse:
+        assert row_rel(got[t], want[t]) <= 1e-2
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("H,Hkv,T", [(4, 4, 64), (4, 2, 64), (8, 2, 33), (6, 2, 43), (16, 1, 65), (3, 1, 2)], ids=str)
+@pytest.mark.parametrize("n_kv", [127, 128, 129, 256, 777, 2050])
+def test_edges(dev, D, H, Hkv, T, n_kv):
+    """row blocks that are full, ragged, or begin inside a token; caches of less than a tile, whole tiles, a position more; the mask's rows start on
+    2-byte, 4-byte and 16-byte boundaries"""
+    q, k, v, mask = synth_case(H, Hkv, D, T, n_kv, seed=D + H * T + n_kv)
+    check(dev, q, k, v, mask, D ** -0.5)
+    if T >= 64:
+        check(dev, q, k, v, None, D ** -0.5)
+
+
+@pytest.mark.parametrize("n_kv", [1, 5])
+def test_a_cache_of_a_few_positions(dev, n_kv):
+    q, k, v, _ = synth_case(8, 2, 128, 64, n_kv, seed=n_kv, causal=False)
+    check(dev, q, k, v, None, 0.09)
+
+
+@pytest.mark.parametrize("n_kv", [1100, 1104])
+def test_masks_of_any_values(dev, n_kv):
+    """finite biases, the type's lowest value, hidden and clear tiles, rows that see nothing or only the last position"""
+    rng = np.random.default_rng(n_kv)
+    H, Hkv, D, T = 8, 4, 128, 70
+    q, k, v, _ = synth_case(H, Hkv, D, T, n_kv, seed=3, causal=False)
+    m = (rng.standard_normal((T, n_kv)) * 2).astype(np.float16)
+    m[:, 128:384] = 0.0
+    m[:, 512:768] = -np.inf
+    m[10:20, :] = np.float16(-65504.0)
+    m[10:20, 1000] = 0.0
+    m[21, :] = np.float16(-65504.0)
+    m[30:34, :] = -np.inf
+    m[40:50, :] = -np.inf
+    m[40:50, n_kv - 1] = 0.0
+    check(dev, q, k, v, m.view(np.uint16), D ** -0.5, coarse=[21])
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_maxima_that_grow_along_the_cache(dev, D):
+    """scores that rise by far more than 2^8 from tile to tile, and fall for other rows: outputs are rescaled often, or never"""
+    H, Hkv, T, n_kv = 4, 2, 100, 1500
+    q, k, v, mask = synth_case(H, Hkv, D, T, n_kv, seed=D, causal=True)
+    ramp = (np.arange(n_kv) / 100.0).astype(np.float32)
+    kf = k.view(np.float16).astype(np.float32)
+    kf[:, :, 0] = ramp
+    q[:, ::2, 0] = 8.0 * D ** 0.5
+    q[:, 1::2, 0] = -8.0 * D ** 0.5
+    check(dev, q, kf.astype(np.float16).view(np.uint16), v, mask, D ** -0.5)
+
+
+def test_a_negative_scale(dev):
+    q, k, v, mask = synth_case(8, 2, 64, 80, 900, seed=8)
+    check(dev, q, k, v, mask, -0.125)
+
+
+def test_strided_views(dev):
+    """q token-major, the cache head-major with gaps, mask rows with a stride of their own and an odd start"""
+    H, Hkv, D, T, n_kv = 8, 2, 128, 66, 530
+    q, k, v, mask = synth_case(H, Hkv, D, T, n_kv, seed=21)
+    pad = 8
+    kc = np.full((Hkv, n_kv + 3, D + pad), 0x7E00, np.uint16)   # NaN between the rows
+    vc = kc.copy()
+    kc[:, :n_kv, :D], vc[:, :n_kv, :D] = k, v
+    mc = np.zeros((T, n_kv + 7), np.uint16)
+    mc[:, 1:1 + n_kv] = mask
+    dq, dk, dv, dm = (dev.device_array(np.ascontiguousarray(x)) for x in (np.transpose(q, (1, 0, 2)), kc, vc, mc))
+    dst = dev.DeviceBuffer(4 * T * H * D)
+    a = dev.FlashAttnArgs()
+    a.dk, a.dv, a.n_tok, a.n_head, a.n_head_kv, a.n_kv = D, D, T, H, Hkv, n_kv
+    a.q, a.q_nb1, a.q_nb2 = dq.ptr, H * D * 4, D * 4
+    a.k, a.k_nb1, a.k_nb2 = dk.ptr, (D + pad) * 2, (n_kv + 3) * (D + pad) * 2
+    a.v, a.v_nb1, a.v_nb2 = dv.ptr, (D + pad) * 2, (n_kv + 3) * (D + pad) * 2
+    a.mask, a.mask_nb1 = dm.ptr + 2, (n_kv + 7) * 2
+    a.scale, a.dst, a.mode = D ** -0.5, dst.ptr, 1
+    dev.check(dev.lib.b200_flash_attn_ext(C.byref(a), None), "flash_attn_ext")
+    check(dev, q, k, v, mask, D ** -0.5, dst.download(np.float32, T * H * D).reshape(T, H, D))
+
+
+def test_few_rows_over_a_long_cache_keep_the_decode_kernel_where_it_can(dev):
+    """16 rows over more than 8192 positions: the same function whichever kernel takes them (an odd cache: the prompt kernel)"""
+    for n_kv in (8704, 8705):
+        q, k, v, mask = synth_case(8, 2, 128, 16, n_kv, seed=n_kv)
+        check(dev, q, k, v, mask, 128 ** -0.5)
