@@ -156,7 +156,7 @@ int launch_repack(int type, int64_t n_rows, int64_t k, const uint8_t *src_blocks
 int launch_dequantize(int type, int64_t n_rows, int64_t k, const uint8_t *tiles, float *out, cudaStream_t s);
 int launch_gemv(int type, int route, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts,
                 float *dst, int64_t lddst, cudaStream_t s, ActF16 f16 = ActF16{});
-bool gemv_wants_f16_acts(int type, int route, int64_t n, int64_t m);   // whether launch_gemv reads them where it is given them
+bool gemv_wants_f16_acts(int type, int route, int64_t n, int64_t k, int64_t m);   // whether launch_gemv reads them where it is given them
 
 int launch_gemm_mma(int mode, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst,
                     cudaStream_t s);
@@ -166,7 +166,11 @@ bool gemm_small_multi_enabled();
 int launch_gemm_rows_ring(int count, const int64_t *n, int64_t k, int64_t m, const uint8_t *const *tiles, ActView acts, float *const *dst,
                           const int64_t *lddst, cudaStream_t s);
 void gemm_rows_ring_debug_wait(int spin_limit, int skip_unit);
-bool gemv_rows_add_fusable(int type, int route, int64_t m);
+bool gemv_rows_add_fusable(int type, int route, int64_t n, int64_t m);
+// a few activation rows, fast numerics (gemm_few.cu)
+bool few_takes(int type, int route, int64_t n, int64_t k, int64_t m);
+bool few_takes_experts(int type, int64_t k, int64_t act_rows, int64_t n_expert, int64_t pairs);
+int launch_gemm_few(int type, int count, const int64_t *n, int64_t k, int64_t m, const uint8_t *const *tiles, ActView acts, float *const *dst, const int64_t *lddst, cudaStream_t s);
 int launch_gemm_tcgen05(int mode, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst,
                         cudaStream_t s);
 // Q8_0 / Q4_0 / MXFP4 / Q6_K prompt mat-muls on tcgen05 kind::i8 (gemm_tcgen05_i8.cu)
@@ -176,8 +180,21 @@ int launch_gemm_tcgen05_i8(int type, int64_t n, int64_t k, int64_t m, const uint
 int gemm_b32_pick_for(int type, int64_t n, int64_t m, int sms);
 bool gemm_b32_wins(int type, int64_t n, int64_t m);
 int launch_gemm_b32(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActF16 acts, float *dst, int64_t lddst, cudaStream_t s);
+// MUL_MAT_ID, grouped by expert: column block w of the mat-mul is a work item: up to 32 (token, slot) pairs routed to one
+// expert.  *n_items items are in use (the other CTAs leave at once); work_expert[w] names the expert, col_act[32 w + c] the
+// quantized activation row of column c and col_out[32 w + c] the output row (pair index), -1 for the unused columns
+// of a short item.  Null work_expert: a plain mat-mul.
+struct GroupMap {
+    const int *n_items;
+    const int *work_expert;
+    const int *col_act;
+    const int *col_out;
+    int64_t expert_bytes;
+};
+
 // MUL_MAT_ID with the pairs grouped by expert on the device (MXFP4 / Q4_0 experts on the 8x8 route): gemm_tcgen05_i8.cu
 size_t mmid_grouped_scratch_bytes(int64_t n_expert, int64_t n_pairs);
+int launch_gemm_few_grouped(int type, int64_t n, int64_t k, int64_t n_expert, int64_t pairs, int64_t act_rows, const uint8_t *tiles, ActView acts, float *dst, const GroupMap &gm, int64_t max_items, cudaStream_t s);   // gemm_few.cu
 int launch_mul_mat_id_grouped(int type, int64_t n, int64_t k, int64_t n_expert, int64_t ne11, int64_t n_tok, int64_t n_ids, const uint8_t *tiles,
                               ActView acts, const int32_t *ids, float *dst, void *lists, cudaStream_t s);
 // which Q4_K gemm-chain prompt kernel the time model prefers on a GPU of sm_count SMs: 0 integer, 3 / 4 two-pass with 64 / 128 columns
@@ -509,6 +526,24 @@ __device__ __forceinline__ float e8m0_half_to_f32(uint32_t e) {
     // 2^(e-128): crates/ggml/src/quants.rs:682-691
     uint32_t bits = e < 2 ? (0x00200000u << e) : ((e - 1) << 23);
     return __uint_as_float(bits);
+}
+// every byte's sign bit in all its bits (the selector mode that __byte_perm leaves out)
+__device__ __forceinline__ uint32_t sign_bytes(uint32_t x) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %1, 0xba98;" : "=r"(r) : "r"(x));
+    return r;
+}
+// eight 4-bit codes -> eight signed bytes of 2 * E2M1 (crates/ggml/src/quants.rs:660): of the low nibbles and of the high ones.  Byte permutes look
+// up the values of three bits, four nibbles at a time, in a positive and a negative table; a permute that spreads sign bits makes the masks between
+// them.  15 instructions where a look-up per four separated codes took 27: 4096 x 4096 on 128 rows 46 -> 39 us (Q4_0 31); MUL_MAT_ID
+// of 128 experts (768 x 2048, 512 tokens of 8) 211 -> 176 with mmid_items_kernel
+__device__ __forceinline__ void mxfp4_values(uint32_t x, uint32_t *lo, uint32_t *hi) {
+    const uint32_t s0 = x & 0x77777777u, s1 = s0 >> 16;
+    const uint32_t p0 = __byte_perm(0x03020100u, 0x0c080604u, s0), p1 = __byte_perm(0x03020100u, 0x0c080604u, s1);   // nibbles 0 .. 3 and 4 .. 7
+    const uint32_t n0 = __byte_perm(0xfdfeff00u, 0xf4f8fafcu, s0), n1 = __byte_perm(0xfdfeff00u, 0xf4f8fafcu, s1);
+    const uint32_t ml = sign_bytes(x << 4), mh = sign_bytes(x);   // 0xff where the code's sign bit is set
+    *lo = (__byte_perm(p0, p1, 0x6420) & ~ml) | (__byte_perm(n0, n1, 0x6420) & ml);
+    *hi = (__byte_perm(p0, p1, 0x7531) & ~mh) | (__byte_perm(n0, n1, 0x7531) & mh);
 }
 #endif
 

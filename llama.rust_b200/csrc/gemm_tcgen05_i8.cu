@@ -94,38 +94,8 @@ __device__ __forceinline__ void tmem_ld16(int (&v)[16], uint32_t taddr) {
                  : "memory");
 }
 
-// every byte's sign bit in all its bits (the selector mode that __byte_perm leaves out)
-__device__ __forceinline__ uint32_t sign_bytes(uint32_t x) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %1, 0xba98;" : "=r"(r) : "r"(x));
-    return r;
-}
-// eight 4-bit codes -> eight signed bytes of 2 * E2M1 (crates/ggml/src/quants.rs:660): of the low nibbles and of the high ones.  Byte permutes look
-// up the values of three bits, four nibbles at a time, in a positive and a negative table; a permute that spreads sign bits makes the masks between
-// them.  15 instructions where a look-up per four separated codes took 27: 4096 x 4096 on 128 rows 46 -> 39 us (Q4_0 31); MUL_MAT_ID
-// of 128 experts (768 x 2048, 512 tokens of 8) 211 -> 176 with mmid_items_kernel
-__device__ __forceinline__ void mxfp4_values(uint32_t x, uint32_t *lo, uint32_t *hi) {
-    const uint32_t s0 = x & 0x77777777u, s1 = s0 >> 16;
-    const uint32_t p0 = __byte_perm(0x03020100u, 0x0c080604u, s0), p1 = __byte_perm(0x03020100u, 0x0c080604u, s1);   // nibbles 0 .. 3 and 4 .. 7
-    const uint32_t n0 = __byte_perm(0xfdfeff00u, 0xf4f8fafcu, s0), n1 = __byte_perm(0xfdfeff00u, 0xf4f8fafcu, s1);
-    const uint32_t ml = sign_bytes(x << 4), mh = sign_bytes(x);   // 0xff where the code's sign bit is set
-    *lo = (__byte_perm(p0, p1, 0x6420) & ~ml) | (__byte_perm(n0, n1, 0x6420) & ml);
-    *hi = (__byte_perm(p0, p1, 0x7531) & ~mh) | (__byte_perm(n0, n1, 0x7531) & mh);
-}
 // four nibbles (one per byte) minus 8, as signed bytes: no borrow between bytes ((n | 0x80) - 8 keeps bit 7 set, then flip it)
 __device__ __forceinline__ uint32_t nibbles_minus8(uint32_t x) { return ((x | 0x80808080u) - 0x08080808u) ^ 0x80808080u; }
-
-// MUL_MAT_ID, grouped by expert: CTA column blockIdx.x is work item w = up to 32 (token, slot) pairs routed to one
-// expert.  *n_items items are in use (the other CTAs leave at once); work_expert[w] names the expert, col_act[32 w + c] the
-// quantized activation row of column c and col_out[32 w + c] the output row (pair index), -1 for the unused columns
-// of a short item.  Null work_expert: a plain mat-mul.
-struct GroupMap {
-    const int *n_items;
-    const int *work_expert;
-    const int *col_act;
-    const int *col_out;
-    int64_t expert_bytes;
-};
 
 struct TiBars {
     uint64_t full[3], empty[3], tfull[TI_TSTAGES], tempty[TI_TSTAGES];
@@ -566,7 +536,8 @@ size_t mmid_grouped_scratch_bytes(int64_t n_expert, int64_t n_pairs) {
 }
 int launch_mul_mat_id_grouped(int type, int64_t n, int64_t k, int64_t n_expert, int64_t ne11, int64_t n_tok, int64_t n_ids, const uint8_t *tiles,
                               ActView acts, const int32_t *ids, float *dst, void *lists, cudaStream_t s) {
-    B200_REQUIRE(type == B200_TYPE_MXFP4 || type == B200_TYPE_Q4_0, "mul_mat_id grouped: type %d is not a 32-element-block type on the 8x8 route", type);
+    const bool few = few_takes_experts(type, k, ne11 * n_tok, n_expert, n_tok * n_ids);
+    B200_REQUIRE(few || type == B200_TYPE_MXFP4 || type == B200_TYPE_Q4_0, "mul_mat_id grouped: type %d is not a 32-element-block type on the 8x8 route", type);
     const int64_t n_pairs = n_tok * n_ids;
     B200_REQUIRE(n_pairs < 0x7fffffffLL / TI_COLS && n_expert < (1 << 20), "mul_mat_id grouped: too many pairs or experts");
     const int64_t max_items = mmid_max_items(n_expert, n_pairs);
@@ -581,6 +552,7 @@ int launch_mul_mat_id_grouped(int type, int64_t n, int64_t k, int64_t n_expert, 
     gm.col_act = col_act;
     gm.col_out = col_out;
     gm.expert_bytes = (int64_t)((n + TILE_ROWS - 1) / TILE_ROWS) * (k / GROUP_K) * chunk_bytes(type);
+    if (few) return launch_gemm_few_grouped(type, n, k, n_expert, n_pairs, ne11 * n_tok, tiles, acts, dst, gm, max_items, s);
     if (type == B200_TYPE_MXFP4) return launch_i8<B200_TYPE_MXFP4>(n, k, TI_COLS, tiles, acts, dst, n, s, gm, max_items);
     return launch_i8<B200_TYPE_Q4_0>(n, k, TI_COLS, tiles, acts, dst, n, s, gm, max_items);
 }

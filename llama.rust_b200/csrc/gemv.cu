@@ -875,7 +875,8 @@ static int64_t gemv_stream_max_tiles() {
 }
 
 // whether launch_gemv takes (type, route, m activation rows) to a few-rows kernel, which can add a tensor to its result as it stores it
-bool gemv_rows_add_fusable(int type, int route, int64_t m) {
+bool gemv_rows_add_fusable(int type, int route, int64_t n, int64_t m) {
+    if (m < 32 && few_takes(type, route, n, GROUP_K, m)) return true;   // whatever K is; of more rows either kernel may be the one
     if (!(m >= GEMM_MMA_MIN_COLS && m < 32 && gemm_mma_enabled() && gemm_small_multi_enabled())) return false;
     return (type == B200_TYPE_Q4_K && route == B200_ROUTE_REPACK && m % 4 == 0) || (type == B200_TYPE_Q6_K && route == B200_ROUTE_TILED);
 }
@@ -889,6 +890,7 @@ int launch_gemv_rows_multi(int type, int route, int count, const int64_t *n, int
     const bool whole = route == B200_ROUTE_TILED || (route == B200_ROUTE_REPACK && m % 4 == 0);   // no tail rows on another chain
     int64_t rows = 0;
     for (int e = 0; e < count; e++) rows += n[e];
+    if (count > 1 && count <= 3 && few_takes(type, route, rows, k, m)) return launch_gemm_few(type, count, n, k, m, tiles, acts, dst, lddst, s);
     if (count > 1 && type == B200_TYPE_Q4_K && whole && (rows >= 2048 || (fe && fe[0] == '2')) && m >= GEMM_FAST_MIN_COLS && m >= GEMM_TCGEN05_MIN_COLS && gemm_mma_enabled() && gemm_tcgen05_enabled() &&
         gemm_tcgen05_f16_choice() < 0 && numerics_mode() == 1 && !no_scratch_mode() && !(fe && fe[0] == '0'))
         return launch_gemm_kq_fast_multi(type, count, n, k, m, tiles, acts, dst, lddst, s);
@@ -909,12 +911,13 @@ static bool block32_on_tcgen05(int type, int route, int64_t m) {
     return m >= GEMM_MMA_MIN_COLS && gemm_tcgen05_enabled() && gemm_mma_enabled() &&
            (((type == B200_TYPE_Q4_0 || type == B200_TYPE_MXFP4) && route == B200_ROUTE_REPACK) || (type == B200_TYPE_Q8_0 && route == B200_ROUTE_ROWDOT && numerics_mode() == 1));
 }
-bool gemv_wants_f16_acts(int type, int route, int64_t n, int64_t m) { return block32_on_tcgen05(type, route, m) && gemm_b32_wins(type, n, m); }
+bool gemv_wants_f16_acts(int type, int route, int64_t n, int64_t k, int64_t m) { return block32_on_tcgen05(type, route, m) && !few_takes(type, route, n, k, m) && gemm_b32_wins(type, n, m); }
 
 int launch_gemv(int type, int route, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst,
                 int64_t lddst, cudaStream_t s, ActF16 f16) {
     B200_REQUIRE(k % GROUP_K == 0, "gemv: k = %lld must be a multiple of 256", (long long)k);
     const int nb = (int)(k / GROUP_K);
+    if (few_takes(type, route, n, k, m)) return launch_gemm_few(type, 1, &n, k, m, &tiles, acts, &dst, &lddst, s);
     // the bulk-copy streaming kernel wins while every CTA has at most one row tile (no second wave to
     // overlap); beyond that the register-staged kernel with two CTAs per SM keeps more warps busy
     if (type == B200_TYPE_Q4_K && route == B200_ROUTE_REPACK && m == 1 && gemv_ksplit_enabled() && !no_scratch_mode() && nb >= 8 &&
@@ -1044,6 +1047,8 @@ int launch_mul_mat_id(int type, int64_t n, int64_t k, int64_t n_expert, int64_t 
     const bool repack = n % 8 == 0;
     // enough pairs to fill tensor-core tiles: grouped by expert, every expert's weights read once (same per-block chain,
     // same bits as the per-pair kernels below)
+    if (((type != B200_TYPE_MXFP4 && type != B200_TYPE_Q4_0) || repack) && few_takes_experts(type, k, ne11 * n_tok, n_expert, pairs) && mmid_grouped_enabled())
+        return launch_mul_mat_id_grouped(type, n, k, n_expert, ne11, n_tok, n_ids, tiles, acts, ids, dst, counts, s);
     if ((type == B200_TYPE_MXFP4 || type == B200_TYPE_Q4_0) && repack && pairs >= 64 && mmid_grouped_enabled() && gemm_tcgen05_enabled())
         return launch_mul_mat_id_grouped(type, n, k, n_expert, ne11, n_tok, n_ids, tiles, acts, ids, dst, counts, s);
     if (type == B200_TYPE_MXFP4 && repack) return launch_generic<TraitsB32<true>, 1>(n, nb, tiles, acts, dst, n, s, pm, pairs);
