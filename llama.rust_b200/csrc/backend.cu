@@ -140,6 +140,10 @@ struct BackendCtx {
     std::vector<StepPlan> plans;
     bool persistent_decode = false; // B200_DECODE_PERSISTENT=1 / decode_persistent=1: on
     uint64_t current_key = 0;       // node_list_key of the list being computed (0: not known)
+    // a step's inputs on their way to the device (backend_set_inputs): host memory that a kernel reads
+    uint8_t *stage = nullptr;
+    cudaEvent_t stage_read = nullptr;   // recorded behind that kernel
+    bool stage_used = false;
     TpGroup *tp = nullptr;        // the tensor-parallel group whose collectives the TP_* nodes run (owned by the driver)
 };
 constexpr size_t SHADOW_MAX_BYTES = 1 << 20;
@@ -1977,46 +1981,51 @@ static int run_nodes(BackendCtx *bc, ggml_cgraph *g) {
 // between tokens: positions reach ROPE through the position tensor on the device (rope_prepare), and the
 // key below covers everything else a node's launches are derived from.
 // the key is recomputed on every graph_compute, over a few hundred KB for a 32-layer decode step: eight bytes
-// per multiply (a byte-wise chain of dependent multiplies cost a third of a millisecond per token)
-static uint64_t fnv(uint64_t h, const void *p, size_t n) {
-    const uint8_t *b = (const uint8_t *)p;
-    size_t i = 0;
-    for (; i + 8 <= n; i += 8) {
-        uint64_t w;
-        memcpy(&w, b + i, 8);
+// per multiply (a byte-wise chain of dependent multiplies cost a third of a millisecond per token).
+// Four chains side by side: one multiply after the other took about 2 ns per eight bytes, 25 us of a one-token step of 8 layers
+struct NodeHash {
+    uint64_t h[4] = {0xcbf29ce484222325ull, 0x9ae16a3b2f90404full, 0xc3a5c85c97cb3127ull, 0xb492b66fbe98f273ull};
+    static uint64_t step(uint64_t h, uint64_t w) {
         h = (h ^ w) * 0x9e3779b97f4a7c15ull;
-        h ^= h >> 32;
+        return h ^ h >> 32;
     }
-    for (; i < n; i++) h = (h ^ b[i]) * 0x100000001b3ull;
-    return h;
-}
+    void add(const void *p, size_t n) {
+        const uint8_t *b = (const uint8_t *)p;
+        size_t i = 0;
+        for (; i + 32 <= n; i += 32) {
+            uint64_t w[4];
+            memcpy(w, b + i, 32);
+            for (int k = 0; k < 4; k++) h[k] = step(h[k], w[k]);
+        }
+        for (int k = 0; i < n; i += 8, k++) {   // the rest, its length beside it
+            uint64_t w = 0;
+            memcpy(&w, b + i, std::min<size_t>(8, n - i));
+            h[k] = step(h[k], w ^ (uint64_t)n << 56);
+        }
+    }
+    uint64_t value() const { return step(step(step(h[0], h[1]), h[2]), h[3]); }
+};
 static uint64_t node_list_key(const BackendCtx *bc, const ggml_cgraph *g) {
-    uint64_t h = 0xcbf29ce484222325ull;
-    h = fnv(h, &bc->cpu_threads, sizeof(int));
-    h = fnv(h, &bc->silu_wide, sizeof(int));
-    h = fnv(h, &bc->fuse_siblings, sizeof(bool));
-    h = fnv(h, &bc->fuse_glue, sizeof(bool));
-    h = fnv(h, &bc->fuse_prologue, sizeof(bool));
-    const int numerics = numerics_mode();
-    h = fnv(h, &numerics, sizeof(int));
-    h = fnv(h, &bc->persistent_decode, sizeof(bool));
-    h = fnv(h, &g->n_nodes, sizeof(int));
+    NodeHash h;
+    const int32_t head[8] = {bc->cpu_threads, bc->silu_wide, bc->fuse_siblings, bc->fuse_glue, bc->fuse_prologue, numerics_mode(), bc->persistent_decode, g->n_nodes};
+    h.add(head, sizeof(head));
     for (int i = 0; i < g->n_nodes; i++) {
         const ggml_tensor *t = g->nodes[i];
         if (!t) continue;
-        h = fnv(h, &t->type, sizeof(int32_t));
-        h = fnv(h, t->ne, sizeof(t->ne) + sizeof(t->nb));
-        h = fnv(h, &t->op, sizeof(int32_t) + sizeof(t->op_params));
-        h = fnv(h, &t->data, sizeof(void *));
+        struct { uint64_t type; const void *data; uint64_t sources; uint64_t index; } own = {(uint64_t)t->type, t->data, 0, (uint64_t)i};
+        for (int s = 0; s < GGML_MAX_SRC; s++) own.sources |= (uint64_t)(t->src[s] != nullptr) << s;
+        h.add(&own, sizeof(own));
+        h.add(t->ne, sizeof(t->ne) + sizeof(t->nb));
+        h.add(&t->op, sizeof(int32_t) + sizeof(t->op_params));
         for (int s = 0; s < GGML_MAX_SRC; s++) {
             const ggml_tensor *src = t->src[s];
             if (!src) continue;
-            h = fnv(h, &src->type, sizeof(int32_t));
-            h = fnv(h, src->ne, sizeof(src->ne) + sizeof(src->nb));
-            h = fnv(h, &src->data, sizeof(void *));
+            const uint64_t where[2] = {(uint64_t)src->type, (uint64_t)(uintptr_t)src->data};
+            h.add(where, sizeof(where));
+            h.add(src->ne, sizeof(src->ne) + sizeof(src->nb));
         }
     }
-    return h;
+    return h.value();
 }
 static void drop_captured(BackendCtx *bc) {
     for (auto &c : bc->captured)
@@ -2122,6 +2131,8 @@ static void backend_free(ggml_backend_t be) {
     }
     if (bc->act) cudaFree(bc->act);
     if (bc->rope_dev) cudaFree(bc->rope_dev);
+    if (bc->stage) cudaFreeHost(bc->stage);
+    if (bc->stage_read) cudaEventDestroy(bc->stage_read);
     for (auto &t : bc->rope_by_pos)
         if (t.dev) cudaFree(t.dev);
     cudaStreamDestroy(bc->stream);
@@ -2142,6 +2153,59 @@ static void backend_set_tensor_async(ggml_backend_t be, ggml_tensor *t, const vo
     cudaSetDevice(bc->device);
     shadow_note_write(c, t, data, offset, size);
     if (b200_memcpy_h2d((uint8_t *)t->data + offset, data, size, bc->stream) != B200_STATUS_SUCCESS) note(c, "set_tensor_async");
+}
+// Several small tensors at once, ordered like set_tensor_async and as free of their sources on return: the bytes go to page-locked memory,
+// and one kernel carries them to where they belong.  A step of a decode loop has five or six such inputs, and a copy each, with the GPU waiting,
+// was 4 to 5 us of every token.  What is not a plain tensor of whole words in a buffer of this backend, or too large, takes set_tensor_async.
+constexpr size_t STAGE_BYTES = 128 << 10;
+constexpr int STAGE_PARTS = 12;
+struct StageParts {
+    const uint8_t *src[STAGE_PARTS];
+    uint8_t *dst[STAGE_PARTS];
+    uint32_t words[STAGE_PARTS];
+};
+__global__ void __launch_bounds__(256) stage_inputs_kernel(const StageParts p) {
+    const uint32_t *src = (const uint32_t *)p.src[blockIdx.y];
+    uint32_t *dst = (uint32_t *)p.dst[blockIdx.y];
+    const uint32_t words = p.words[blockIdx.y], whole = ((uintptr_t)dst & 15) == 0 ? words / 4 : 0;   // the sources start on 16-byte boundaries
+    const uint32_t i0 = blockIdx.x * 256 + threadIdx.x, step = gridDim.x * 256;
+    for (uint32_t i = i0; i < whole; i += step) ((uint4 *)dst)[i] = ((const uint4 *)src)[i];
+    for (uint32_t i = 4 * whole + i0; i < words; i += step) dst[i] = src[i];
+}
+static int backend_set_inputs(ggml_backend_t be, int n, ggml_tensor *const *tensors, const void *const *data, const size_t *bytes) {
+    BackendCtx *bc = (BackendCtx *)be->context;
+    B200_CUDA(cudaSetDevice(bc->device));
+    if (!bc->stage && (cudaHostAlloc((void **)&bc->stage, STAGE_BYTES, cudaHostAllocDefault) != cudaSuccess || cudaEventCreateWithFlags(&bc->stage_read, cudaEventDisableTiming) != cudaSuccess)) {
+        cudaGetLastError();
+        if (bc->stage) cudaFreeHost(bc->stage);
+        bc->stage = nullptr;
+    }
+    if (bc->stage_used) B200_CUDA(cudaEventSynchronize(bc->stage_read));
+    StageParts p = {};
+    int parts = 0;
+    size_t at = 0, most = 0;
+    for (int i = 0; i < n; i++) {
+        ggml_tensor *t = tensors[i];
+        if (!t || !t->buffer || bytes[i] == 0) continue;
+        if (!bc->stage || is_tiled_tensor(t) || !in_our_buffer(t) || bytes[i] % 4 || ((uintptr_t)t->data & 3) || at + bytes[i] > STAGE_BYTES || parts == STAGE_PARTS) {
+            backend_set_tensor_async(be, t, data[i], 0, bytes[i]);
+            continue;
+        }
+        shadow_note_write(bctx(t->buffer), t, data[i], 0, bytes[i]);
+        memcpy(bc->stage + at, data[i], bytes[i]);
+        p.src[parts] = bc->stage + at;
+        p.dst[parts] = (uint8_t *)t->data;
+        p.words[parts++] = (uint32_t)(bytes[i] / 4);
+        at += (bytes[i] + 15) / 16 * 16;
+        most = std::max(most, bytes[i]);
+    }
+    if (parts == 0) return B200_STATUS_SUCCESS;
+    const unsigned gx = (unsigned)std::min<size_t>(8, (most + 4095) / 4096);
+    stage_inputs_kernel<<<dim3(gx, (unsigned)parts), 256, 0, bc->stream>>>(p);
+    B200_CUDA(cudaGetLastError());
+    B200_CUDA(cudaEventRecord(bc->stage_read, bc->stream));
+    bc->stage_used = true;
+    return B200_STATUS_SUCCESS;
 }
 static void backend_get_tensor_async(ggml_backend_t be, const ggml_tensor *t, void *data, size_t offset, size_t size) {
     BackendCtx *bc = (BackendCtx *)be->context;
@@ -2273,6 +2337,7 @@ static void *reg_get_proc_address(ggml_backend_reg_t, const char *name) {
     if (name && strcmp(name, "b200_backend_set_cpu_threads") == 0) return (void *)backend_set_cpu_threads;
     if (name && strcmp(name, "b200_backend_get_stream") == 0) return (void *)backend_get_stream;
     if (name && strcmp(name, "b200_backend_set_tp") == 0) return (void *)backend_set_tp;
+    if (name && strcmp(name, "b200_backend_set_inputs") == 0) return (void *)backend_set_inputs;
     return nullptr;
 }
 

@@ -111,6 +111,17 @@ struct Sequence {
     int32_t slot = -1;
 };
 
+// A step's result on its way to the caller: pieces that a few page-locked slots take in turn, so that the copy out of one overlaps the transfer
+// into the next, and the device error word behind them
+struct ReadBack {
+    static constexpr size_t SLOT = 256 << 10;
+    static constexpr int SLOTS = 4;
+    uint8_t *host = nullptr;              // SLOTS slots, then the error word
+    cudaEvent_t landed[SLOTS] = {};
+    bool ready();                         // makes them at the first call; false: cannot be had
+    void release();
+};
+
 }  // namespace b200
 
 struct b200_llama {
@@ -121,6 +132,8 @@ struct b200_llama {
     ggml_backend_t backend = nullptr;
     ggml_backend_buffer_type_t buft = nullptr;
     void *stream = nullptr;
+    int (*set_inputs)(ggml_backend_t, int, ggml_tensor *const *, const void *const *, const size_t *) = nullptr;   // the backend's, where it has one
+    b200::ReadBack back;
     std::map<std::string, std::unique_ptr<b200::Weight>> weights;
     std::set<std::string> tensors_set;    // placed tensors set so far (a device tensor may be put together from several)
     ggml_backend_buffer_t kv_buf = nullptr, compute_buf = nullptr;

@@ -19,11 +19,54 @@ int64_t n_kv_for(const b200_llama *c, int32_t high) {
     return std::min<int64_t>(c->n_ctx, std::max<int64_t>(KV_PAD, padded));
 }
 
-void set_input(ggml_tensor *t, const void *data, size_t bytes) { t->buffer->iface.set_tensor(t->buffer, t, data, 0, bytes); }
 // the per-step inputs: ordered on the backend's stream ahead of the step's graph, no wait per copy
-void set_input_async(ggml_backend_t be, ggml_tensor *t, const void *data, size_t bytes) {
-    if (be->iface.set_tensor_async) be->iface.set_tensor_async(be, t, data, 0, bytes);
-    else set_input(t, data, bytes);
+struct Inputs {
+    static constexpr int MOST = 10;
+    ggml_tensor *t[MOST];
+    const void *data[MOST];
+    size_t bytes[MOST];
+    int n = 0;
+    void add(ggml_tensor *tensor, const void *d, size_t b) {
+        t[n] = tensor;
+        data[n] = d;
+        bytes[n++] = b;
+    }
+    int send(b200_llama *c) {
+        if (c->set_inputs) return c->set_inputs(c->backend, n, t, data, bytes);
+        for (int i = 0; i < n; i++) {
+            if (c->backend->iface.set_tensor_async) c->backend->iface.set_tensor_async(c->backend, t[i], data[i], 0, bytes[i]);
+            else t[i]->buffer->iface.set_tensor(t[i]->buffer, t[i], data[i], 0, bytes[i]);
+        }
+        return B200_STATUS_SUCCESS;
+    }
+};
+
+// Logits and the kernels' error word to the host, and the end of the step.  A copy into pageable memory (and another one for the word) took
+// 30 us for one row of 32000 logits and 200 for sixteen; this way 15 and 110, of which the caller's fresh pages were touched while the GPU worked.
+int read_back(b200_llama *c, const void *dev, uint8_t *out, size_t bytes, int *code) {
+    cudaStream_t s = (cudaStream_t)c->stream;
+    ReadBack &r = c->back;
+    int *word = nullptr;
+    int rc = device_error_word(&word);
+    if (rc != B200_STATUS_SUCCESS) return rc;
+    volatile int *host_word = (volatile int *)(r.host + ReadBack::SLOTS * ReadBack::SLOT);
+    const size_t pieces = (bytes + ReadBack::SLOT - 1) / ReadBack::SLOT;
+    const auto length = [&](size_t i) { return std::min(ReadBack::SLOT, bytes - i * ReadBack::SLOT); };
+    const auto ask = [&](size_t i) -> cudaError_t {
+        const cudaError_t e = cudaMemcpyAsync(r.host + i % ReadBack::SLOTS * ReadBack::SLOT, (const uint8_t *)dev + i * ReadBack::SLOT, length(i), cudaMemcpyDeviceToHost, s);
+        return e == cudaSuccess ? cudaEventRecord(r.landed[i % ReadBack::SLOTS], s) : e;
+    };
+    B200_CUDA(cudaMemcpyAsync((void *)host_word, word, sizeof(int), cudaMemcpyDeviceToHost, s));
+    for (size_t i = 0; i < pieces && i < ReadBack::SLOTS; i++) B200_CUDA(ask(i));
+    for (size_t at = 0; at < bytes; at += 4096) ((volatile uint8_t *)out)[at] = ((volatile uint8_t *)out)[at];
+    for (size_t i = 0; i < pieces; i++) {
+        B200_CUDA(cudaEventSynchronize(r.landed[i % ReadBack::SLOTS]));
+        memcpy(out + i * ReadBack::SLOT, r.host + i % ReadBack::SLOTS * ReadBack::SLOT, length(i));
+        if (i + ReadBack::SLOTS < pieces) B200_CUDA(ask(i + ReadBack::SLOTS));
+    }
+    B200_CUDA(cudaStreamSynchronize(s));
+    *code = *host_word;
+    return B200_STATUS_SUCCESS;
 }
 
 // graph_compute over the first `total` nodes: the whole step is one node list, the collectives of a tensor-parallel
@@ -37,6 +80,25 @@ int run_graph(b200_llama *c, Graph *g, int total) {
 }
 
 }  // namespace
+
+bool b200::ReadBack::ready() {
+    if (host) return true;
+    bool ok = cudaMallocHost((void **)&host, SLOTS * SLOT + 64) == cudaSuccess;
+    for (int i = 0; i < SLOTS && ok; i++) ok = cudaEventCreateWithFlags(&landed[i], cudaEventDisableTiming) == cudaSuccess;
+    if (!ok) {
+        cudaGetLastError();
+        release();
+    }
+    return ok;
+}
+void b200::ReadBack::release() {
+    for (cudaEvent_t &e : landed) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
+    if (host) cudaFreeHost(host);
+    host = nullptr;
+}
 
 extern "C" {
 
@@ -90,6 +152,7 @@ static int context_new(std::unique_ptr<Arch> arch, int device, int32_t n_ctx, in
     typedef void *(*get_stream_fn)(ggml_backend_t);
     get_stream_fn get_stream = (get_stream_fn)reg->iface.get_proc_address(reg, "b200_backend_get_stream");
     c->stream = get_stream ? get_stream(c->backend) : nullptr;
+    c->set_inputs = (decltype(c->set_inputs))reg->iface.get_proc_address(reg, "b200_backend_set_inputs");
     int rc = c->arch->alloc_memory(c.get());
     if (rc != B200_STATUS_SUCCESS) { b200_llama_free(c.release()); return rc; }
     c->cell_pos.assign(n_ctx, -1);
@@ -169,6 +232,7 @@ void b200_llama_free(b200_llama *c) {
     if (c->kv_buf) c->kv_buf->iface.free_buffer(c->kv_buf);
     for (auto &kv : c->weights)
         if (kv.second->buf) kv.second->buf->iface.free_buffer(kv.second->buf);
+    c->back.release();
     if (c->backend) c->backend->iface.free(c->backend);
     if (c->tp) tp_group_destroy(c->tp);
     delete c;
@@ -515,30 +579,41 @@ int b200_llama_decode_seqs(b200_llama *c, const int32_t *tokens, const int32_t *
 
     // inputs land with synchronous copies after the previous step has drained
     c->backend->iface.synchronize(c->backend);
-    set_input_async(c->backend, g->tokens, tokens, (size_t)n * 4);
-    set_input_async(c->backend, g->pos, pos, (size_t)n * 4);
-    if (g->prev) set_input_async(c->backend, g->prev, c->prev_host.data(), (size_t)n * 4);
+    Inputs in;
+    in.add(g->tokens, tokens, (size_t)n * 4);
+    in.add(g->pos, pos, (size_t)n * 4);
+    if (g->prev) in.add(g->prev, c->prev_host.data(), (size_t)n * 4);
     if (masked) {
-        set_input_async(c->backend, g->mask, c->mask_host.data(), c->mask_host.size() * 2);
-        set_input_async(c->backend, g->row_idx, c->idx_host.data(), (size_t)n * 8);
+        in.add(g->row_idx, c->idx_host.data(), (size_t)n * 8);
     } else {
-        set_input_async(c->backend, g->cells, c->cells_host.data(), (size_t)n * 4);
-        set_input_async(c->backend, g->row_seg, c->row_seg_host.data(), (size_t)n * 4);
-        set_input_async(c->backend, g->seg, c->seg_host.data(), c->seg_host.size() * 4);
-        if (!c->tab_host.empty()) set_input_async(c->backend, g->tab, c->tab_host.data(), c->tab_host.size() * 4);
+        in.add(g->cells, c->cells_host.data(), (size_t)n * 4);
+        in.add(g->row_seg, c->row_seg_host.data(), (size_t)n * 4);
+        in.add(g->seg, c->seg_host.data(), c->seg_host.size() * 4);
+        if (!c->tab_host.empty()) in.add(g->tab, c->tab_host.data(), c->tab_host.size() * 4);
     }
-    set_input_async(c->backend, g->out_ids, out_rows, (size_t)n_out * 4);
+    in.add(g->out_ids, out_rows, (size_t)n_out * 4);
+    if (masked) in.add(g->mask, c->mask_host.data(), c->mask_host.size() * 2);   // the largest last
+    int rc = in.send(c);
+    if (rc != B200_STATUS_SUCCESS) return rc;
 
-    int rc = run_graph(c, g, (int)g->nodes.size() - (argmax ? 0 : 1));   // the ARGMAX node is last
+    rc = run_graph(c, g, (int)g->nodes.size() - (argmax ? 0 : 1));   // the ARGMAX node is last
     if (rc != B200_STATUS_SUCCESS) return rc;
     c->last = g;
     if (!masked) trim_sequences(c, seq_ids, n);
-    if (logits) c->backend->iface.get_tensor_async(c->backend, g->logits, logits, 0, (size_t)c->arch->n_vocab() * n_out * 4);
+    int code = 0;
+    const bool back = logits && c->stream && c->back.ready();
+    if (back) {
+        rc = read_back(c, g->logits->data, (uint8_t *)logits, (size_t)c->arch->n_vocab() * n_out * 4, &code);
+        if (rc != B200_STATUS_SUCCESS) return rc;
+    } else if (logits) {
+        c->backend->iface.get_tensor_async(c->backend, g->logits, logits, 0, (size_t)c->arch->n_vocab() * n_out * 4);
+    }
     if (argmax) c->backend->iface.get_tensor_async(c->backend, g->argmax, argmax, 0, (size_t)n_out * 4);
     c->backend->iface.synchronize(c->backend);
-    int code = 0;
-    rc = b200_kernel_error(&code);
-    if (rc != B200_STATUS_SUCCESS) return rc;
+    if (!back || code) {   // reading the word this way also clears it
+        rc = b200_kernel_error(&code);
+        if (rc != B200_STATUS_SUCCESS) return rc;
+    }
     B200_REQUIRE(code == 0, "llama_decode: a kernel reported error code %d", code);
     return B200_STATUS_SUCCESS;
 }
