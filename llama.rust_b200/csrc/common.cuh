@@ -429,6 +429,8 @@ inline int64_t grouped_pad(int64_t channels) { return (channels + 7) / 8 * 8; }
 int launch_grouped_store(const GroupedArgs &a, cudaStream_t s);
 int launch_grouped_decode(const GroupedArgs &a, cudaStream_t s);   // stores the rows' own cells too
 int launch_grouped_attn(const GroupedArgs &a, cudaStream_t s);     // their cells have been stored
+bool grouped_tc_takes(const GroupedArgs &a);                       // grouped_attn_tcgen05.cu: BF16 cells
+int launch_grouped_attn_tc(const GroupedArgs &a, int *err, cudaStream_t s);
 
 // scratch owned by the library (one growing allocation per device)
 int scratch_get(size_t bytes, void **ptr);

@@ -1002,6 +1002,7 @@ template <typename Y>
 int run_bf16(const GroupedArgs &a, int *err, cudaStream_t s) {
     const int d = a.dim, e = a.vdim;
     if (a.n_cells > 0x7fffffffLL) return run_any<__nv_bfloat16, Y>(a, err, s);
+    if (grouped_tc_takes(a)) return launch_grouped_attn_tc(a, err, s);
     if (d <= 64 && e <= 64) return run_mma<Y, 64, 64>(a, err, s);
     if (d <= 96 && e <= 96) return run_mma<Y, 96, 96>(a, err, s);
     if (d <= 128 && e <= 128) return run_mma<Y, 128, 128>(a, err, s);
