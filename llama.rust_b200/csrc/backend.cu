@@ -2118,6 +2118,51 @@ static int backend_graph_compute(ggml_backend_t be, ggml_cgraph *g) {
 }
 
 // ---- backend -------------------------------------------------------------------------------------
+// Page-locked memory of a backend: STAGE_BYTES for its inputs, then HOST_RESULT_BYTES for a caller that reads results through it
+// ("b200_backend_host_block").  Making such a block takes 2 ms, a third of a short model's first call, so a few outlive their backends.
+constexpr size_t STAGE_BYTES = 128 << 10;
+constexpr size_t HOST_BLOCKS_KEPT = 4;
+static std::mutex g_host_mu;
+static std::vector<uint8_t *> g_host_blocks;   // free ones, usable from every device
+static uint8_t *host_block_take() {
+    {
+        std::lock_guard<std::mutex> lk(g_host_mu);
+        if (!g_host_blocks.empty()) {
+            uint8_t *b = g_host_blocks.back();
+            g_host_blocks.pop_back();
+            return b;
+        }
+    }
+    void *b = nullptr;
+    if (cudaHostAlloc(&b, STAGE_BYTES + HOST_RESULT_BYTES, cudaHostAllocPortable) == cudaSuccess) return (uint8_t *)b;
+    cudaGetLastError();
+    return nullptr;
+}
+static void host_block_return(uint8_t *b) {
+    if (!b) return;
+    {
+        std::lock_guard<std::mutex> lk(g_host_mu);
+        if (g_host_blocks.size() < HOST_BLOCKS_KEPT) {
+            g_host_blocks.push_back(b);
+            return;
+        }
+    }
+    cudaFreeHost(b);
+}
+static bool stage_ready(BackendCtx *bc) {
+    if (bc->stage && bc->stage_read) return true;
+    if (!bc->stage) bc->stage = host_block_take();
+    if (bc->stage && !bc->stage_read && cudaEventCreateWithFlags(&bc->stage_read, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        bc->stage_read = nullptr;
+    }
+    return bc->stage && bc->stage_read;
+}
+static void *backend_host_block(ggml_backend_t be) {
+    BackendCtx *bc = (BackendCtx *)be->context;
+    cudaSetDevice(bc->device);
+    return stage_ready(bc) ? bc->stage + STAGE_BYTES : nullptr;
+}
 static const char *backend_get_name(ggml_backend_t be) { return ((BackendCtx *)be->context)->name.c_str(); }
 static void backend_free(ggml_backend_t be) {
     BackendCtx *bc = (BackendCtx *)be->context;
@@ -2131,7 +2176,7 @@ static void backend_free(ggml_backend_t be) {
     }
     if (bc->act) cudaFree(bc->act);
     if (bc->rope_dev) cudaFree(bc->rope_dev);
-    if (bc->stage) cudaFreeHost(bc->stage);
+    host_block_return(bc->stage);
     if (bc->stage_read) cudaEventDestroy(bc->stage_read);
     for (auto &t : bc->rope_by_pos)
         if (t.dev) cudaFree(t.dev);
@@ -2157,7 +2202,6 @@ static void backend_set_tensor_async(ggml_backend_t be, ggml_tensor *t, const vo
 // Several small tensors at once, ordered like set_tensor_async and as free of their sources on return: the bytes go to page-locked memory,
 // and one kernel carries them to where they belong.  A step of a decode loop has five or six such inputs, and a copy each, with the GPU waiting,
 // was 4 to 5 us of every token.  What is not a plain tensor of whole words in a buffer of this backend, or too large, takes set_tensor_async.
-constexpr size_t STAGE_BYTES = 128 << 10;
 constexpr int STAGE_PARTS = 12;
 struct StageParts {
     const uint8_t *src[STAGE_PARTS];
@@ -2175,11 +2219,7 @@ __global__ void __launch_bounds__(256) stage_inputs_kernel(const StageParts p) {
 static int backend_set_inputs(ggml_backend_t be, int n, ggml_tensor *const *tensors, const void *const *data, const size_t *bytes) {
     BackendCtx *bc = (BackendCtx *)be->context;
     B200_CUDA(cudaSetDevice(bc->device));
-    if (!bc->stage && (cudaHostAlloc((void **)&bc->stage, STAGE_BYTES, cudaHostAllocDefault) != cudaSuccess || cudaEventCreateWithFlags(&bc->stage_read, cudaEventDisableTiming) != cudaSuccess)) {
-        cudaGetLastError();
-        if (bc->stage) cudaFreeHost(bc->stage);
-        bc->stage = nullptr;
-    }
+    const bool staged = stage_ready(bc);
     if (bc->stage_used) B200_CUDA(cudaEventSynchronize(bc->stage_read));
     StageParts p = {};
     int parts = 0;
@@ -2187,7 +2227,7 @@ static int backend_set_inputs(ggml_backend_t be, int n, ggml_tensor *const *tens
     for (int i = 0; i < n; i++) {
         ggml_tensor *t = tensors[i];
         if (!t || !t->buffer || bytes[i] == 0) continue;
-        if (!bc->stage || is_tiled_tensor(t) || !in_our_buffer(t) || bytes[i] % 4 || ((uintptr_t)t->data & 3) || at + bytes[i] > STAGE_BYTES || parts == STAGE_PARTS) {
+        if (!staged || is_tiled_tensor(t) || !in_our_buffer(t) || bytes[i] % 4 || ((uintptr_t)t->data & 3) || at + bytes[i] > STAGE_BYTES || parts == STAGE_PARTS) {
             backend_set_tensor_async(be, t, data[i], 0, bytes[i]);
             continue;
         }
@@ -2338,6 +2378,7 @@ static void *reg_get_proc_address(ggml_backend_reg_t, const char *name) {
     if (name && strcmp(name, "b200_backend_get_stream") == 0) return (void *)backend_get_stream;
     if (name && strcmp(name, "b200_backend_set_tp") == 0) return (void *)backend_set_tp;
     if (name && strcmp(name, "b200_backend_set_inputs") == 0) return (void *)backend_set_inputs;
+    if (name && strcmp(name, "b200_backend_host_block") == 0) return (void *)backend_host_block;
     return nullptr;
 }
 

@@ -432,6 +432,7 @@ int launch_grouped_attn(const GroupedArgs &a, cudaStream_t s);     // their cell
 bool grouped_tc_takes(const GroupedArgs &a);                       // grouped_attn_tcgen05.cu: BF16 cells
 int launch_grouped_attn_tc(const GroupedArgs &a, int *err, cudaStream_t s);
 
+constexpr size_t HOST_RESULT_BYTES = (1 << 20) + 256;   // of a backend's page-locked block (backend.cu): what the decode driver reads results through
 // scratch owned by the library (one growing allocation per device)
 int scratch_get(size_t bytes, void **ptr);
 int scratch_get_kx(size_t bytes, void **ptr);   // a second block, for the K-split exchange of the decode mat-mul

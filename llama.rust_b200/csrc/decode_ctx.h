@@ -116,9 +116,9 @@ struct Sequence {
 struct ReadBack {
     static constexpr size_t SLOT = 256 << 10;
     static constexpr int SLOTS = 4;
-    uint8_t *host = nullptr;              // SLOTS slots, then the error word
+    uint8_t *host = nullptr;              // SLOTS slots, then the error word: the backend's
     cudaEvent_t landed[SLOTS] = {};
-    bool ready();                         // makes them at the first call; false: cannot be had
+    bool ready(ggml_backend_t be, void *(*block)(ggml_backend_t));   // asks for them at the first call; false: cannot be had
     void release();
 };
 
@@ -133,6 +133,7 @@ struct b200_llama {
     ggml_backend_buffer_type_t buft = nullptr;
     void *stream = nullptr;
     int (*set_inputs)(ggml_backend_t, int, ggml_tensor *const *, const void *const *, const size_t *) = nullptr;   // the backend's, where it has one
+    void *(*host_block)(ggml_backend_t) = nullptr;
     b200::ReadBack back;
     std::map<std::string, std::unique_ptr<b200::Weight>> weights;
     std::set<std::string> tensors_set;    // placed tensors set so far (a device tensor may be put together from several)

@@ -81,9 +81,11 @@ int run_graph(b200_llama *c, Graph *g, int total) {
 
 }  // namespace
 
-bool b200::ReadBack::ready() {
+bool b200::ReadBack::ready(ggml_backend_t be, void *(*block)(ggml_backend_t)) {
+    static_assert(SLOTS * SLOT + sizeof(int) <= HOST_RESULT_BYTES, "the backend's block holds the slots and the error word");
     if (host) return true;
-    bool ok = cudaMallocHost((void **)&host, SLOTS * SLOT + 64) == cudaSuccess;
+    host = block ? (uint8_t *)block(be) : nullptr;
+    bool ok = host != nullptr;
     for (int i = 0; i < SLOTS && ok; i++) ok = cudaEventCreateWithFlags(&landed[i], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
@@ -96,7 +98,6 @@ void b200::ReadBack::release() {
         if (e) cudaEventDestroy(e);
         e = nullptr;
     }
-    if (host) cudaFreeHost(host);
     host = nullptr;
 }
 
@@ -153,6 +154,7 @@ static int context_new(std::unique_ptr<Arch> arch, int device, int32_t n_ctx, in
     get_stream_fn get_stream = (get_stream_fn)reg->iface.get_proc_address(reg, "b200_backend_get_stream");
     c->stream = get_stream ? get_stream(c->backend) : nullptr;
     c->set_inputs = (decltype(c->set_inputs))reg->iface.get_proc_address(reg, "b200_backend_set_inputs");
+    c->host_block = (decltype(c->host_block))reg->iface.get_proc_address(reg, "b200_backend_host_block");
     int rc = c->arch->alloc_memory(c.get());
     if (rc != B200_STATUS_SUCCESS) { b200_llama_free(c.release()); return rc; }
     c->cell_pos.assign(n_ctx, -1);
@@ -601,7 +603,7 @@ int b200_llama_decode_seqs(b200_llama *c, const int32_t *tokens, const int32_t *
     c->last = g;
     if (!masked) trim_sequences(c, seq_ids, n);
     int code = 0;
-    const bool back = logits && c->stream && c->back.ready();
+    const bool back = logits && c->stream && c->back.ready(c->backend, c->host_block);
     if (back) {
         rc = read_back(c, g->logits->data, (uint8_t *)logits, (size_t)c->arch->n_vocab() * n_out * 4, &code);
         if (rc != B200_STATUS_SUCCESS) return rc;
