@@ -581,7 +581,7 @@ int b200_mul_mat_q8_add(int type, int64_t n, int64_t k, const void *dev_w, const
 
 int b200_mul_mat_q8_rows_add_fusable(int type, int64_t n, int64_t m) {
     if (!is_quant_type(type) || n <= 0 || m <= 0) return 0;
-    return gemv_rows_add_fusable(type, pick_route(type, n, m), n, m) ? 1 : 0;
+    return gemv_rows_add_fusable(type, pick_route(type, n, m), n, GROUP_K, m) ? 1 : 0;   // the call itself looks at K too
 }
 
 int b200_mul_mat_q8_rows_add(int type, int64_t n, int64_t k, int64_t m, const void *dev_w, const void *dev_act, int act_kind, float *dev_dst, int64_t lddst,
@@ -592,7 +592,7 @@ int b200_mul_mat_q8_rows_add(int type, int64_t n, int64_t k, int64_t m, const vo
     B200_REQUIRE(dev_w && dev_act && dev_dst && dev_addend && dev_sum, "mul_mat_q8_rows_add: null pointer");
     B200_REQUIRE(lddst >= n && ld_addend >= n && ld_sum >= n, "mul_mat_q8_rows_add: row strides smaller than the rows");
     const int route = pick_route(type, n, m);
-    B200_REQUIRE(gemv_rows_add_fusable(type, route, n, m), "mul_mat_q8_rows_add: type %d with %lld activation rows does not take a few-rows kernel", type, (long long)m);
+    B200_REQUIRE(gemv_rows_add_fusable(type, route, n, k, m), "mul_mat_q8_rows_add: type %d with %lld activation rows does not take a few-rows kernel", type, (long long)m);
     B200_REQUIRE(act_kind == act_kind_for(type, route, m), "mul_mat_q8_rows_add: activation kind %d does not fit type %d", act_kind, type);
     ActView a = act_carve(const_cast<void *>(dev_act), m, k).view();
     a.addend = dev_addend;

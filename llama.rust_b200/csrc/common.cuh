@@ -166,7 +166,7 @@ bool gemm_small_multi_enabled();
 int launch_gemm_rows_ring(int count, const int64_t *n, int64_t k, int64_t m, const uint8_t *const *tiles, ActView acts, float *const *dst,
                           const int64_t *lddst, cudaStream_t s);
 void gemm_rows_ring_debug_wait(int spin_limit, int skip_unit);
-bool gemv_rows_add_fusable(int type, int route, int64_t n, int64_t m);
+bool gemv_rows_add_fusable(int type, int route, int64_t n, int64_t k, int64_t m);
 // a few activation rows, fast numerics (gemm_few.cu)
 bool few_takes(int type, int route, int64_t n, int64_t k, int64_t m);
 bool few_takes_experts(int type, int64_t k, int64_t act_rows, int64_t n_expert, int64_t pairs);

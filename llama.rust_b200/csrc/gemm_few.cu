@@ -646,7 +646,7 @@ bool few_takes(int type, int route, int64_t n, int64_t k, int64_t m) {
 // MXFP4 (Q4_0) against int8 tiles of 32 pairs: 128 experts, 128 pairs 83 -> 52 (64 -> 39), 512 pairs 121 -> 67 (92 -> 50), 1024 pairs 123 -> 80
 // (94 -> 62); 32 pairs an expert 174 -> 189 (137 -> 153)
 bool few_takes_experts(int type, int64_t k, int64_t act_rows, int64_t n_expert, int64_t pairs) {
-    if (numerics_mode() != 1 || pairs < 64 || act_rows * (k / GROUP_K) >= (1ll << 24)) return false;
+    if (numerics_mode() != 1 || pairs < 64 || pairs >= 0x7fffffffLL / 32 || n_expert >= (1 << 20) || act_rows * (k / GROUP_K) >= (1ll << 24)) return false;
     const char *e = getenv("B200_GEMM_FEW");
     if (e && e[0] == '0') return false;
     const int64_t avg = pairs / (n_expert < pairs ? n_expert : pairs);

@@ -875,8 +875,8 @@ static int64_t gemv_stream_max_tiles() {
 }
 
 // whether launch_gemv takes (type, route, m activation rows) to a few-rows kernel, which can add a tensor to its result as it stores it
-bool gemv_rows_add_fusable(int type, int route, int64_t n, int64_t m) {
-    if (m < 32 && few_takes(type, route, n, GROUP_K, m)) return true;   // whatever K is; of more rows either kernel may be the one
+bool gemv_rows_add_fusable(int type, int route, int64_t n, int64_t k, int64_t m) {
+    if (m < 32 && few_takes(type, route, n, k, m)) return true;   // of more rows either kernel may be the one
     if (!(m >= GEMM_MMA_MIN_COLS && m < 32 && gemm_mma_enabled() && gemm_small_multi_enabled())) return false;
     return (type == B200_TYPE_Q4_K && route == B200_ROUTE_REPACK && m % 4 == 0) || (type == B200_TYPE_Q6_K && route == B200_ROUTE_TILED);
 }

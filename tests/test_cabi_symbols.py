@@ -131,3 +131,23 @@ def test_rows_add_refuses_bad_arguments_before_touching_a_device():
     assert b"activation kind" in mod.lib.b200_last_error()
     # nothing to do
     assert f(mod.Q4_K, 0, 4096, 16, one, one, mod.ACT_Q8_K_MIXED, one, 4096, one, 4096, one, 4096, None) == 0
+
+
+def test_rows_add_refuses_rows_too_long_for_the_few_rows_kernel():
+    """fast numerics: Q8_0 rows whose activations are past the few-rows kernel's 32-bit offsets go to a kernel without the residual add, so the
+    call refuses them; rows just within are refused for their activation kind only, which is looked at after that"""
+    mod = b200.load()
+    f = mod.lib.b200_mul_mat_q8_rows_add
+    f.restype = ctypes.c_int
+    i64, vp = ctypes.c_int64, ctypes.c_void_p
+    f.argtypes = [ctypes.c_int, i64, i64, i64, vp, vp, ctypes.c_int, vp, i64, vp, i64, vp, i64, vp]
+    one = 256
+    before = mod.lib.b200_get_numerics()
+    mod.lib.b200_set_numerics(1)
+    try:
+        limit = (1 << 24) // 16 * 256      # 16 rows of so many values are 2^24 groups
+        for k, word in ((limit, b"few-rows kernel"), (limit - 256, b"activation kind")):
+            assert f(mod.Q8_0, 8, k, 16, one, one, mod.ACT_Q8_K_MIXED, one, 8, one, 8, one, 8, None) != 0
+            assert word in mod.lib.b200_last_error(), k
+    finally:
+        mod.lib.b200_set_numerics(before)
