@@ -236,7 +236,7 @@ fa_decode_mma_kernel(b200_flash_attn_args a, DmDims d, float scale_log2, float *
     }
     auto tile_at = [&](int i) -> int64_t { return listed ? l_base + vis_list[i] * l_step : tile0 + (int64_t)i; };
 
-    // ldmatrix addressing (see flash_attn_prefill.cu): K non-transposed, V transposed
+    // ldmatrix addressing: K non-transposed (matrices of 8 positions x 8 halves), V transposed
     const int k_row = (lane & 7) + ((lane >> 4) << 3), k_col = ((lane >> 3) & 1) * 16;
     const int v_row = (lane & 7) + (((lane >> 3) & 1) << 3), v_col = (lane >> 4) * 16;
 
