@@ -591,6 +591,7 @@ bool flash_attn_rows_visible(const b200_flash_attn_args *a, cudaStream_t s, int 
 bool flash_attn_fast_rows(const b200_flash_attn_args *a, cudaStream_t s, int *rc);                                  // flash_attn_fast.cu
 bool flash_attn_fast_prompt(const b200_flash_attn_args *a, cudaStream_t s, int *rc);                                // flash_attn_prompt.cu
 bool flash_attn_decode_mma(const b200_flash_attn_args *a, cudaStream_t s, int *rc);                                 // flash_attn_decode_mma.cu
+bool flash_attn_decode_mma_takes(const b200_flash_attn_args *a);                                                    // flash_attn_decode_mma.cu
 
 // B200_FA_DECODE_MMA=0 keeps fast-mode attention of fewer than 64 query rows off the tensor-core flash-decoding kernel: single
 // rows then take the CUDA-core kernel (the one the persistent decode step carries), several rows the exact kernels
@@ -667,16 +668,16 @@ extern "C" int b200_flash_attn_ext(const struct b200_flash_attn_args *args, void
     // than it (measured on 16 sequences over 10240 cells).
     const bool policy = args->mode == 0 && numerics_mode() == 1;
     if ((args->mode == 1 || policy) && args->n_tok < 64) {
-        if (fa_decode_mma_enabled()) {
+        // What the decode kernel does not take (heads in groups that do not divide 16, mask rows off 4 bytes) keeps the kernels below, which read
+        // q and the weights in F32, or as the CPU does, and no position that a row does not see.
+        if (fa_decode_mma_enabled() && flash_attn_decode_mma_takes(args)) {
             // Two to 63 rows.  The prompt kernel computes 128 rows at a time with its positions over a cluster, the decode kernel 16 rows (whole
             // tokens) that skip what none of them sees.  32 heads of 128 on 8 KV heads, us decode / prompt kernel: a causal batch of 16 rows
             // over 2048 positions 22.8 / 13.1, 8192 36 / 19, 32768 95 / 44 (63 rows 344 / 60); sequences that see a 16th each 19.1 / 12.6,
             // 22.7 / 21.9, 46 / 60 (of 63 sequences 66 / 52).  Above 8192 positions so few rows are more likely sequences than a prompt's.
-            // What the decode kernel does not take (mask rows of an odd length) is the prompt kernel's as well.
             const bool wide = args->n_tok > 1 && (args->n_kv <= 8192 || args->n_tok >= 32);
             if (wide && flash_attn_fast_prompt(args, (cudaStream_t)stream, &rc)) return rc;
             if (flash_attn_decode_mma(args, (cudaStream_t)stream, &rc)) return rc;
-            if (args->n_tok > 1 && flash_attn_fast_prompt(args, (cudaStream_t)stream, &rc)) return rc;
         }
         if ((args->mode == 1 || args->n_tok == 1) && flash_attn_fast_rows(args, (cudaStream_t)stream, &rc)) return rc;
     }

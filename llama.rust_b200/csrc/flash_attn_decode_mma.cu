@@ -411,8 +411,8 @@ __device__ int g_dm_counters_dev[4096];
 
 }  // namespace
 
-// true: the tensor-core decode kernel took the call (*rc is its status); false: not a shape it handles
-bool flash_attn_decode_mma(const b200_flash_attn_args *a, cudaStream_t s, int *rc) {
+// the launch's shape; false: not a call this kernel handles.  A device that cannot be asked fails in *rc
+static bool decode_mma_plan(const b200_flash_attn_args *a, DmDims *dims, int *device, int *sm_count, int *rc) {
     *rc = B200_STATUS_SUCCESS;
     if (a->sinks || a->max_bias != 0.0f || a->logit_softcap != 0.0f || a->dk != a->dv || (a->dk != 64 && a->dk != 128) || a->n_tok >= 64 || a->n_kv == 0 ||
         a->n_tok == 0)
@@ -421,7 +421,7 @@ bool flash_attn_decode_mma(const b200_flash_attn_args *a, cudaStream_t s, int *r
     if (a->q_nb1 % 8 || a->q_nb2 % 8 || ((uintptr_t)a->q & 7) || ((uintptr_t)a->dst & 15)) return false;
     if (a->k_nb1 % 16 || a->v_nb1 % 16 || a->k_nb2 % 16 || a->v_nb2 % 16 || ((uintptr_t)a->k & 15) || ((uintptr_t)a->v & 15)) return false;
     if (a->mask && (a->mask_nb1 % 4 || ((uintptr_t)a->mask & 3))) return false;
-    DmDims d;
+    DmDims &d = *dims;
     d.T = (int)a->n_tok; d.H = (int)a->n_head; d.H_kv = (int)a->n_head_kv; d.group = d.H / d.H_kv;
     d.n_kv = a->n_kv;
     d.row_blocks = (d.T * d.group + DM_BM - 1) / DM_BM;
@@ -442,6 +442,24 @@ bool flash_attn_decode_mma(const b200_flash_attn_args *a, cudaStream_t s, int *r
     d.tiles_per_split = (int)((n_tiles + want - 1) / want);
     d.n_splits = (int)((n_tiles + d.tiles_per_split - 1) / d.tiles_per_split);
     if (d.T > 1 && d.tiles_per_split > DM_MAX_LIST) return false;
+    *device = dev;
+    *sm_count = sms;
+    return true;
+}
+
+// whether flash_attn_decode_mma would take the call
+bool flash_attn_decode_mma_takes(const b200_flash_attn_args *a) {
+    DmDims d;
+    int dev = 0, sms = 0, rc = B200_STATUS_SUCCESS;
+    return decode_mma_plan(a, &d, &dev, &sms, &rc) && rc == B200_STATUS_SUCCESS;
+}
+
+// true: the tensor-core decode kernel took the call (*rc is its status); false: not a shape it handles
+bool flash_attn_decode_mma(const b200_flash_attn_args *a, cudaStream_t s, int *rc) {
+    DmDims d;
+    int dev = 0, sms = 0;
+    if (!decode_mma_plan(a, &d, &dev, &sms, rc)) return false;
+    if (*rc != B200_STATUS_SUCCESS) return true;
     {
         const char *e = getenv("B200_FA_DECODE_STRIDED");
         d.strided = !(e && e[0] == '0');   // on unless switched off

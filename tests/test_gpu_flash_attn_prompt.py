@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 import b200
+import orc
 from test_gpu_flash_attn import synth_case
 from test_gpu_flash_attn_fast import ref64, row_rel
 
@@ -119,8 +120,33 @@ def test_strided_views(dev):
     check(dev, q, k, v, mask, D ** -0.5, dst.download(np.float32, T * H * D).reshape(T, H, D))
 
 
-def test_few_rows_over_a_long_cache_keep_the_decode_kernel_where_it_can(dev):
-    """16 rows over more than 8192 positions: the same function whichever kernel takes them (an odd cache: the prompt kernel)"""
+def test_few_rows_over_a_long_cache(dev):
+    """16 rows over more than 8192 positions: the same function whichever kernel takes them"""
     for n_kv in (8704, 8705):
         q, k, v, mask = synth_case(8, 2, 128, 16, n_kv, seed=n_kv)
         check(dev, q, k, v, mask, 128 ** -0.5)
+
+
+@pytest.mark.parametrize("H,Hkv,n_kv", [(6, 2, 300), (5, 1, 640), (8, 2, 301), (7, 1, 1023)], ids=str)
+def test_few_rows_that_the_decode_kernel_refuses_keep_their_precision(dev, H, Hkv, n_kv):
+    """groups of heads that do not divide 16, mask rows off 4 bytes: under mode 1 the kernel that keeps q and the weights in F32 (1e-5 of float64 with q as
+    it is, where q rounded to f16 alone is 2^-11 off), under the fast policy the CPU's bits, which NaN in a cell that nobody sees does not change"""
+    T, D = 5, 128
+    q, k, v, _ = synth_case(H, Hkv, D, T, n_kv, seed=H + n_kv, causal=False)
+    m = np.zeros((T, n_kv), np.float16)
+    m[:, 40:44] = -np.inf
+    for t in range(T):
+        m[t, n_kv - T + t + 1:] = -np.inf
+    mask = m.view(np.uint16)
+    want = ref64(q, k, v, mask, D ** -0.5)
+    cpu, _ = orc.flash_attn(q, k, v, mask, D ** -0.5)
+    got = dev.flash_attn(q, dev.KvCacheView(k, v), mask, D ** -0.5, mode=1)
+    assert row_rel(got, want) <= 1e-5
+    k, v = k.copy(), v.copy()
+    k[:, 41], v[:, 42] = 0x7E00, 0x7C00
+    dev.set_numerics(dev.FAST)
+    try:
+        got = dev.flash_attn(q, dev.KvCacheView(k, v), mask, D ** -0.5)
+    finally:
+        dev.set_numerics(dev.EXACT)
+    assert np.array_equal(got.view(np.uint32), cpu.view(np.uint32))
