@@ -117,4 +117,82 @@ __device__ __forceinline__ float2 pa_ld_peer2(uint32_t addr) {
     return v;
 }
 
+// ---- rows whose output is not finite ------------------------------------------------------------------------------
+// The products run over whole tiles, so what a cell holds that a row does not see meets that row with weight 0: 0 * Inf and NaN scores spoil it.  A
+// row that ends with anything but finite numbers is therefore computed once more, by a warp, from the cells it sees alone: nothing where all is
+// finite, and the definition's Inf and NaN where they belong.  (4096 positions take a row a quarter of a millisecond; a NaN score, as of a query with
+// a NaN, ends it at the first 32.)
+__device__ __forceinline__ bool pa_finite(float x) { return fabsf(x) < INFINITY; }
+template <bool BF16>
+__device__ __forceinline__ float2 pa_two(uint32_t w) {
+    if (BF16) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    return __half22float2(*(const __half2 *)&w);
+}
+// Row x of the swizzled query operand at q against n entries.  entry(i, &bias, &key, &value): whether the row sees entry i, its addend (log2 units) and
+// its 16-byte aligned key and value rows of D elements.  acc[2 e], acc[2 e + 1]: this lane's output channels 64 e + 2 lane and + 1, not yet divided by
+// the sum; top: the maximum in use (log2 units, -inf: sees nothing)
+template <int D, bool BF16, typename Entry>
+__device__ __forceinline__ void pa_row_again(const uint8_t *q, int x, float scale_log2, int n, const Entry &entry, float (&acc)[D / 32], float *top, float *sum) {
+    const int lane = threadIdx.x & 31;
+    const uint8_t *const qrow = q + (x >> 3) * 1024 + (x & 7) * 128;
+    float m = -INFINITY, l = 0.0f;
+#pragma unroll
+    for (int e = 0; e < D / 32; e++) acc[e] = 0.0f;
+#pragma unroll 1
+    for (int base = 0; base < n; base += 32) {   // a lane has an entry's score, then two channels of each 64
+        const uint8_t *key = nullptr, *value = nullptr;
+        float bias = 0.0f, s = -INFINITY;
+        const bool sees = base + lane < n && entry(base + lane, &bias, &key, &value);
+        if (sees) {
+            float dot = 0.0f;
+#pragma unroll 2
+            for (int c = 0; c < D / 8; c++) {
+                const uint4 k4 = *(const uint4 *)(key + 16 * c), q4 = *(const uint4 *)(qrow + (c >> 3) * (128 * 128) + (((c & 7) ^ (x & 7)) << 4));
+                const uint32_t kw[4] = {k4.x, k4.y, k4.z, k4.w}, qw[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float2 a = pa_two<BF16>(kw[i]), b = pa_two<BF16>(qw[i]);
+                    dot = fmaf(a.x, b.x, dot);
+                    dot = fmaf(a.y, b.y, dot);
+                }
+            }
+            s = fmaf(dot, scale_log2, bias);
+        }
+        if (__any_sync(0xffffffffu, sees && !(s < INFINITY))) {   // NaN, or a weight of exp(inf - inf)
+            m = 0.0f;
+            l = NAN;
+#pragma unroll
+            for (int e = 0; e < D / 32; e++) acc[e] = NAN;
+            break;
+        }
+        float mx = s;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (mx == -INFINITY) continue;
+        const float mn = fmaxf(m, mx), al = pa_ex2(m - mn), w = pa_ex2(s - mn);
+        m = mn;
+        float ws = w;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
+        l = fmaf(l, al, ws);
+#pragma unroll
+        for (int e = 0; e < D / 32; e++) acc[e] *= al;
+        const uint32_t seen = __ballot_sync(0xffffffffu, sees);
+#pragma unroll 4
+        for (int j = 0; j < 32; j++) {
+            const float wj = __shfl_sync(0xffffffffu, w, j);
+            const uint8_t *vj = (const uint8_t *)__shfl_sync(0xffffffffu, (unsigned long long)value, j);
+            if (!(seen >> j & 1)) continue;
+#pragma unroll
+            for (int e = 0; e < D / 64; e++) {
+                const float2 v = pa_two<BF16>(*(const uint32_t *)(vj + 128 * e + 4 * lane));
+                acc[2 * e] = fmaf(wj, v.x, acc[2 * e]);
+                acc[2 * e + 1] = fmaf(wj, v.y, acc[2 * e + 1]);
+            }
+        }
+    }
+    *top = m;
+    *sum = l;
+}
+
 }  // namespace b200

@@ -15,6 +15,7 @@
 //     in F16 with the same relative rounding, and the sums are F32 either way.
 //   * Six warps read the mask ahead of everyone and sort the CTA's (row block, tile) pairs into: all zero (no mask read at all in the
 //     softmax), all minus infinity (skipped by every role), mixed (each row reads its 128 mask values).
+//   * A row whose output is not finite is computed again from what it sees alone (pa_row_again): the tiles' products multiply hidden cells by 0.
 //   * The positions are dealt out to the CTAs of a cluster, tile by tile, where there are too few row blocks for the GPU; the
 //     partial outputs meet in shared memory and every CTA finishes its share of the rows.
 // Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device error word.
@@ -71,8 +72,8 @@ struct PaShared {
 };
 
 struct PaArgs {
-    const unsigned char *q, *mask;
-    int64_t q_nb1, q_nb2, mask_nb1;
+    const unsigned char *q, *mask, *k, *v;   // k, v: only for rows that are computed again
+    int64_t q_nb1, q_nb2, mask_nb1, k_nb1, k_nb2, v_nb1, v_nb2;
     float *dst;
     int64_t n_kv, rows;
     int n_tok, n_head, group, splits, n_tiles, mask_wide;
@@ -491,9 +492,10 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         pa_fence_after();
         asm volatile("bar.sync 1, 256;" ::: "memory");
         const float ma = sh.ml[0][r][0], mb = sh.ml[1][r][0], mm = fmaxf(ma, mb);
-        // no output where the group visited no tile or the row saw nothing in them
-        const float wa = ma == -INFINITY ? 0.0f : pa_ex2(ma - mm), wb = mb == -INFINITY ? 0.0f : pa_ex2(mb - mm);
-        const float lt = (ma == -INFINITY ? 0.0f : wa * sh.ml[0][r][1]) + (mb == -INFINITY ? 0.0f : wb * sh.ml[1][r][1]);
+        // No output where the group visited no tile or the row saw nothing in them.  Their sum is 0 then, or NaN: a maximum does not show a NaN
+        const bool ina = ma != -INFINITY, inb = mb != -INFINITY;
+        const float wa = ina ? pa_ex2(ma - mm) : 1.0f, wb = inb ? pa_ex2(mb - mm) : 1.0f;
+        const float lt = wa * sh.ml[0][r][1] + wb * sh.ml[1][r][1];
         asm volatile("bar.sync 1, 256;" ::: "memory");
         if (g == 0) {
             sh.ml[0][r][0] = mm;
@@ -509,7 +511,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 pa_wait_ld();
 #pragma unroll
                 for (int e = 0; e < 32; e++) {
-                    const float u = wa != 0.0f ? wa * __uint_as_float(x[e]) : 0.0f, v = wb != 0.0f ? wb * __uint_as_float(y[e]) : 0.0f;
+                    const float u = ina ? wa * __uint_as_float(x[e]) : 0.0f, v = inb ? wb * __uint_as_float(y[e]) : 0.0f;
                     x[e] = __float_as_uint(u + v);
                 }
 #pragma unroll
@@ -527,6 +529,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         // this CTA's share of the rows: a warp per row, the CTAs' partial outputs under their common maximum
         const int lo = PA_M * rank / a.splits, hi = PA_M * (rank + 1) / a.splits;
         const uint32_t ml = pa_smem(&sh.ml[0][0][0]);
+        uint32_t again = 0;   // which of this warp's rows are not finite
         for (int r = lo + warp; r < hi; r += PA_THREADS / 32) {
             const int64_t row = row0 + r;
             if (row >= a.rows) break;
@@ -542,7 +545,10 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             for (int e = 0; e < D / 32; e++) acc[e] = 0.0f;
 #pragma unroll
             for (int p = 0; p < PA_MAX_SPLITS; p++) {
-                if (st[p].x == -INFINITY) continue;
+                if (st[p].x == -INFINITY) {
+                    sum += st[p].y;   // 0 or NaN
+                    continue;
+                }
                 const float w = pa_ex2(st[p].x - top);
                 sum += w * st[p].y;
                 const uint32_t src = pa_mapa(kv_s + (uint32_t)(r * C::PITCH + lane * 2) * 4, (uint32_t)p);
@@ -553,8 +559,34 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     acc[2 * e + 1] += w * v.y;
                 }
             }
+            bool fine = pa_finite(sum);
+#pragma unroll
+            for (int e = 0; e < D / 32; e++) fine = fine && pa_finite(acc[e]);
+            if (!__all_sync(0xffffffffu, fine)) again |= 1u << ((r - lo - warp) / (PA_THREADS / 32));
             const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;   // a row that sees nothing gives zeros, as on the CPU
             const int tok = (int)(row / a.group), head = hk * a.group + (int)(row - (int64_t)tok * a.group);
+            float *out = a.dst + ((int64_t)tok * a.n_head + head) * D + lane * 2;
+#pragma unroll
+            for (int e = 0; e < D / 64; e++) *(float2 *)(out + e * 64) = make_float2(acc[2 * e] * inv, acc[2 * e + 1] * inv);
+        }
+#pragma unroll 1
+        for (; again; again &= again - 1) {
+            const int r = lo + warp + (__ffs(again) - 1) * (PA_THREADS / 32);
+            const int64_t row = row0 + r;
+            const int tok = (int)(row / a.group), head = hk * a.group + (int)(row - (int64_t)tok * a.group);
+            const uint8_t *const k = a.k + (int64_t)hk * a.k_nb2, *const v = a.v + (int64_t)hk * a.v_nb2;
+            const uint16_t *const seen = a.mask ? (const uint16_t *)(a.mask + (int64_t)tok * a.mask_nb1) : nullptr;
+            float acc[D / 32], top, sum;
+            pa_row_again<D, false>(q_g, r, a.scale_log2, (int)a.n_kv, [&](int i, float *bias, const uint8_t **key, const uint8_t **value) {
+                if (seen) {
+                    if (seen[i] == 0xFC00) return false;
+                    *bias = f16_bits_to_f32(seen[i]) * PA_LOG2E;
+                }
+                *key = k + i * a.k_nb1;
+                *value = v + i * a.v_nb1;
+                return true;
+            }, acc, &top, &sum);
+            const float inv = sum == 0.0f ? 0.0f : 1.0f / sum;
             float *out = a.dst + ((int64_t)tok * a.n_head + head) * D + lane * 2;
 #pragma unroll
             for (int e = 0; e < D / 64; e++) *(float2 *)(out + e * 64) = make_float2(acc[2 * e] * inv, acc[2 * e + 1] * inv);
@@ -652,6 +684,12 @@ bool flash_attn_fast_prompt(const b200_flash_attn_args *a, cudaStream_t s, int *
     p.mask = (const unsigned char *)a->mask;
     p.mask_nb1 = a->mask_nb1;
     p.mask_wide = a->mask && a->mask_nb1 % 16 == 0 && ((uintptr_t)a->mask & 15) == 0;
+    p.k = (const unsigned char *)a->k;
+    p.v = (const unsigned char *)a->v;
+    p.k_nb1 = a->k_nb1;
+    p.k_nb2 = a->k_nb2;
+    p.v_nb1 = a->v_nb1;
+    p.v_nb2 = a->v_nb2;
     p.dst = a->dst;
     p.n_kv = a->n_kv;
     p.rows = rows;

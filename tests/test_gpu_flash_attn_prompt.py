@@ -150,3 +150,69 @@ def test_few_rows_that_the_decode_kernel_refuses_keep_their_precision(dev, H, Hk
     finally:
         dev.set_numerics(dev.EXACT)
     assert np.array_equal(got.view(np.uint32), cpu.view(np.uint32))
+
+
+def plain(q, k, v, mask, scale):
+    """float64, a row at a time over the positions it sees; a score of NaN or +Inf makes the row NaN"""
+    H, T, D = q.shape
+    G = H // k.shape[0]
+    kf, vf = k.view(np.float16).astype(np.float64), v.view(np.float16).astype(np.float64)
+    out = np.zeros((T, H, D))
+    for h in range(H):
+        for t in range(T):
+            see = np.arange(k.shape[1]) if mask is None else np.flatnonzero(mask[t] != 0xFC00)
+            if len(see) == 0:
+                continue
+            s = kf[h // G, see] @ q[h, t].astype(np.float16).astype(np.float64) * scale
+            if mask is not None:
+                s = s + mask[t, see].view(np.float16).astype(np.float64)
+            if not (s < np.inf).all():
+                out[t, h] = np.nan
+                continue
+            p = np.exp(s - s.max())
+            out[t, h] = (p / p.sum()) @ vf[h // G, see]
+    return out
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("H,Hkv,T,n_kv,causal", [(8, 2, 64, 256, True), (8, 2, 40, 2056, True), (4, 4, 130, 777, True), (6, 2, 70, 333, True), (8, 4, 96, 640, False)], ids=str)
+def test_values_that_are_not_finite(dev, D, H, Hkv, T, n_kv, causal):
+    """A NaN in a query makes its row NaN and no other; NaN and Inf in cells reach the rows that see them and no other, wherever the tiles end: hidden
+    from some rows of a tile, from a whole softmax group's tiles, from all rows of a cluster's CTA.  Rows that meet nothing of it keep their bits."""
+    scale = D ** -0.5
+    q, k, v, mask = synth_case(H, Hkv, D, T, n_kv, seed=D + T, causal=causal)
+    if mask is not None:
+        mask = mask.copy()
+        mask[:, 130:140] = 0xFC00        # cells that nobody sees, inside a tile that all see
+        mask[5, :] = 0xFC00
+    clean = dev.flash_attn(q, dev.KvCacheView(k, v), mask, scale, mode=1)
+    q, k, v = q.copy(), k.copy(), v.copy()
+    q[1, 7, 3] = np.nan                  # one head of one token
+    q[:, 5, 0] = np.nan                  # a token that sees nothing under the mask
+    if mask is not None:
+        k[:, 131], v[:, 132], v[:, 133, 1] = 0x7E00, 0x7E00, 0xFC00
+    v[0, n_kv - 3, 2] = 0x7C00           # Inf in one channel of a late position: hidden from most rows of a causal batch
+    k[Hkv - 1, n_kv - 9, 4] = 0x7E00     # a NaN key
+    got = dev.flash_attn(q, dev.KvCacheView(k, v), mask, scale, mode=1)
+    assert dev.kernel_error() == 0
+    with np.errstate(all="ignore"):
+        want = plain(q, k, v, mask, scale)
+    assert (np.isnan(got) == np.isnan(want)).all() and (np.isinf(got) == np.isinf(want)).all()
+    fine = np.isfinite(want).all(axis=2)
+    assert fine.any() and not fine.all()
+    assert row_rel(got[fine], want[fine]) <= TOL
+    if mask is None:
+        untouched = fine.copy()
+        untouched[:, H - H // Hkv:] = False
+        assert np.array_equal(got[untouched].view(np.uint32), clean[untouched].view(np.uint32))
+
+
+def test_a_softmax_group_and_a_cta_that_see_nothing_but_nan(dev):
+    """keys of tiles 1, 3, .. are NaN (one of two groups of softmax warps; with more tiles than row blocks, whole CTAs of a cluster): no row is finite"""
+    for n_kv, T in ((256, 64), (2048, 64), (2048, 300)):
+        q, k, v, _ = synth_case(4, 2, 128, T, n_kv, seed=n_kv + T, causal=False)
+        k = k.copy()
+        for t in range(1, n_kv // 128, 2):
+            k[:, 128 * t:128 * (t + 1)] = 0x7E00
+        got = dev.flash_attn(q, dev.KvCacheView(k, v), None, 0.09, mode=1)
+        assert np.isnan(got).all()
