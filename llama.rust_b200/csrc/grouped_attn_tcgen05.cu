@@ -9,6 +9,7 @@
 //     one after the other (a prompt's mostly do) come by one tensor-map copy of 32 rows, others by gathering copies of four rows each;
 //   * a weight stays a 32-bit value to 2^-17: it enters the second product as two BF16 parts, each half of the tensor-memory columns its score
 //     came from, with two sets of MMAs;
+//   * a row whose output is not finite is computed again from the entries it sees alone (pa_row_again): the products multiply hidden ones by 0;
 //   * what a row sees is arithmetic: only tiles at an edge of it compare entries, with three thresholds of the row's.
 // What it takes, beside the other kernel: at grouped_tc_takes.
 // Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device error word.
@@ -348,9 +349,10 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
         pa_fence_after();
         asm volatile("bar.sync 1, 256;" ::: "memory");
         const float ma = sh.ml[0][r][0], mb = sh.ml[1][r][0], mm = fmaxf(ma, mb);
-        // no output where the group had no tile or the row saw nothing in them
-        const float wa = ma == -INFINITY ? 0.0f : pa_ex2(ma - mm), wb = mb == -INFINITY ? 0.0f : pa_ex2(mb - mm);
-        const float lt = (ma == -INFINITY ? 0.0f : wa * sh.ml[0][r][1]) + (mb == -INFINITY ? 0.0f : wb * sh.ml[1][r][1]);
+        // no output where the group had no tile or the row saw nothing in them.  Their sum is 0 then, or NaN: a maximum does not show a NaN
+        const bool ina = ma != -INFINITY, inb = mb != -INFINITY;
+        const float wa = ina ? pa_ex2(ma - mm) : 1.0f, wb = inb ? pa_ex2(mb - mm) : 1.0f;
+        const float lt = wa * sh.ml[0][r][1] + wb * sh.ml[1][r][1];
         asm volatile("bar.sync 1, 256;" ::: "memory");
         if (g == 0) {
             sh.ml[0][r][0] = mm;
@@ -366,7 +368,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
                 pa_wait_ld();
 #pragma unroll
                 for (int e = 0; e < 32; e++) {
-                    const float u = wa != 0.0f ? wa * __uint_as_float(x[e]) : 0.0f, v = wb != 0.0f ? wb * __uint_as_float(y[e]) : 0.0f;
+                    const float u = ina ? wa * __uint_as_float(x[e]) : 0.0f, v = inb ? wb * __uint_as_float(y[e]) : 0.0f;
                     x[e] = __float_as_uint(u + v);
                 }
 #pragma unroll
@@ -385,6 +387,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
     float sinks[GA_M / 16];   // of the rows warp, warp + 16, ..: all on their way at once
 #pragma unroll
     for (int i = 0; i < GA_M / 16; i++) sinks[i] = a.sink ? a.sink[hk * group + (warp + 16 * i) % group] * 1.4426950408889634f : -INFINITY;
+    uint32_t again = 0;   // which of this warp's rows are not finite
 #pragma unroll
     for (int i = 0; i < GA_M / 16; i++) {
         const int x = warp + 16 * i, tok = x / group, head = hk * group + x - tok * group;
@@ -393,12 +396,41 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
         const float mf = fmaxf(m, sinks[i]), w = pa_ex2(m - mf), f = w / (lt * w + pa_ex2(sinks[i] - mf));
         const float *part = (const float *)(q_g + GA_M * D * 2) + (size_t)x * C::PITCH;
         Y *y = (Y *)a.y + (row0 + tok) * a.ldy + (int64_t)head * a.vdim;
+        bool fine = pa_finite(lt);
 #pragma unroll
         for (int c = 0; c < C::CHUNKS; c++) {
             const int j = 64 * c + 2 * lane;
             const float2 v = *(const float2 *)(part + j);
+            fine = fine && pa_finite(v.x) && pa_finite(v.y);
             if (j < a.vdim) y[j] = from_f32<Y>(v.x * f);
             if (j + 1 < a.vdim) y[j + 1] = from_f32<Y>(v.y * f);
+        }
+        if (!__all_sync(0xffffffffu, fine)) again |= 1u << i;
+    }
+#pragma unroll 1
+    for (; again; again &= again - 1) {
+        const int x = warp + 16 * (__ffs(again) - 1), tok = x / group, head = hk * group + x - tok * group, p = pos0 + tok;
+        const int h0 = min(en.kept - 1, p), l1 = max(en.kept, p - window - en.lo + en.kept + 1), h1 = min(en.total - 1, p - en.lo + en.kept);
+        const __nv_bfloat16 *const cache = (const __nv_bfloat16 *)a.cache + (int64_t)hk * (a.dim + a.vdim);
+        const int kept = sg[SEG_KEPT], key0 = sg[SEG_KEY0];
+        const int64_t tab0 = sg[SEG_TAB0];
+        float acc[D / 32], m, lt;
+        pa_row_again<D, true>(q_g, x, a.scale * 1.4426950408889634f, en.total, [&](int e, float *, const uint8_t **key, const uint8_t **value) {
+            if (!(e <= h0 || (e >= l1 && e <= h1))) return false;
+            const int at_pos = en.position(e);
+            const int64_t at = tab0 + (at_pos < kept ? at_pos : kept + at_pos - key0);
+            if ((at_pos >= kept && at_pos < key0) || at < 0 || at >= a.n_tab || a.tab[at] < 0 || a.tab[at] >= a.n_cells) return false;   // reported above
+            *key = (const uint8_t *)(cache + (int64_t)a.tab[at] * a.ldc);
+            *value = *key + 2 * a.dim;
+            return true;
+        }, acc, &m, &lt);
+        const float sink = a.sink ? a.sink[head] * 1.4426950408889634f : -INFINITY;
+        const float mf = fmaxf(m, sink), w = pa_ex2(m - mf), f = w / (lt * w + pa_ex2(sink - mf));
+        Y *y = (Y *)a.y + (row0 + tok) * a.ldy + (int64_t)head * a.vdim;
+#pragma unroll
+        for (int c = 0; c < C::CHUNKS; c++) {
+            y[64 * c + 2 * lane] = from_f32<Y>(acc[2 * c] * f);
+            y[64 * c + 2 * lane + 1] = from_f32<Y>(acc[2 * c + 1] * f);
         }
     }
 }

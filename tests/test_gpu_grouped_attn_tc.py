@@ -64,3 +64,24 @@ def test_cells_that_do_not_stand_together(ll):
         m.decode_seqs([a[i], b[i]], [i, i], [0, 1], [0])
     m.seq_rm(0)
     check(feed(m, toks, 280, 2), Expected(cfg, w, toks, "bfloat16"), "holes")
+
+
+@pytest.mark.parametrize("name", ["128, four heads a key head", "128, a head each, everything rotates", "64, two heads a key head"])
+def test_a_token_of_nan(ll, name):
+    """its query, key and value are NaN: the rows that see it are NaN (sinks or not), those before it and those that it has left the window of keep
+    what they are without it, in the tiles that hold it too"""
+    cfg = M.config([dict(CASES[name], mlp=None)], width=64, bigram=None)
+    w = M.weights(cfg, 37)
+    toks = np.array(M.tokens(cfg, 400, 38))
+    toks[toks == 100] = 99
+    bad = 170
+    clean = Expected(cfg, w, toks, "bfloat16")
+    toks[bad] = 100
+    w["embed"] = w["embed"].copy()
+    w["embed"][100, 3] = np.nan
+    mask = CASES[name]["mixer"]["mask"]
+    sees = np.array([i >= bad and i - bad < mask["size"] for i in range(400)])
+    got = feed(model(ll, cfg, w, "bfloat16"), toks, 400)[:, :100]   # (token 100's own logit is NaN in every row)
+    assert np.isnan(got[sees]).all() and np.isfinite(got[~sees]).all()
+    e = M.error(got[~sees], clean.rows[~sees][:, :100])
+    assert (e < clean.limit[~sees]).all()
