@@ -1,8 +1,8 @@
 // FLASH_ATTN_EXT, fast mode, prompt batches: attention on the tcgen05 tensor cores, head sizes 64 and 128.
 //
 //   softmax(q k^T * scale + mask) v        (crates/ggml/src/flash_attn.rs:482-736), for hosts that accept the tolerance asked of
-// F16-KV attention (1e-3): q is rounded to f16 as the CPU rounds it (flash_attn.rs:433), the weights are rounded to f16 for the
-// second product, everything else is F32.
+// F16-KV attention (1e-3): q is rounded to f16 as the CPU rounds it (flash_attn.rs:433), the weights of 64 and more query rows are rounded to
+// f16 for the second product, those of fewer rows go in as two f16 parts (SPLIT), everything else is F32.
 //   * A CTA takes 128 rows of one KV head, a row being (token, query head of the KV head's group) with the heads of a token adjacent,
 //     so that every K / V tile and every mask row is shared by the group.  Row r is lane r of tensor memory.
 //   * K and V come in tiles of 128 positions by TMA (128-byte swizzle; positions past the cache read as zeros), K a K-major and V an
@@ -11,15 +11,20 @@
 //     tensor memory), its own unnormalised output and its own running maximum and sum, so that one group's exponentials hide the
 //     other's products; the two are added at the end.  A thread owns a whole row: no exchange between threads.
 //   * The weights go back into tensor memory over the scores they came from, as the A operand of p v: shared memory carries K, V and q only.
-//   * The output is rescaled only when a row's maximum grows by more than 2^8 over the one in use: until then weights of up to 256 stand
-//     in F16 with the same relative rounding, and the sums are F32 either way.
+//   * With one-part weights the maximum in use is the running one, so that a row's largest weights are exactly 1 and lose nothing.  Let it lag
+//     by up to 2^8 and the output is rescaled less often (47 us for the 50 below), but those weights are rounded like any other: 2.05e-4 of
+//     float64 for 1.90e-4, and 1.36e-4 for 6.5e-5 with scores three times as wide (maxima per 64 positions, as mma.sync kernels have
+//     them: 1.93e-4 and 7.6e-5).  Two parts take no harm from it: there the output is rescaled only when a row's maximum grows by more than
+//     2^8 over the one in use, and the sums take the weights as they are.
+//   * Two parts cost 14 % at 512 rows over 4096 positions, 8 % at 16 over 2048; 5e-7 to 5e-6 of float64.  The decode kernel, which takes a maximum per
+//     16 positions, is 1.4e-4 away (2e-5 with wide scores, 3e-7 where each 16 hold one position that a row sees): one part would be further.
 //   * Six warps read the mask ahead of everyone and sort the CTA's (row block, tile) pairs into: all zero (no mask read at all in the
 //     softmax), all minus infinity (skipped by every role), mixed (each row reads its 128 mask values).
 //   * A row whose output is not finite is computed again from what it sees alone (pa_row_again): the tiles' products multiply hidden cells by 0.
 //   * The positions are dealt out to the CTAs of a cluster, tile by tile, where there are too few row blocks for the GPU; the
 //     partial outputs meet in shared memory and every CTA finishes its share of the rows.
 // Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device error word.
-// What bounds it (512 rows of 32 heads over 4096 positions, 8 KV heads of 128: 49 us; the mma.sync kernel in its place before took 169, 0.19 of
+// What bounds it (512 rows of 32 heads over 4096 positions, 8 KV heads of 128: 50 us; the mma.sync kernel in its place before took 169, 0.19 of
 // the rate the products alone would allow): a tile of 128 x 128 costs about 1850 SM clocks, 1024 of them exponentials (16 a clock) and as many
 // products, which two groups overlap only in part; and about 10 us of a launch are its beginning (q, the first tiles) and end.  On the way: one
 // lane that walked the tiles and issued the products with its descriptors in ordinary registers 67.8 us; the warp together, one elected
@@ -40,7 +45,6 @@ constexpr int PA_RING = 16;                            // tiles whose class the 
 constexpr int PA_MAX_SPLITS = 8;
 constexpr int PA_ERR_WAIT = 4;
 constexpr float PA_LOG2E = 1.4426950408889634f;
-constexpr float PA_LAZY = 8.0f;                        // log2 of the growth of a maximum that is let pass
 enum { PA_CLEAR = 0, PA_MIXED = 1, PA_HIDDEN = 2 };
 
 template <int D>
@@ -81,10 +85,11 @@ struct PaArgs {
     int *err;
 };
 
-template <int D>
+template <int D, bool SPLIT>
 __global__ void __launch_bounds__(PA_THREADS, 1)
 fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, const PaArgs a) {
     using C = PaCfg<D>;
+    constexpr float LAZY = SPLIT ? 8.0f : 0.0f;   // log2 of the growth of a maximum that is let pass
     extern __shared__ uint8_t pa_raw[];
     __shared__ PaShared sh;
     pdl_trigger();
@@ -251,9 +256,11 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 pa_fence_after();
                 if (leader) {
 #pragma unroll
-                    for (int ks = 0; ks < PA_N / 16; ks++)
-                        pa_mma_ts(tmem + C::O_COL + (uint32_t)(g * D), tmem + (uint32_t)(g * PA_N + ks * 8), v_desc + (uint32_t)(s * (C::TILE >> 4) + ks * 128), C::IDESC_O,
-                                  j > 0 || ks > 0);
+                    for (int part = 0; part < (SPLIT ? 2 : 1); part++)   // the weights' high parts, then their low parts
+#pragma unroll
+                        for (int ks = 0; ks < PA_N / 16; ks++)
+                            pa_mma_ts(tmem + C::O_COL + (uint32_t)(g * D), tmem + (uint32_t)(g * PA_N + part * 64 + ks * 8), v_desc + (uint32_t)(s * (C::TILE >> 4) + ks * 128),
+                                      C::IDESC_O, j > 0 || ks > 0 || part > 0);
                     pa_commit(&sh.empty[s]);
                 }
                 seq++;
@@ -443,7 +450,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             if (j == 0) {
                 m = top;
             } else {
-                const bool grow = top > m + PA_LAZY;   // also when nothing was seen before
+                const bool grow = top > m + LAZY;   // also when nothing was seen before
                 if (__any_sync(0xffffffffu, grow)) {
                     // the group's former product is complete: the scores that were waited for were issued behind it
                     const float al = grow ? pa_ex2(m - top) : 1.0f;
@@ -466,18 +473,26 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             const uint64_t sc2 = pa_pair(sc, sc), sub2 = pa_pair(-sub, -sub);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                uint32_t p[32];
+                uint32_t p[32], low[SPLIT ? 32 : 1];
 #pragma unroll
                 for (int c = 0; c < 32; c++) {
                     const float2 x = pa_split(pa_fma2(pa_pair(__uint_as_float(s[64 * h + 2 * c]), __uint_as_float(s[64 * h + 2 * c + 1])), sc2, sub2));
-                    const __half2 w = __floats2half2_rn(pa_ex2(x.x), pa_ex2(x.y));
-                    // the sum takes the weights as the second product will see them (rounded to f16): what is common to a row's
-                    // numerator and denominator cancels
+                    const float2 e = make_float2(pa_ex2(x.x), pa_ex2(x.y));
+                    const __half2 w = __floats2half2_rn(e.x, e.y);
                     const float2 f = __half22float2(w);
-                    ps[c & 1] = pa_add2(ps[c & 1], pa_pair(f.x, f.y));
                     p[c] = *(const uint32_t *)&w;
+                    if (SPLIT) {
+                        const __half2 rest = __floats2half2_rn(e.x - f.x, e.y - f.y);
+                        low[SPLIT ? c : 0] = *(const uint32_t *)&rest;
+                        ps[c & 1] = pa_add2(ps[c & 1], pa_pair(e.x, e.y));
+                    } else {
+                        // the sum takes the weights as the second product will see them (rounded to f16): what is common to a row's
+                        // numerator and denominator cancels
+                        ps[c & 1] = pa_add2(ps[c & 1], pa_pair(f.x, f.y));
+                    }
                 }
                 pa_st32(t_s + (uint32_t)(32 * h), p);
+                if (SPLIT) pa_st32(t_s + (uint32_t)(64 + 32 * h), low);
             }
             const float2 p0 = pa_split(ps[0]), p1 = pa_split(ps[1]);
             l += (p0.x + p1.x) + (p0.y + p1.y);
@@ -619,7 +634,7 @@ bool cache_map(CUtensorMap *map, const void *base, int D, int64_t heads, int64_t
     return cache_tile_map(map, base, D, heads, n_kv, nb1, nb2, PA_N);
 }
 
-template <int D>
+template <int D, bool SPLIT>
 int launch(const CUtensorMap &km, const CUtensorMap &vm, PaArgs &p, int64_t blocks, int64_t heads, int dev, cudaStream_t s) {
     static std::mutex mu;
     static int clusters[64][PA_MAX_SPLITS];
@@ -627,7 +642,7 @@ int launch(const CUtensorMap &km, const CUtensorMap &vm, PaArgs &p, int64_t bloc
     {
         std::lock_guard<std::mutex> lk(mu);
         if (!known[dev]) {
-            B200_CUDA(cudaFuncSetAttribute(fa_prompt_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaCfg<D>::SMEM));
+            B200_CUDA(cudaFuncSetAttribute(fa_prompt_kernel<D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaCfg<D>::SMEM));
             B200_CUDA(cudaDeviceGetAttribute(&clusters[dev][0], cudaDevAttrMultiProcessorCount, dev));
             for (int n = 2; n <= PA_MAX_SPLITS; n++) {
                 cudaLaunchConfig_t cfg = {};
@@ -640,7 +655,7 @@ int launch(const CUtensorMap &km, const CUtensorMap &vm, PaArgs &p, int64_t bloc
                 cfg.dynamicSmemBytes = PaCfg<D>::SMEM;
                 cfg.attrs = attr;
                 cfg.numAttrs = 1;
-                if (cudaOccupancyMaxActiveClusters(&clusters[dev][n - 1], fa_prompt_kernel<D>, &cfg) != cudaSuccess) {
+                if (cudaOccupancyMaxActiveClusters(&clusters[dev][n - 1], fa_prompt_kernel<D, SPLIT>, &cfg) != cudaSuccess) {
                     cudaGetLastError();
                     clusters[dev][n - 1] = 0;
                 }
@@ -650,8 +665,8 @@ int launch(const CUtensorMap &km, const CUtensorMap &vm, PaArgs &p, int64_t bloc
     }
     p.splits = pick_splits(blocks * heads, p.n_tiles, clusters[dev]);
     const dim3 grid((unsigned)(blocks * p.splits), (unsigned)heads);
-    if (p.splits == 1) return launch_pdl(fa_prompt_kernel<D>, grid, dim3(PA_THREADS), PaCfg<D>::SMEM, s, km, vm, p);
-    return launch_pdl_cluster(fa_prompt_kernel<D>, grid, dim3(PA_THREADS), (unsigned)p.splits, PaCfg<D>::SMEM, s, km, vm, p);
+    if (p.splits == 1) return launch_pdl(fa_prompt_kernel<D, SPLIT>, grid, dim3(PA_THREADS), PaCfg<D>::SMEM, s, km, vm, p);
+    return launch_pdl_cluster(fa_prompt_kernel<D, SPLIT>, grid, dim3(PA_THREADS), (unsigned)p.splits, PaCfg<D>::SMEM, s, km, vm, p);
 }
 
 }  // namespace
@@ -700,7 +715,9 @@ bool flash_attn_fast_prompt(const b200_flash_attn_args *a, cudaStream_t s, int *
     // a row's maximum is taken before the scale, which must then not be negative: its sign goes to q
     p.scale_log2 = fabsf(a->scale) * PA_LOG2E;
     p.q_sign = a->scale < 0.0f ? -1.0f : 1.0f;
-    *rc = D == 128 ? launch<128>(km, vm, p, blocks, a->n_head_kv, dev, s) : launch<64>(km, vm, p, blocks, a->n_head_kv, dev, s);
+    // two-part weights where the decode kernel's are the measure (the caller sends it 2 to 63 rows)
+    if (a->n_tok < 64) *rc = D == 128 ? launch<128, true>(km, vm, p, blocks, a->n_head_kv, dev, s) : launch<64, true>(km, vm, p, blocks, a->n_head_kv, dev, s);
+    else *rc = D == 128 ? launch<128, false>(km, vm, p, blocks, a->n_head_kv, dev, s) : launch<64, false>(km, vm, p, blocks, a->n_head_kv, dev, s);
     return true;
 }
 

@@ -2,8 +2,8 @@
 over one to eight CTAs, mask rows on and off 16-byte boundaries, tiles that are clear, hidden or mixed, running maxima that grow (-m gpu).
 
 Tolerance, per output row relative to the row's largest magnitude, against float64 with q rounded to f16 (as the operation rounds it): the weights
-are rounded to f16 before the second product and in the sum alike, 2^-11 of each weight, which over a row gives at most 2 * 2^-11 = 9.8e-4
-of the largest |v|; 1e-3 as asked of F16-KV attention."""
+of 64 and more rows are rounded to f16 before the second product and in the sum alike, 2^-11 of each weight, which over a row gives at most
+2 * 2^-11 = 9.8e-4 of the largest |v|; 1e-3 as asked of F16-KV attention."""
 import ctypes as C
 
 import numpy as np
@@ -216,3 +216,42 @@ def test_a_softmax_group_and_a_cta_that_see_nothing_but_nan(dev):
             k[:, 128 * t:128 * (t + 1)] = 0x7E00
         got = dev.flash_attn(q, dev.KvCacheView(k, v), None, 0.09, mode=1)
         assert np.isnan(got).all()
+
+
+def q16(q):
+    return q.astype(np.float16).astype(np.float32)
+
+
+def norm_rel(got, want):
+    return float(np.linalg.norm(got - want) / np.linalg.norm(want))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("wide", [1.0, 3.0])
+@pytest.mark.parametrize("T,n_kv", [(64, 4096), (300, 1500)])
+def test_weights_of_prompts_lose_no_more_than_under_running_maxima(dev, T, n_kv, wide, D):
+    """the limit is the distance that rounding each weight to f16 under the running maximum of 64-position tiles alone makes, and a twentieth"""
+    H, Hkv = 8, 4
+    q, k, v, mask = synth_case(H, Hkv, D, T, n_kv, seed=T + D)
+    q, scale = q * wide / q.std(), D ** -0.5 / k.view(np.float16).astype(np.float32).std()
+    want = ref64(q16(q), k, v, mask, scale)
+    kf, vf, m = k.view(np.float16).astype(np.float64), v.view(np.float16).astype(np.float64), mask.view(np.float16).astype(np.float64)
+    rounded = np.empty_like(want)
+    for h in range(H):
+        s = q16(q)[h].astype(np.float64) @ kf[h // 2].T * scale + m
+        top = np.stack([s[:, :64 * (t // 64 + 1)].max(axis=1) for t in range(0, n_kv, 64)], axis=1).repeat(64, axis=1)[:, :n_kv]
+        w = np.exp(s - top).astype(np.float16) * np.exp(top - s.max(axis=1, keepdims=True))
+        rounded[:, h] = (w / w.sum(axis=1, keepdims=True)) @ vf[h // 2]
+    got = dev.flash_attn(q, dev.KvCacheView(k, v), mask, scale, mode=1)
+    assert norm_rel(got, want) <= 1.05 * norm_rel(rounded, want)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("wide", [1.0, 3.0])
+@pytest.mark.parametrize("T,n_kv", [(2, 1024), (16, 2048), (63, 4096)])
+def test_weights_of_a_few_rows_are_two_parts(dev, T, n_kv, wide, D):
+    """weights to 2^-22 of themselves and 2^-25 of the largest, sums of up to 4096 F32 terms: 1e-5, where f16 weights are 2e-4 away"""
+    q, k, v, mask = synth_case(8, 2, D, T, n_kv, seed=T + D)
+    q, scale = q * wide / q.std(), D ** -0.5 / k.view(np.float16).astype(np.float32).std()
+    got = dev.flash_attn(q, dev.KvCacheView(k, v), mask, scale, mode=1)
+    assert norm_rel(got, ref64(q16(q), k, v, mask, scale)) <= 1e-5
