@@ -14,8 +14,10 @@
 //   per super-block, where the exact kernels' chains take four or eight.
 //   Q8_0, Q4_0, MXFP4: the exact integer dot of each 32-element block times d_w d_x (exact in f32 for f16 scales), added in f32; the dot comes
 //   out of the product as a float already (the accumulator starts at the bits of 1.5 * 2^23).
-// Every output is within a few f32 roundings of the exact sum over the quantized operands: 7e-8 to 1.2e-7 of the result's norm at K = 4096 and
-// 14336, where the chains it stands in for are 7e-8 to 6.9e-7 away.
+// Every output is within a few f32 roundings of the exact sum over the quantized operands: from float64, of the result's norm, at K = 2048, 4096 and
+// 14336, Q4_K 9e-8 / 9e-8 / 1.0e-7 where the chains it stands in for are 3e-7 / 4.5e-7 / 9e-7, Q6_K 5.4e-8 / 6.1e-8 / 6.8e-8 (5.8e-8 / 7.8e-8 / 1.4e-7),
+// Q8_0 and Q4_0 7e-8 / 8e-8 / 1.1e-7 (1.4e-7 / 2.0e-7 / 3.8e-7), MXFP4 6e-8 / 6e-8 / 9e-8 (1.1e-7 / 1.8e-7 / 3.6e-7).  (Q6_K short rows: added up warp
+// after warp, and with a super-block's product rounded before it meets the activation's scale, they were 6.5e-8.)
 // What was tried: 32 columns per CTA (128 registers: spills; 255: one CTA per SM; both slower than two passes of 16 columns), a warp per tile in place
 // of shared tiles (no change), 8-byte activation fragments straight from L2 (slower by a tenth at 16 columns), a CTA per tile without the
 // walk (28672 x 4096 on 16 rows 30 us, so 27), scales fetched byte by byte.  Figures against the other kernels: at few_takes below.
@@ -100,6 +102,7 @@ __device__ __forceinline__ uint64_t few_add2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ float few_or_zero(float x) { return fabsf(x) < INFINITY ? x : 0.0f; }
 // the integers 0 .. 63 in two bytes of x as f16
 __device__ __forceinline__ uint32_t few_byte_f16x2(uint32_t x, uint32_t selector) {
     const uint32_t h = __byte_perm(x, 0x64646464u, selector);   // 1024 + byte
@@ -333,6 +336,7 @@ struct FewChunk {
         const int lane = threadIdx.x & 31, g8 = lane >> 2, t = lane & 3;
         uint32_t mn[2][2][2];
         float dw[2][2], dm[2][2];
+        uint64_t dr2[2][2];   // Q6_K: for what rounding a product leaves out, which is added first (an infinite scale has none)
 #pragma unroll
         for (int mt = 0; mt < 2; mt++)
 #pragma unroll
@@ -347,13 +351,14 @@ struct FewChunk {
                     mn[mt][r][1] = few_byte_f16x2(((x.w >> 4) & 0x0f0f0f0fu) | (((x.z >> 6) & 0x03030303u) << 4), sel);
                 } else {
                     dw[mt][r] = f16_bits_to_f32(*(const uint16_t *)(w + 6656 + row * 2));
+                    dr2[mt][r] = few_pair(few_or_zero(dw[mt][r]), few_or_zero(dw[mt][r]));
                 }
             }
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) {
             if (GROUPED && nt >= nt_live) continue;
             const float d0 = __shfl_sync(0xffffffffu, dx[nt], 8 * t), d1 = __shfl_sync(0xffffffffu, dx[nt], 8 * t + 4);   // of columns 2 t and 2 t + 1
-            const uint64_t dx2 = few_pair(d0, d1);
+            const uint64_t dx2 = few_pair(d0, d1), dxr2 = few_pair(few_or_zero(d0), few_or_zero(d1));
             uint32_t b0 = 0, b1 = 0;
             if (TYPE == B200_TYPE_Q4_K) {
                 b0 = few_short_f16x2(bs[nt][0]);
@@ -366,8 +371,10 @@ struct FewChunk {
 #pragma unroll
                 for (int r = 0; r < 2; r++) {
                     const int *i2 = &ig[KQ ? mt : 0][KQ ? nt : 0][2 * r];
-                    uint64_t v = few_mul2(few_pair((float)i2[0], (float)i2[1]), few_pair(dw[mt][r], dw[mt][r]));
+                    const uint64_t i2f = few_pair((float)i2[0], (float)i2[1]), d2 = few_pair(dw[mt][r], dw[mt][r]);
+                    uint64_t v = few_mul2(i2f, d2);
                     if (TYPE == B200_TYPE_Q4_K) v = few_fma2(few_pair(mg[2 * r], mg[2 * r + 1]), few_pair(dm[mt][r], dm[mt][r]), v);
+                    else acc[mt][nt][r] = few_fma2(few_fma2(i2f, dr2[mt][r], few_mul2(i2f, dr2[mt][r]) ^ 0x8000000080000000ull), dxr2, acc[mt][nt][r]);
                     acc[mt][nt][r] = few_fma2(v, dx2, acc[mt][nt][r]);
                 }
             }
@@ -387,7 +394,7 @@ gemm_few_kernel(const FewArgs a) {
     const int rank = (int)(blockIdx.x % (unsigned)a.splits), idx = (int)(blockIdx.x / (unsigned)a.splits);
     // row tiles first, first + walkers, .. of the launch, for one column block
     const int block = GROUPED ? idx / a.walkers : idx % a.col_blocks, first = GROUPED ? idx - block * a.walkers : idx / a.col_blocks;
-    // A tile's groups in 16 classes, b % 16, each summed in order by one warp; an output is the sum over w of (class w + class w + 8), whether
+    // A tile's groups in 16 classes, b % 16, each summed in order by one warp; an output is the sum, by halves, over w of (class w + class w + 8), whether
     // this CTA has all of them (a warp class w, then class w + 8) or the CTAs of a pair have eight each: the same bits either way
     const int c0 = warp + 8 * rank, n0 = c0 < a.nb ? (a.nb - 1 - c0) / 16 + 1 : 0;
     const int n1 = a.splits == 1 && warp + 8 < a.nb ? (a.nb - 9 - warp) / 16 + 1 : 0, mine = n0 + n1;
@@ -527,9 +534,10 @@ gemm_few_kernel(const FewArgs a) {
         if (a.splits == 1) {
             for (int i = tid; i < nt_live * 8 * 32; i += FEW_THREADS) {
                 const int at = (i >> 5) * FEW_PITCH + (i & 31);
-                float v = 0.0f;
-                for (int p = 0; p < w0; p++) v += p < w1 ? first_sums[p * PLANE + at] + red[p * PLANE + at] : red[p * PLANE + at];
-                store(i >> 5, i & 31, v);
+                float v[8];
+#pragma unroll
+                for (int p = 0; p < 8; p++) v[p] = p < w1 ? first_sums[p * PLANE + at] + red[p * PLANE + at] : p < w0 ? red[p * PLANE + at] : 0.0f;
+                store(i >> 5, i & 31, ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
             }
             __syncthreads();   // the sums have been read: the next tile's activations may be staged
         } else {
@@ -546,11 +554,10 @@ gemm_few_kernel(const FewArgs a) {
                     if (p < w0) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x[2 * p]) : "r"(p0 + at + p * PLANE * 4) : "memory");
                     if (p < w1) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x[2 * p + 1]) : "r"(p1 + at + p * PLANE * 4) : "memory");
                 }
-                float v = 0.0f;
+                float v[8];
 #pragma unroll
-                for (int p = 0; p < 8; p++)
-                    if (p < w0) v += p < w1 ? x[2 * p] + x[2 * p + 1] : x[2 * p];
-                store(i >> 5, i & 31, v);
+                for (int p = 0; p < 8; p++) v[p] = p < w1 ? x[2 * p] + x[2 * p + 1] : x[2 * p];
+                store(i >> 5, i & 31, ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
             }
             // nobody's sums change or go while the other reads them
             asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");

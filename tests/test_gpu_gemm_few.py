@@ -119,3 +119,33 @@ def test_experts(dev, fast, ty, experts, top, tokens, ne11):
         for s in range(top):
             lim = bound(ty, W[ids[t, s]], k, B[t, s % ne11][None])[0]
             assert (np.abs(got[t, s].astype(np.float64) - want[t, s]) <= lim).all()
+
+
+def exact_q6_K(W, x):
+    """[m, n] in float64 over the quantized operands: six-bit codes, int8 scales, f16 and f32 factors as they are"""
+    n, m, k = W.shape[0], x.shape[0], x.shape[1]
+    b = W.reshape(n, -1, 210)
+    lo, hi, s = b[..., :128].astype(int), b[..., 128:192].astype(int), b[..., 192:208].copy().view(np.int8).astype(np.float64)
+    q = np.empty(b.shape[:2] + (2, 4, 32))
+    for half in range(2):
+        for part in range(4):
+            byte = lo[..., 64 * half + 32 * (part & 1):][..., :32]
+            q[..., half, part, :] = ((byte >> 4 if part >= 2 else byte & 15) | (hi[..., 32 * half:32 * half + 32] >> 2 * part & 3) << 4) - 32
+    w = q.reshape(b.shape[:2] + (16, 16)) * s[..., None] * b[..., 208:210].copy().view(np.float16).astype(np.float64)[..., None]
+    a = np.frombuffer(b"".join(np.ascontiguousarray(orc.quantize_q8_K(r)).tobytes() for r in x), np.uint8).reshape(m, -1, 292)
+    a = a[..., :4].copy().view(np.float32).astype(np.float64) * a[..., 4:260].copy().view(np.int8)
+    return a.reshape(m, k) @ w.reshape(n, k).T
+
+
+@pytest.mark.parametrize("k", [256, 512, 1024, 2048, 4096])
+@pytest.mark.parametrize("m", [8, 48])
+def test_q6_k_is_no_further_from_exact_than_the_chain(dev, fast, k, m):
+    """rows of a few super-blocks, where the exact kernels' chain of one fma each is the most accurate: distances over 256 x m outputs, a twentieth for
+    their spread"""
+    W = synth.weights(orc.Q6_K, 256, k, seed=k)
+    x = synth.activations(m, k, seed=m)
+    chain, route = orc.mul_mat(orc.Q6_K, W, x)
+    assert route == orc.ROUTE_TILED
+    want = exact_q6_K(W, x)
+    got = dev.mul_mat(dev.Weight(orc.Q6_K, W, k), x)
+    assert np.linalg.norm(got - want) <= 1.05 * np.linalg.norm(chain - want)
