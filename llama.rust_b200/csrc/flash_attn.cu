@@ -671,11 +671,19 @@ extern "C" int b200_flash_attn_ext(const struct b200_flash_attn_args *args, void
         // What the decode kernel does not take (heads in groups that do not divide 16, mask rows off 4 bytes) keeps the kernels below, which read
         // q and the weights in F32, or as the CPU does, and no position that a row does not see.
         if (fa_decode_mma_enabled() && flash_attn_decode_mma_takes(args)) {
-            // Two to 63 rows.  The prompt kernel computes 128 rows at a time with its positions over a cluster, the decode kernel 16 rows (whole
-            // tokens) that skip what none of them sees.  32 heads of 128 on 8 KV heads, us decode / prompt kernel: a causal batch of 16 rows
-            // over 2048 positions 22.8 / 13.1, 8192 36 / 19, 32768 95 / 44 (63 rows 344 / 60); sequences that see a 16th each 19.1 / 12.6,
-            // 22.7 / 21.9, 46 / 60 (of 63 sequences 66 / 52).  Above 8192 positions so few rows are more likely sequences than a prompt's.
-            const bool wide = args->n_tok > 1 && (args->n_kv <= 8192 || args->n_tok >= 32);
+            // The prompt kernel computes 128 rows at a time with its positions over a cluster, the decode kernel 16 rows (whole tokens) that skip what
+            // none of them sees; the host does not know whether the rows are a prompt's or sequences', each with a stretch of its own.  Measured on
+            // both, on rows of unequal stretches and on alternating cells, in ten groupings of heads; us, decode / prompt kernel, 32 heads of 128 on
+            // 8 KV heads, 16 rows: 512 positions 15.3 / 11.6 (sequences 14.6 / 11.7), 2048 20.5 / 13.2 (17.7 / 13.2), 4096 25 / 16 (20 / 16).
+            //   * Fewer than 12 rows leave most of the 128 empty (32 heads on 32, 8 rows over 4096: 26 / 29 where one row has most cells).
+            //   * Small launches lose to the cluster's beginning and end: 8 heads on 2, 16 rows over 512 positions 10.6 / 11.7, 48 over 256 11.2 / 16.
+            //   * Above 4096 positions sequences are the decode kernel's, which walks each one's tiles alone: 32 of them over 8192 20 / 23, over
+            //     32768 50 / 69 (16 heads on 4: 29 / 67), although a prompt's rows would be quicker here (56 / 23, 180 / 56).  With about 2000
+            //     (row, head) pairs either is quicker here: 63 rows of 32 heads over 8192 21 / 21 (95 / 27), over 32768 65 / 57 (342 / 71).
+            //   * With heads of 64 the decode kernel has half as much to do and this one the same exponentials: 8 heads on 1, 24 rows over 512
+            //     positions 8.6 / 11.2, 48 sequences over 1536 with 8 heads on 2 10.6 / 11.7, 63 over 4096 on one key head 18 / 21.
+            const int64_t pairs = args->n_tok * args->n_head;
+            const bool wide = args->dk == 128 && args->n_tok >= 12 && args->n_kv >= 512 && (args->n_kv <= 4096 ? pairs * args->n_kv >= 12 * 8 * 1024 : pairs >= 2000);
             if (wide && flash_attn_fast_prompt(args, (cudaStream_t)stream, &rc)) return rc;
             if (flash_attn_decode_mma(args, (cudaStream_t)stream, &rc)) return rc;
         }

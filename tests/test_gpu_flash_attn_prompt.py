@@ -174,8 +174,10 @@ def plain(q, k, v, mask, scale):
     return out
 
 
-@pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("H,Hkv,T,n_kv,causal", [(8, 2, 64, 256, True), (8, 2, 40, 2056, True), (4, 4, 130, 777, True), (6, 2, 70, 333, True), (8, 4, 96, 640, False)], ids=str)
+NOT_FINITE = [(8, 2, 64, 256, True), (8, 2, 40, 2056, True), (8, 2, 16, 1032, True), (4, 4, 130, 777, True), (6, 2, 70, 333, True), (8, 4, 96, 640, False)]
+
+
+@pytest.mark.parametrize("D,H,Hkv,T,n_kv,causal", [(D, *c) for D in (64, 128) for c in NOT_FINITE if D == 128 or c[2] >= 64], ids=str)   # (fewer rows of 64: another kernel)
 def test_values_that_are_not_finite(dev, D, H, Hkv, T, n_kv, causal):
     """A NaN in a query makes its row NaN and no other; NaN and Inf in cells reach the rows that see them and no other, wherever the tiles end: hidden
     from some rows of a tile, from a whole softmax group's tiles, from all rows of a cluster's CTA.  Rows that meet nothing of it keep their bits."""
@@ -246,12 +248,23 @@ def test_weights_of_prompts_lose_no_more_than_under_running_maxima(dev, T, n_kv,
     assert norm_rel(got, want) <= 1.05 * norm_rel(rounded, want)
 
 
-@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("wide", [1.0, 3.0])
-@pytest.mark.parametrize("T,n_kv", [(2, 1024), (16, 2048), (63, 4096)])
-def test_weights_of_a_few_rows_are_two_parts(dev, T, n_kv, wide, D):
-    """weights to 2^-22 of themselves and 2^-25 of the largest, sums of up to 4096 F32 terms: 1e-5, where f16 weights are 2e-4 away"""
+@pytest.mark.parametrize("T,n_kv", [(12, 1024), (16, 2049), (63, 4096)])
+def test_weights_of_a_few_rows_are_two_parts(dev, T, n_kv, wide):
+    """weights to 2^-22 of themselves and 2^-25 of the largest, sums of up to 4096 F32 terms: 1e-5, where f16 weights are 2e-4 away (2049 positions: mask
+    rows off 4 bytes, the kernel in F32)"""
+    D = 128
     q, k, v, mask = synth_case(8, 2, D, T, n_kv, seed=T + D)
     q, scale = q * wide / q.std(), D ** -0.5 / k.view(np.float16).astype(np.float32).std()
     got = dev.flash_attn(q, dev.KvCacheView(k, v), mask, scale, mode=1)
-    assert norm_rel(got, ref64(q16(q), k, v, mask, scale)) <= 1e-5
+    assert norm_rel(got, ref64(q16(q) if n_kv % 2 == 0 else q, k, v, mask, scale)) <= 1e-5
+
+
+@pytest.mark.parametrize("T,H,Hkv,D,n_kv,prompt_kernel", [(11, 32, 8, 128, 2048, False), (12, 32, 8, 128, 2048, True), (12, 32, 8, 128, 510, False), (16, 8, 2, 128, 512, False),
+                                                          (16, 32, 8, 64, 2048, False), (32, 32, 8, 128, 4096, True), (32, 32, 8, 128, 4098, False), (63, 32, 8, 128, 4098, True)], ids=str)
+def test_which_few_rows_it_takes(dev, T, H, Hkv, D, n_kv, prompt_kernel):
+    """told apart by their distance from float64: f16 weights under maxima of 16 positions (the decode kernel), or two parts"""
+    q, k, v, mask = synth_case(H, Hkv, D, T, n_kv, seed=T + n_kv)
+    got = dev.flash_attn(q, dev.KvCacheView(k, v), mask, D ** -0.5, mode=1)
+    e = norm_rel(got, ref64(q16(q), k, v, mask, D ** -0.5))
+    assert e <= 1e-5 if prompt_kernel else 2e-5 < e <= 2.5e-4
