@@ -121,6 +121,8 @@ int b200_prompt_kernel_choice(int64_t n, int64_t m, int sm_count);
 /* The same for Q4_0, Q8_0 (fast numerics) and MXFP4 mat-muls of 8 and more activation rows: 0 = integer tcgen05 kernel, 64 / 128 = the f16
  * tcgen05 kernel with that many activation rows per tile (both give the same bits); -1 = bad arguments. */
 int b200_block32_kernel_choice(int type, int64_t n, int64_t m, int sm_count);
+/* The same for quantized mat-muls of 2 and more activation rows under the fast numerics: 1 = the few-rows kernel, 0 = another; -1 = bad arguments. */
+int b200_few_rows_kernel_choice(int type, int64_t n, int64_t k, int64_t m, int sm_count);
 /* The same for BF16 mat-muls of more than 16 activation rows: 64 / 128 / 256 = tiles of 128 weight rows and that many activation rows, 2 = tiles
  * of 256 x 256 by pairs of SMs; -1 = bad arguments. */
 int b200_bf16_kernel_choice(int64_t n, int64_t k, int64_t m, int sm_count);
@@ -190,9 +192,11 @@ int b200_mul_mat_q8(int type, int64_t n, int64_t k, int64_t m, const void *dev_w
  * (crates/llama/src/graph_arch.rs:209,226; crates/ggml/src/compute.rs:1174) without a second kernel. */
 int b200_mul_mat_q8_add(int type, int64_t n, int64_t k, const void *dev_w, const void *dev_act, int act_kind, float *dev_dst,
                         const float *dev_addend, float *dev_sum, int route, void *stream);
-/* The same for the 8 to 31 activation rows of a batched decode step (a multiple of 4 for Q4_K): every row c also gets
- * dev_sum[c * ld_sum + i] = dst[c * lddst + i] + dev_addend[c * ld_addend + i].  Only the shapes the few-rows kernels take:
- * b200_mul_mat_q8_rows_add_fusable says (1 / 0) whether (type, n weight rows, m activation rows) is one; the call refuses the others. */
+/* The same for the activation rows of a batched decode step, up to 31: every row c also gets dev_sum[c * ld_sum + i] = dst[c * lddst + i] +
+ * dev_addend[c * ld_addend + i].  Only the shapes the few-rows kernels take: b200_mul_mat_q8_rows_add_fusable says (1 / 0) whether (type, n weight
+ * rows, m activation rows) is one; the call refuses the others.  Under the fast numerics these are all types from 2 rows on while m * k / 256 is
+ * below 2^24 (longer rows are refused, except as follows); under the exact ones, and of any length, Q4_K (n a multiple of 8, m of 4) and Q6_K
+ * from 8 rows on. */
 int b200_mul_mat_q8_rows_add_fusable(int type, int64_t n, int64_t m);
 int b200_mul_mat_q8_rows_add(int type, int64_t n, int64_t k, int64_t m, const void *dev_w, const void *dev_act, int act_kind, float *dev_dst,
                              int64_t lddst, const float *dev_addend, int64_t ld_addend, float *dev_sum, int64_t ld_sum, void *stream);

@@ -214,6 +214,10 @@ int b200_debug_decode_step_times(unsigned long long *out, int n) { return decode
 void b200_debug_decode_step_wait(int spin_limit, int skip_cta, int skip_barrier) { decode_persistent_debug(spin_limit, skip_cta, skip_barrier); }
 
 int b200_prompt_kernel_choice(int64_t n, int64_t m, int sm_count) { return gemm_chain_pick_for(n, m, sm_count); }
+int b200_few_rows_kernel_choice(int type, int64_t n, int64_t k, int64_t m, int sm_count) {
+    if (!is_quant_type(type) || n <= 0 || k <= 0 || k % GROUP_K || m <= 0 || sm_count <= 0) return -1;
+    return few_takes_for(type, pick_route(type, n, m), n, k, m, sm_count) ? 1 : 0;
+}
 int b200_bf16_kernel_choice(int64_t n, int64_t k, int64_t m, int sm_count) { return n <= 0 || k <= 0 || m <= 0 || sm_count <= 0 ? -1 : gemm_bf16_pick_for(n, k, m, sm_count); }
 int b200_block32_kernel_choice(int type, int64_t n, int64_t m, int sm_count) {
     if ((type != B200_TYPE_Q4_0 && type != B200_TYPE_Q8_0 && type != B200_TYPE_MXFP4) || n <= 0 || m <= 0 || sm_count <= 0) return -1;

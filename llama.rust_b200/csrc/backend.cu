@@ -707,7 +707,7 @@ static bool fuses_mul_mat_rows_add(const ggml_tensor *mm, const ggml_tensor *add
     const ggml_tensor *other = add->src[0] == mm ? add->src[1] : add->src[1] == mm ? add->src[0] : nullptr;
     if (!other || other == mm || !same_shape(other, mm) || !other->data || !add->data) return false;
     if (mm->nb[0] != 4 || other->nb[0] != 4 || add->nb[0] != 4 || other->type != B200_TYPE_F32 || add->type != B200_TYPE_F32) return false;
-    if (w->ne[0] >= (1ll << 27) || !b200_mul_mat_q8_rows_add_fusable(w->type, w->ne[1], mm->ne[1])) return false;   // few_takes' 32-bit offsets
+    if (mm->ne[1] * (w->ne[0] / GROUP_K) >= FEW_ACT_GROUPS || !b200_mul_mat_q8_rows_add_fusable(w->type, w->ne[1], mm->ne[1])) return false;   // (it does not know the row length)
     // the sum must not land on the mat-mul's result, activations or weights
     return !ranges_overlap(add->data, ggml_nbytes(add), mm->data, ggml_nbytes(mm)) && !ranges_overlap(add->data, ggml_nbytes(add), x->data, ggml_nbytes(x)) &&
            !ranges_overlap(add->data, ggml_nbytes(add), w->data, ggml_nbytes(w));

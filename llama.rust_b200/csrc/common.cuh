@@ -168,7 +168,9 @@ int launch_gemm_rows_ring(int count, const int64_t *n, int64_t k, int64_t m, con
 void gemm_rows_ring_debug_wait(int spin_limit, int skip_unit);
 bool gemv_rows_add_fusable(int type, int route, int64_t n, int64_t k, int64_t m);
 // a few activation rows, fast numerics (gemm_few.cu)
+constexpr int64_t FEW_ACT_GROUPS = 1ll << 24;   // it keeps 32-bit byte offsets into the activations: fewer groups of 256 than this
 bool few_takes(int type, int route, int64_t n, int64_t k, int64_t m);
+bool few_takes_for(int type, int route, int64_t n, int64_t k, int64_t m, int sms);
 bool few_takes_experts(int type, int64_t k, int64_t act_rows, int64_t n_expert, int64_t pairs);
 int launch_gemm_few(int type, int count, const int64_t *n, int64_t k, int64_t m, const uint8_t *const *tiles, ActView acts, float *const *dst, const int64_t *lddst, cudaStream_t s);
 int launch_gemm_tcgen05(int mode, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst,
@@ -179,6 +181,7 @@ int launch_gemm_tcgen05_i8(int type, int64_t n, int64_t k, int64_t m, const uint
 // Q8_0 / Q4_0 / MXFP4 mat-muls of many rows on tcgen05 kind::f16 (gemm_b32_tcgen05.cu)
 int gemm_b32_pick_for(int type, int64_t n, int64_t m, int sms);
 bool gemm_b32_wins(int type, int64_t n, int64_t m);
+int sm_count();   // of the current device; 148 where there is none
 int launch_gemm_b32(int type, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActF16 acts, float *dst, int64_t lddst, cudaStream_t s);
 // MUL_MAT_ID, grouped by expert: column block w of the mat-mul is a work item: up to 32 (token, slot) pairs routed to one
 // expert.  *n_items items are in use (the other CTAs leave at once); work_expert[w] names the expert, col_act[32 w + c] the

@@ -448,11 +448,6 @@ template <int TYPE>
 int launch_b32_nc(int nc, const BqCall &c, int sms, cudaStream_t s) {
     return nc == 128 ? launch_b32<TYPE, 128>(c, sms, s) : launch_b32<TYPE, 64>(c, sms, s);
 }
-int sm_count() {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    return sms;
-}
 
 // ns of a wave of tiles per 32-element block, with 64 and 128 columns (4096 x 4096 on 256 rows 48 us, on 512 rows 72 us), and of the int8
 // kernel's 32 columns (4096 x 4096 on 64 rows 31 us; MXFP4 38)
@@ -463,6 +458,12 @@ int b32_columns(int64_t row_blocks, int64_t m, int sms) {
 }
 
 }  // namespace
+
+int sm_count() {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    return sms;
+}
 
 // the columns of launch_gemm_b32's tiles where it is the quicker one, else 0: the int8 kernel (gemm_tcgen05_i8.cu) has tiles of 32 columns, which
 // pays while they make few waves.  Same results.  us of a call with the int8 kernel and with this one, Q8_0: 14336 x 4096 on 512 rows

@@ -20,8 +20,9 @@
 // after warp, and with a super-block's product rounded before it meets the activation's scale, they were 6.5e-8.)
 // What was tried: 32 columns per CTA (128 registers: spills; 255: one CTA per SM; both slower than two passes of 16 columns), a warp per tile in place
 // of shared tiles (no change), 8-byte activation fragments straight from L2 (slower by a tenth at 16 columns), a CTA per tile without the
-// walk (28672 x 4096 on 16 rows 30 us, so 27), scales fetched byte by byte.  Figures against the other kernels: at few_takes below.
+// walk (28672 x 4096 on 16 rows 30 us; with it 27), scales fetched byte by byte.  Figures against the other kernels: at few_takes below.
 // Waits are bounded: one that runs out records error code 4, and the CTA ends once its own copies have landed.
+#include <algorithm>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -568,7 +569,7 @@ gemm_few_kernel(const FewArgs a) {
 // CTAs (a cluster) that share a tile's K: a pair where there are fewer tiles than about 1.4 per SM.  us, whole calls, 1 / 2 / 4 / 8 CTAs (Q4_K, 16 rows,
 // each tile a CTA of its own): 14336 x 4096 16.6 / 24.6 / 34.7 / 63.8, 4096 x 14336 21.2 / 16.8 / 19.5 / 27.0, 1024 x 4096 on 32 rows
 // 19.9 / 13.9 / 12.2 / 12.5.  More than a pair would need sums in another order: a matrix alone and one among its siblings give the same bits
-int few_splits(int64_t ctas, int nb) { return ctas < 200 && nb > 8 ? 2 : 1; }
+int few_splits(int64_t ctas, int nb, int sms) { return ctas * 20 < (int64_t)sms * 27 && nb > 8 ? 2 : 1; }
 
 template <int TYPE, int NT, bool GROUPED>
 int few_launch(FewArgs &a, int64_t column_blocks, int64_t live_blocks, int64_t act_rows, cudaStream_t s) {
@@ -584,9 +585,9 @@ int few_launch(FewArgs &a, int64_t column_blocks, int64_t live_blocks, int64_t a
         B200_CUDA(cudaFuncSetAttribute(gemm_few_kernel<TYPE, NT, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
         attr_done[dev] = true;
     }
-    B200_REQUIRE(act_rows * a.nb < (1ll << 24), "gemm few: %lld activation rows of %d super-blocks are too many", (long long)act_rows, a.nb);
+    B200_REQUIRE(act_rows * a.nb < FEW_ACT_GROUPS, "gemm few: %lld activation rows of %d super-blocks are too many", (long long)act_rows, a.nb);
     const int64_t tiles = a.tile_start[3];
-    a.splits = few_splits(tiles * live_blocks, a.nb);
+    a.splits = few_splits(tiles * live_blocks, a.nb, sms[dev]);
     static_assert(SMEM * 2 + 4096 <= 227 * 1024, "two CTAs per SM");
     const int64_t slots = 2 * (int64_t)sms[dev];
     // walks over the row tiles: as many CTAs as run at once; of experts, whose number of items the host does not know, twice that
@@ -607,19 +608,25 @@ int few_launch_nt(FewArgs &a, int64_t m, cudaStream_t s) {
 
 }  // namespace
 
-// Whether m activation rows are few.  Up to 31 always, K-quants up to 63 (48 rows of 14336 x 4096: Q4_K 38 / 66, Q6_K 48 / 67).  us of whole calls, this kernel / the others, for 8 and 16 rows: 14336 x 4096 Q4_K 13 / 25 and
-// 17 / 26, Q6_K 15 / 22 and 22 / 26, Q8_0 14 / 24 and 17 / 25, Q4_0 13 / 23 and 17 / 24, MXFP4 20 / 29 and 24 / 30; 4096 x 14336 Q8_0
-// 14 / 67 and 17 / 70; and 2 and 4 rows 13 / 36 and 13 / 71 (Q8_0), 12 / 14 and 12 / 29 (Q4_K, 14336 x 4096).
-// Above that by the measured time of each in microseconds, x = 10^6 weights, b = blocks of 16 rows: here 8 + c x b (c = 0.165, Q6_K 0.21, MXFP4 0.25:
-// instructions, 50 to 60 % of what a SM issues; the weights are unpacked again for every block);
-//   K-quants on the fast tcgen05 kernel (2048 weight rows and up): 20 + 0.45 x, Q6_K 20 + 0.82 x, while its rows fit one block of 256;
-//   K-quants of fewer weight rows, on the exact kernels: 2 a super-block of K, Q6_K 2.5 (one wave);
-//   the others on int8 tiles of 128 x 32: 5 + 1.5 a wave and super-block, MXFP4 1.9, where the f16 kernel is not the better one.
-// 4096 x 14336 on 32 rows: Q4_K 113 -> 25, Q6_K 143 -> 32, Q8_0 91 -> 24; 4096 x 4096 on 64: Q4_K 28 -> 19, Q8_0 31 -> 17; 1024 x 4096
-// Q6_K on 512: 48 -> 40.
-bool few_takes(int type, int route, int64_t n, int64_t k, int64_t m) {
-    if (numerics_mode() != 1 || m < 2 || n <= 0 || m * (k / GROUP_K) >= (1ll << 24)) return false;   // 32-bit byte offsets into the activations
-    const bool kq = type == B200_TYPE_Q4_K || type == B200_TYPE_Q6_K;
+// Whether m activation rows are few, on a GPU of sms SMs.  us, weights from HBM, the others / this kernel:
+//   * Up to 31 rows: 14336 x 4096 on 8 and 16 rows Q4_K 25 / 13 and 27 / 18, Q6_K 24 / 17 and 28 / 25, Q8_0 24 / 14 and 25 / 17, Q4_0 23 / 13 and
+//     24 / 17, MXFP4 29 / 20 and 30 / 24; 4096 x 14336 Q8_0 67 / 14 and 70 / 17, on 2 and 4 rows 36 / 13 and 71 / 13.  But not Q6_K on 9 to 31 rows of
+//     up to 16 super-blocks, which the exact kernel (gemm_mma.cu) does as quickly or quicker, n from 1000 to 32000: 6144 x 2048 on 20
+//     12.4 / 14.4, 4096 x 4096 on 12 9.9 / 10.9, 32000 x 4096 on 12 45 / 47 (14336 x 4096 on 31 43 / 39).  One rule for every n: a matrix alone and
+//     one among its siblings take the same kernel.
+//   * K-quants up to 63 rows: 14336 x 4096 on 48 Q4_K 65 / 38, Q6_K 70 / 53, 1000 x 2048 on 32 29 / 8.
+//   * Above that by estimates, in microseconds, x = 10^6 weights, b = blocks of 16 rows: here 8 + c x b (instructions, 50 to 60 % of what a SM
+//     issues: the weights are unpacked again for every block; more with less than 8 super-blocks, where warps have none), against
+//       K-quants on the fast tcgen05 kernel (2048 weight rows and up, its rows in one block of 256): by its weights or, in few tiles, by its
+//       latency a super-block, whichever says less;
+//       K-quants of fewer weight rows, on the exact kernels: a latency a super-block too (one wave);
+//       the others on int8 tiles of 128 x 32: 5 + 1.5 a wave and super-block, MXFP4 1.9, where the f16 kernel is not the better one.
+//     The estimates are a little high for this kernel and low for the others: over 1190 products (n 512 to 32000, k 1024 to 14336, 32 to 512
+//     rows, the five types) one that is taken is more than 3 % slower (6144 x 2048 Q4_K on 112 rows 23.6 / 24.5).  4096 x 14336 on 32 rows: Q4_K
+//     113 / 24, Q6_K 143 / 35, Q8_0 91 / 24; 4096 x 4096 on 64: Q4_K 28 / 19, Q8_0 31 / 17; 1024 x 4096 Q6_K on 512 55 / 43.
+bool few_takes_for(int type, int route, int64_t n, int64_t k, int64_t m, int sms) {
+    if (m < 2 || n <= 0 || m * (k / GROUP_K) >= FEW_ACT_GROUPS) return false;   // 32-bit byte offsets into the activations
+    const bool q6 = type == B200_TYPE_Q6_K, kq = type == B200_TYPE_Q4_K || q6;
     switch (type) {
         case B200_TYPE_Q4_K: break;
         case B200_TYPE_Q6_K:
@@ -634,26 +641,33 @@ bool few_takes(int type, int route, int64_t n, int64_t k, int64_t m) {
             break;
         default: return false;
     }
+    if (q6 && route == B200_ROUTE_TILED && m > 8 && m < 32 && k <= 16 * GROUP_K) return false;
+    if (m < 32 || (kq && m < GEMM_FAST_MIN_COLS)) return true;
+    if (m > (kq && n >= 2048 ? 256 : 512)) return false;
+    const double x = (double)n * (double)k * 1e-6 * 148 / sms, nb = (double)(k / GROUP_K), blocks = (double)((m + 15) / 16);   // per SM as on 148
+    if (kq) {
+        const double unpacking = (q6 ? 0.25 : 0.175) * x * blocks, here = 8.0 + unpacking + (nb < 8 ? unpacking * (8.0 / nb - 1.0) * 0.4 : 0.0);
+        if (n < 2048) return here < 7.0 + (q6 ? 2.5 : 1.8) * nb;
+        return here < std::min(20.0 + (q6 ? 0.80 : 0.40) * x, 9.0 + (q6 ? 2.4 : 1.9) * nb);
+    }
+    if (gemm_b32_pick_for(type, n, m, sms) != 0) return false;
+    const int64_t waves = (((n + 127) / 128) * ((m + 31) / 32) + sms - 1) / sms;
+    return 8.0 + (type == B200_TYPE_MXFP4 ? 0.25 : 0.182) * x * blocks < 5.0 + (type == B200_TYPE_MXFP4 ? 1.9 : 1.5) * nb * (double)waves;
+}
+// whether launch_gemv comes here: the fast numerics policy, and no switch for another kernel (B200_GEMM_FEW=0, B200_GEMM_FAST; read per call)
+bool few_takes(int type, int route, int64_t n, int64_t k, int64_t m) {
+    if (numerics_mode() != 1) return false;
     const char *e = getenv("B200_GEMM_FEW");
     if (e && e[0] == '0') return false;
-    if (m < 32 || (kq && m < GEMM_FAST_MIN_COLS)) return true;   // whatever n: a matrix alone and one among its siblings take the same kernel
-    if (m > 512 || (kq && m >= GEMM_FAST_MIN_COLS && getenv("B200_GEMM_FAST"))) return false;   // B200_GEMM_FAST asks for one of the other kernels
-    const double x = (double)n * (double)k * 1e-6, nb = (double)(k / GROUP_K), blocks = (double)((m + 15) / 16);
-    const double here = 8.0 + (type == B200_TYPE_Q6_K ? 0.21 : type == B200_TYPE_MXFP4 ? 0.25 : 0.165) * x * blocks;
-    if (kq) {
-        if (n >= 2048) return here < 20.0 + (type == B200_TYPE_Q6_K ? 0.82 : 0.45) * x;
-        return here < (type == B200_TYPE_Q6_K ? 2.5 : 2.0) * nb;
-    }
-    if (gemm_b32_wins(type, n, m)) return false;
-    const int64_t waves = (((n + 127) / 128) * ((m + 31) / 32) + 147) / 148;
-    return here < 5.0 + (type == B200_TYPE_MXFP4 ? 1.9 : 1.5) * nb * (double)waves;
+    if (m >= GEMM_FAST_MIN_COLS && (type == B200_TYPE_Q4_K || type == B200_TYPE_Q6_K) && getenv("B200_GEMM_FAST")) return false;
+    return few_takes_for(type, route, n, k, m, m < 32 ? 148 : sm_count());   // (of so few rows the number of SMs says nothing)
 }
 // MUL_MAT_ID, the pairs grouped by expert, by the pairs an expert has on average.  768 x 2048, us: Q4_K experts, whose alternative reads an expert's
 // weights once per pair: 128 experts, 512 pairs 68 -> 45, 4096 pairs 502 -> 135; 32 experts, 64 pairs 13 (20 here), 256 pairs 36 -> 23.
 // MXFP4 (Q4_0) against int8 tiles of 32 pairs: 128 experts, 128 pairs 83 -> 52 (64 -> 39), 512 pairs 121 -> 67 (92 -> 50), 1024 pairs 123 -> 80
 // (94 -> 62); 32 pairs an expert 174 -> 189 (137 -> 153)
 bool few_takes_experts(int type, int64_t k, int64_t act_rows, int64_t n_expert, int64_t pairs) {
-    if (numerics_mode() != 1 || pairs < 64 || pairs >= 0x7fffffffLL / 32 || n_expert >= (1 << 20) || act_rows * (k / GROUP_K) >= (1ll << 24)) return false;
+    if (numerics_mode() != 1 || pairs < 64 || pairs >= 0x7fffffffLL / 32 || n_expert >= (1 << 20) || act_rows * (k / GROUP_K) >= FEW_ACT_GROUPS) return false;
     const char *e = getenv("B200_GEMM_FEW");
     if (e && e[0] == '0') return false;
     const int64_t avg = pairs / (n_expert < pairs ? n_expert : pairs);

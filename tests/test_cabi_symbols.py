@@ -151,3 +151,23 @@ def test_rows_add_refuses_rows_too_long_for_the_few_rows_kernel():
             assert word in mod.lib.b200_last_error(), k
     finally:
         mod.lib.b200_set_numerics(before)
+
+
+def test_few_rows_kernel_choice():
+    """pure host arithmetic: what is measured to be quicker on the few-rows kernel, for the SMs there are; the limits of its offsets"""
+    mod = b200.load()
+    f = mod.lib.b200_few_rows_kernel_choice
+    f.argtypes = [ctypes.c_int] + [ctypes.c_int64] * 3 + [ctypes.c_int]
+    for ty in (mod.Q4_K, mod.Q6_K, mod.Q8_0, mod.Q4_0, mod.MXFP4):
+        assert f(ty, 4096, 4096, 1, 148) == 0 and f(ty, 4096, 4096, 2, 148) == 1 and f(ty, 4096, 4096, 8, 148) == 1
+        assert f(ty, 14336, 14336, 16, 148) == 1 and f(ty, 14336, 4096, 513, 148) == 0
+        assert f(ty, 8, (1 << 24) // 16 * 256, 16, 148) == 0 and f(ty, 8, (1 << 24) // 16 * 256 - 256, 16, 148) == 1
+        assert f(ty, 4096, 4096, 16, 0) == -1 and f(ty, 4096, 100, 16, 148) == -1
+    # the exact kernel's: Q6_K, 9 to 31 rows of up to 16 super-blocks (fewer rows take the row-dot route)
+    assert [f(mod.Q6_K, 6144, k, m, 148) for k, m in ((2048, 8), (2048, 9), (4096, 31), (4352, 31), (2048, 32))] == [1, 0, 0, 1, 1]
+    # the tcgen05 kernels': K-quants of short rows, batches past its block of 256 rows
+    assert [f(mod.Q6_K, 6144, 2048, m, 148) for m in (64, 80, 112)] == [1, 1, 0]
+    assert [f(mod.Q4_K, 8192, 2048, m, 148) for m in (64, 80, 112)] == [1, 1, 0]
+    assert f(mod.Q4_K, 4096, 4096, 64, 148) == 1 and f(mod.Q4_K, 4096, 14336, 64, 148) == 0 and f(mod.Q4_K, 2048, 8192, 257, 148) == 0 and f(mod.Q4_K, 1024, 8192, 257, 148) == 1
+    # int8 tiles of 128 x 32: with fewer SMs they take more waves, and this kernel more steps
+    assert f(mod.Q8_0, 4096, 4096, 64, 148) == 1 and f(mod.Q8_0, 14336, 4096, 512, 148) == 0
