@@ -21,7 +21,8 @@
 // What was tried: 32 columns per CTA (128 registers: spills; 255: one CTA per SM; both slower than two passes of 16 columns), a warp per tile in place
 // of shared tiles (no change), 8-byte activation fragments straight from L2 (slower by a tenth at 16 columns), a CTA per tile without the
 // walk (28672 x 4096 on 16 rows 30 us; with it 27), scales fetched byte by byte.  Figures against the other kernels: at few_takes below.
-// Waits are bounded: one that runs out records error code 4, and the CTA ends once its own copies have landed.
+// Waits are bounded: one that runs out records error code 4, and its CTA (and the other of a pair) stores neither that tile nor a later one of its
+// walk, and ends once its own copies have landed.
 #include <algorithm>
 #include <cstdlib>
 
@@ -53,16 +54,17 @@ struct FewArgs {
     int nb, splits, col_blocks, walkers;
     GroupMap gm;             // work_expert set: column blocks are the experts' work items
     int *err;
+    unsigned spin;           // polls of a wait
+    int skip;                // test hook: the unit that the first warp of the first CTA does not ask for, -1: none
 };
 
 __device__ __forceinline__ uint32_t few_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool few_wait(uint32_t bar, unsigned parity) {
-    for (unsigned i = 0; i < FEW_SPIN; i++) {
-        unsigned ok;
+// a warp's: the same answer for every lane
+__device__ __forceinline__ bool few_wait(uint32_t bar, unsigned parity, unsigned spin) {
+    unsigned ok = 0;
+    for (unsigned i = 0; i < spin && !ok; i++)
         asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity), "r"(1000u) : "memory");
-        if (ok) return true;
-    }
-    return false;
+    return __all_sync(0xffffffffu, ok != 0);
 }
 __device__ __forceinline__ void few_bulk(uint32_t dst, const void *src, unsigned bytes, uint32_t bar) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -390,6 +392,7 @@ gemm_few_kernel(const FewArgs a) {
     // [warp][slot][chunk]; [warp][staged activations], at a tile's end its sums [warp][column][row]; [warp] the sums of its first class, likewise
     extern __shared__ __align__(128) uint8_t few_raw[];
     __shared__ uint64_t bars[FEW_WARPS * T::SLOTS];
+    __shared__ int gave_up;   // for the other CTA of a pair
     pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = (int)(blockIdx.x % (unsigned)a.splits), idx = (int)(blockIdx.x / (unsigned)a.splits);
@@ -424,7 +427,7 @@ gemm_few_kernel(const FewArgs a) {
     const auto ask = [&](int u) {
         const int me = next_tile >= a.tile_start[2] ? 2 : next_tile >= a.tile_start[1] ? 1 : 0;
         const uint8_t *src = a.tiles[me] + expert + ((int64_t)(next_tile - a.tile_start[me]) * a.nb + group(next_group)) * T::CHUNK;
-        few_bulk(few_smem(slots + (u % T::SLOTS) * T::CHUNK), src, T::CHUNK, bar0 + 8 * (u % T::SLOTS));
+        if (u != a.skip || (blockIdx.x | warp)) few_bulk(few_smem(slots + (u % T::SLOTS) * T::CHUNK), src, T::CHUNK, bar0 + 8 * (u % T::SLOTS));
         if (++next_group == mine) {
             next_group = 0;
             next_tile += a.walkers;
@@ -491,10 +494,11 @@ gemm_few_kernel(const FewArgs a) {
         };
         for (int i = 0; i < mine && ok; i++, u++) {
             const int s = u % T::SLOTS;
-            if (!few_wait(bar0 + 8 * s, (unsigned)(u / T::SLOTS) & 1u)) {
-                // no more copies are asked for, and those on their way are waited for, with a limit again
+            if (!few_wait(bar0 + 8 * s, (unsigned)(u / T::SLOTS) & 1u, a.spin)) {
+                // No more copies are asked for, and those on their way are waited for, with a limit again.  The CTA walks on, for the barriers' sake,
+                // and stores nothing any more
                 if (lane == 0) atomicExch(a.err, FEW_ERR_WAIT);
-                for (int j = 0; j < T::SLOTS && u + j < units; j++) few_wait(bar0 + 8 * ((u + j) % T::SLOTS), (unsigned)((u + j) / T::SLOTS) & 1u);
+                for (int j = 0; j < T::SLOTS && u + j < units; j++) few_wait(bar0 + 8 * ((u + j) % T::SLOTS), (unsigned)((u + j) / T::SLOTS) & 1u, a.spin);
                 ok = false;
                 break;
             }
@@ -517,8 +521,9 @@ gemm_few_kernel(const FewArgs a) {
             __syncwarp();
             if (lane == 0 && u + T::SLOTS < units) ask(u + T::SLOTS);
         }
-        __syncthreads();   // the staged activations have been read
+        const int failed = __syncthreads_or(!ok);   // the staged activations have been read
         put(red);
+        if (tid == 0) gave_up = failed;
         __syncthreads();
         const int me = g >= a.tile_start[2] ? 2 : g >= a.tile_start[1] ? 1 : 0;
         const int64_t row0 = (int64_t)(g - a.tile_start[me]) * TILE_ROWS, n = a.n[me], lddst = a.lddst[me];
@@ -533,7 +538,7 @@ gemm_few_kernel(const FewArgs a) {
         };
         const int w0 = a.nb < 8 ? a.nb : 8, w1 = a.nb - 8 < 8 ? a.nb - 8 : 8;   // classes that there are of the first and of the second eight
         if (a.splits == 1) {
-            for (int i = tid; i < nt_live * 8 * 32; i += FEW_THREADS) {
+            for (int i = tid; !failed && i < nt_live * 8 * 32; i += FEW_THREADS) {
                 const int at = (i >> 5) * FEW_PITCH + (i & 31);
                 float v[8];
 #pragma unroll
@@ -546,7 +551,11 @@ gemm_few_kernel(const FewArgs a) {
             uint32_t p0, p1;   // the first and the second eight classes' sums
             asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p0) : "r"(few_smem(red)), "r"(0));
             asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p1) : "r"(few_smem(red)), "r"(1));
-            for (int i = tid + rank * FEW_THREADS; i < nt_live * 8 * 32; i += FEW_THREADS * 2) {
+            uint32_t other;
+            int other_failed;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(other) : "r"(few_smem(&gave_up)), "r"(rank ^ 1));
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(other_failed) : "r"(other) : "memory");
+            for (int i = tid + rank * FEW_THREADS; !(failed | other_failed) && i < nt_live * 8 * 32; i += FEW_THREADS * 2) {
                 const uint32_t at = (uint32_t)((i >> 5) * FEW_PITCH + (i & 31)) * 4;
                 float x[16];
 #pragma unroll
@@ -571,6 +580,10 @@ gemm_few_kernel(const FewArgs a) {
 // 19.9 / 13.9 / 12.2 / 12.5.  More than a pair would need sums in another order: a matrix alone and one among its siblings give the same bits
 int few_splits(int64_t ctas, int nb, int sms) { return ctas * 20 < (int64_t)sms * 27 && nb > 8 ? 2 : 1; }
 
+// test hook: while a limit is set the waits poll that often, and a.skip is the unit of the first warp that is not asked for
+unsigned g_few_spin = 0;
+int g_few_skip = -1;
+
 template <int TYPE, int NT, bool GROUPED>
 int few_launch(FewArgs &a, int64_t column_blocks, int64_t live_blocks, int64_t act_rows, cudaStream_t s) {
     using T = FewType<TYPE>;
@@ -587,6 +600,8 @@ int few_launch(FewArgs &a, int64_t column_blocks, int64_t live_blocks, int64_t a
     }
     B200_REQUIRE(act_rows * a.nb < FEW_ACT_GROUPS, "gemm few: %lld activation rows of %d super-blocks are too many", (long long)act_rows, a.nb);
     const int64_t tiles = a.tile_start[3];
+    a.spin = g_few_spin ? g_few_spin : FEW_SPIN;
+    a.skip = g_few_spin ? g_few_skip : -1;
     a.splits = few_splits(tiles * live_blocks, a.nb, sms[dev]);
     static_assert(SMEM * 2 + 4096 <= 227 * 1024, "two CTAs per SM");
     const int64_t slots = 2 * (int64_t)sms[dev];
@@ -607,6 +622,11 @@ int few_launch_nt(FewArgs &a, int64_t m, cudaStream_t s) {
 }
 
 }  // namespace
+
+void gemm_few_debug_wait(int spin_limit, int skip_unit) {
+    g_few_spin = spin_limit > 0 ? (unsigned)spin_limit : 0u;
+    g_few_skip = skip_unit;
+}
 
 // Whether m activation rows are few, on a GPU of sms SMs.  us, weights from HBM, the others / this kernel:
 //   * Up to 31 rows: 14336 x 4096 on 8 and 16 rows Q4_K 25 / 13 and 27 / 18, Q6_K 24 / 17 and 28 / 25, Q8_0 24 / 14 and 25 / 17, Q4_0 23 / 13 and

@@ -164,3 +164,54 @@ def test_few_rows_ring_mat_mul_wait_expiry():
     dev.synchronize()
     assert dev.kernel_error() == 0
     assert bits_equal(out.download(np.float32, n * m).reshape(m, n), good)
+
+
+# (rows, type, unit that is not asked for, first row and rows left unwritten); 4096 values a row are 16 groups: two of a warp's without a partner CTA, one with
+FEW = [
+    (4096, orc.Q4_K, 0, 0, 32),          # 128 row tiles by pairs of CTAs: the pair that has tile 0
+    (14336, orc.Q4_K, 1, 0, 32),         # 448 tiles, a CTA alone walks tiles 0 and 296: gives up in its first, ...
+    (14336, orc.Q8_0, 2, 296 * 32, 32),  # ... in its second
+]
+
+
+@pytest.mark.parametrize("n,ty,skip,row0,rows", FEW, ids=str)
+def test_few_rows_mat_mul_wait_expiry(n, ty, skip, row0, rows):
+    """The few-rows kernel of the fast numerics: a warp's chunk never comes, its wait runs out after 20000 polls, the kernel returns and code 4 is
+    reported.  From that tile on its CTA stores nothing (tile 296 neither where it gave up in tile 0), everything else is what an undisturbed
+    launch gives, and the next launch is undisturbed."""
+    dev = b200.load()
+    dev.set_device(0)
+    k, m = 4096, 16
+    W = synth.weights(ty, n, k, seed=91, period=512)
+    w = dev.Weight(ty, W, k)
+    dx = dev.device_array(synth.activations(m, k, seed=92))
+    out = dev.DeviceBuffer(4 * n * m)
+    dev.set_numerics(dev.FAST)
+    try:
+        dev.mul_mat_device(w, dx, m, out)
+        dev.synchronize()
+        assert dev.kernel_error() == 0
+        good = out.download(np.float32, n * m).reshape(m, n).copy()
+        dev.check(dev.lib.b200_memset(out.ptr, 0xFF, 4 * n * m, None), "memset")
+        dev.synchronize()
+        dev.lib.b200_debug_few_rows_wait(20000, skip)
+        try:
+            dev.mul_mat_device(w, dx, m, out)
+            dev.synchronize()           # returns: the wait gave up
+        finally:
+            dev.lib.b200_debug_few_rows_wait(0, -1)
+        assert dev.kernel_error() == 4
+        assert dev.kernel_error() == 0
+        got = out.download(np.uint32, n * m).reshape(m, n)
+        left = np.zeros(n, bool)
+        left[row0:row0 + rows] = True
+        if n == 14336 and row0 == 0:
+            left[296 * 32:297 * 32] = True
+        assert (got[:, left] == 0xFFFFFFFF).all(), "an unfinished tile must not be stored"
+        assert (got[:, ~left] == good.view(np.uint32)[:, ~left]).all()
+        dev.mul_mat_device(w, dx, m, out)
+        dev.synchronize()
+        assert dev.kernel_error() == 0
+        assert bits_equal(out.download(np.float32, n * m).reshape(m, n), good)
+    finally:
+        dev.set_numerics(dev.EXACT)
