@@ -115,6 +115,10 @@ void b200_debug_rows_ring_wait(int spin_limit, int skip_unit);
 /* test hook: the same for the few-rows mat-mul of the fast numerics, whose warps ask for their own weight chunks: the first warp of the launch's first
  * CTA does not ask for its chunk skip_unit.  That CTA leaves the row tile it belongs to, and those after it in its walk, unwritten; code 4. */
 void b200_debug_few_rows_wait(int spin_limit, int skip_unit);
+/* test hook: the prompt-attention kernels on tcgen05 (fast numerics; grouped attention of long BF16 prompts).  While spin_limit > 0 their waits poll at
+ * most that often, and the CTA of the last rows (of a sequence) and the first key head does not ask for the values of the mute_tile-th tile it
+ * visits (-1 = none): a wait runs out, the kernel returns with that CTA's rows unwritten and b200_kernel_error reports code 4.  spin_limit 0 disarms the hook. */
+void b200_debug_attn_wait(int spin_limit, int mute_tile);
 void b200_debug_decode_step_wait(int spin_limit, int skip_cta, int skip_barrier);
 /* Which kernel a Q4_K prompt mat-mul (8x8 gemm route, n weight rows, m >= 32 activation rows) takes on a GPU with
  * sm_count SMs: 0 = integer tcgen05 kernel, 3 / 4 = the two-pass f16-image kernels with 64 / 128 activation rows

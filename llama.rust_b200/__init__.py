@@ -81,6 +81,8 @@ def _load():
     L.b200_debug_rows_ring_wait.restype = None
     L.b200_debug_few_rows_wait.argtypes = [i32, i32]
     L.b200_debug_few_rows_wait.restype = None
+    L.b200_debug_attn_wait.argtypes = [i32, i32]
+    L.b200_debug_attn_wait.restype = None
     L.b200_debug_decode_step_launches.restype = C.c_ulonglong
     L.b200_debug_decode_step_wait.argtypes = [i32, i32, i32]
     L.b200_debug_decode_step_wait.restype = None

@@ -211,6 +211,7 @@ int b200_debug_gemm_fast_profile(unsigned long long *out, int n) { return gemm_f
 void b200_debug_gemm_fast_wait(int spin_limit, int mute_cta) { gemm_fast_debug_wait(spin_limit, mute_cta); }
 void b200_debug_rows_ring_wait(int spin_limit, int skip_unit) { gemm_rows_ring_debug_wait(spin_limit, skip_unit); }
 void b200_debug_few_rows_wait(int spin_limit, int skip_unit) { gemm_few_debug_wait(spin_limit, skip_unit); }
+void b200_debug_attn_wait(int spin_limit, int mute_tile) { attn_debug_wait(spin_limit, mute_tile); }
 int b200_debug_decode_step_times(unsigned long long *out, int n) { return decode_persistent_times(out, n); }
 void b200_debug_decode_step_wait(int spin_limit, int skip_cta, int skip_barrier) { decode_persistent_debug(spin_limit, skip_cta, skip_barrier); }
 

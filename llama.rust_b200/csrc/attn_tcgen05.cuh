@@ -22,14 +22,23 @@ __device__ __forceinline__ bool pa_try(uint64_t *bar, uint32_t parity) {
     asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(pa_smem(bar)), "r"(parity), "r"(1000u) : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool pa_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
-    for (uint32_t it = 0; it < PA_WAIT_LIMIT; it++) {
-        if (pa_try(bar, parity)) return true;
-        if ((it & 255) == 255 && *abort_flag) return false;
+// A warp's: every lane gets the same answer (what follows is done by whole warps).  False: somebody gave up, or this wait did after `limit` polls
+__device__ __forceinline__ bool pa_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
+    bool ok = pa_try(bar, parity);
+    for (uint32_t it = 1; !ok && it < limit; it++) {
+        ok = pa_try(bar, parity);
+        if (!ok && (it & 255) == 255 && *abort_flag) break;
     }
+    if (__all_sync(0xffffffffu, ok)) return true;
     *abort_flag = 1;
     return false;
 }
+// what is on its way when a CTA gives up, or ends, is waited for all the same
+__device__ __forceinline__ void pa_drain(uint64_t *bar, uint32_t parity, uint32_t limit) {
+    for (uint32_t it = 0; it < limit && !pa_try(bar, parity); it++) {}
+}
+// test hook (b200_debug_attn_wait): polls of a wait, and the visited tile whose values the CTA of the last rows and the first key head does not ask for, -1: none
+void attn_wait_hook(uint32_t *limit, int *mute);
 __device__ __forceinline__ void pa_tma(uint32_t dst, const CUtensorMap *map, int x, int head, int pos, uint64_t *bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst), "l"(map), "r"(x), "r"(head),
                  "r"(pos), "r"(pa_smem(bar))

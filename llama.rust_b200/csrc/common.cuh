@@ -435,6 +435,7 @@ int launch_grouped_decode(const GroupedArgs &a, cudaStream_t s);   // stores the
 int launch_grouped_attn(const GroupedArgs &a, cudaStream_t s);     // their cells have been stored
 bool grouped_tc_takes(const GroupedArgs &a);                       // grouped_attn_tcgen05.cu: BF16 cells
 int launch_grouped_attn_tc(const GroupedArgs &a, int *err, cudaStream_t s);
+void attn_debug_wait(int spin_limit, int mute_tile);               // flash_attn_prompt.cu: test hook of the attention kernels on tcgen05
 
 constexpr size_t HOST_RESULT_BYTES = (1 << 20) + 256;   // of a backend's page-locked block (backend.cu): what the decode driver reads results through
 // scratch owned by the library (one growing allocation per device)

@@ -23,7 +23,7 @@
 //   * A row whose output is not finite is computed again from what it sees alone (pa_row_again): the tiles' products multiply hidden cells by 0.
 //   * The positions are dealt out to the CTAs of a cluster, tile by tile, where there are too few row blocks for the GPU; the
 //     partial outputs meet in shared memory and every CTA finishes its share of the rows.
-// Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device error word.
+// Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device error word, and no row of its block is stored.
 // What bounds it (512 rows of 32 heads over 4096 positions, 8 KV heads of 128: 50 us; the mma.sync kernel in its place before took 169, 0.19 of
 // the rate the products alone would allow): a tile of 128 x 128 costs about 1850 SM clocks, 1024 of them exponentials (16 a clock) and as many
 // products, which two groups overlap only in part; and about 10 us of a launch are its beginning (q, the first tiles) and end.  On the way: one
@@ -83,6 +83,8 @@ struct PaArgs {
     int n_tok, n_head, group, splits, n_tiles, mask_wide;
     float scale_log2, q_sign;
     int *err;
+    uint32_t wait_limit;
+    int mute;   // test hook
 };
 
 template <int D, bool SPLIT>
@@ -150,7 +152,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     const int tile = rank + i * a.splits, s = i % PA_RING;
                     int c = ragged && tile == a.n_tiles - 1 ? PA_MIXED : PA_CLEAR;
                     if (a.mask) {
-                        if (!pa_wait(&sh.cfull[s], (uint32_t)(i / PA_RING) & 1u, abort_flag)) break;
+                        if (!pa_wait(&sh.cfull[s], (uint32_t)(i / PA_RING) & 1u, abort_flag, a.wait_limit)) break;
                         c = *(volatile int *)&sh.cls[s];
                         __syncwarp();
                         if (lane == 0) pa_arrive(&sh.cempty[s]);
@@ -163,7 +165,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             };
             auto tell = [&](int t) {
                 const int s = v_told % 8;
-                if (v_told >= 8 && !pa_wait(&sh.vempty[s], ((uint32_t)(v_told / 8) & 1u) ^ 1u, abort_flag)) return false;
+                if (v_told >= 8 && !pa_wait(&sh.vempty[s], ((uint32_t)(v_told / 8) & 1u) ^ 1u, abort_flag, a.wait_limit)) return false;
                 if (lane == 0) {
                     *(volatile int *)&sh.visit[s] = t;
                     pa_arrive(&sh.vfull[s]);
@@ -171,7 +173,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 v_told++;
                 return true;
             };
-            auto wait_slot = [&]() { return pa_wait(&sh.empty[seq % C::SLOTS], ((uint32_t)(seq / C::SLOTS) & 1u) ^ 1u, abort_flag); };
+            auto wait_slot = [&]() { return pa_wait(&sh.empty[seq % C::SLOTS], ((uint32_t)(seq / C::SLOTS) & 1u) ^ 1u, abort_flag, a.wait_limit); };
             auto load = [&](const CUtensorMap *map, int t, uint64_t *bar) {   // into slot `seq`, by lane 0
                 if (lane == 0) {
 #pragma unroll
@@ -179,6 +181,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 }
                 seq++;
             };
+            const int mute = (blockIdx.x | blockIdx.y) == 0 ? a.mute : -1;
             bool ok = true;
             int t[2];
             for (int g = 0; g < 2; g++) {
@@ -204,7 +207,8 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                     *(volatile int *)&sh.more[v % 8] = more;
                     pa_expect(&sh.kv[v % 8], more ? 2 * C::TILE : C::TILE);
                 }
-                load(&vmap, cur, &sh.kv[v % 8]);
+                if (v != mute) load(&vmap, cur, &sh.kv[v % 8]);
+                else seq++;
                 begun = v + 1;
                 if (more) {
                     ok = wait_slot();
@@ -215,10 +219,8 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             }
             // a CTA that gives up still waits (bounded) for the copies it has in flight
             if (*abort_flag) {
-                for (int g = 0; g < 2; g++)
-                    for (uint32_t it = 0; it < PA_WAIT_LIMIT && !pa_try(&sh.kfirst[g], 0); it++) {}
-                for (int p = begun > 8 ? begun - 8 : 0; p < begun; p++)
-                    for (uint32_t it = 0; it < PA_WAIT_LIMIT && !pa_try(&sh.kv[p % 8], (uint32_t)(p / 8) & 1u); it++) {}
+                for (int g = 0; g < 2; g++) pa_drain(&sh.kfirst[g], 0, a.wait_limit);
+                for (int p = begun > 8 ? begun - 8 : 0; p < begun; p++) pa_drain(&sh.kv[p % 8], (uint32_t)(p / 8) & 1u, a.wait_limit);
             }
         } else if (warp == 1) {
             // the whole warp waits, one elected lane issues: descriptors then stay in uniform registers
@@ -240,18 +242,18 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                 seq++;
                 scored++;
             };
-            bool ok = pa_wait(&sh.qready, 0, abort_flag);
+            bool ok = pa_wait(&sh.qready, 0, abort_flag, a.wait_limit);
             for (int g = 0; g < 2 && ok; g++) {
-                ok = pa_wait(&sh.kfirst[g], 0, abort_flag);
+                ok = pa_wait(&sh.kfirst[g], 0, abort_flag, a.wait_limit);
                 pa_fence_after();
                 if (ok && *(volatile int *)&sh.first[g]) scores(g);
             }
             for (int v = 0; v < scored && ok; v++) {
                 const int g = v & 1, j = v >> 1, s = seq % C::SLOTS;
                 // what the products read, then the weights: from there on nothing is waited for
-                ok = pa_wait(&sh.kv[v % 8], (uint32_t)(v / 8) & 1u, abort_flag);
+                ok = pa_wait(&sh.kv[v % 8], (uint32_t)(v / 8) & 1u, abort_flag, a.wait_limit);
                 const bool more = *(volatile int *)&sh.more[v % 8];
-                ok = ok && pa_wait(&sh.pready[g], (uint32_t)j & 1u, abort_flag);
+                ok = ok && pa_wait(&sh.pready[g], (uint32_t)j & 1u, abort_flag, a.wait_limit);
                 if (!ok) break;
                 pa_fence_after();
                 if (leader) {
@@ -268,7 +270,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             }
             if (leader) pa_commit(&sh.done);
             // the operands and tensor memory stay until the products are through, whatever the other roles do
-            for (uint32_t it = 0; it < PA_WAIT_LIMIT && !pa_try(&sh.done, 0); it++) {}
+            pa_drain(&sh.done, 0, a.wait_limit);
         } else if (a.mask) {
             // 16-byte pieces on their boundaries, 16 of a token's 256 bytes and a 17th where they do not begin on one.  What such a piece shares
             // with its neighbours is counted too: a tile then is at worst mixed where it could have been clear or hidden
@@ -325,7 +327,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         }
                 }
                 const bool w_any = __any_sync(0xffffffffu, any != 0), w_seen = __any_sync(0xffffffffu, seen != 0);
-                if (i >= PA_RING && !pa_wait(&sh.cempty[s], ((uint32_t)(i / PA_RING) & 1u) ^ 1u, abort_flag)) break;
+                if (i >= PA_RING && !pa_wait(&sh.cempty[s], ((uint32_t)(i / PA_RING) & 1u) ^ 1u, abort_flag, a.wait_limit)) break;
                 if (lane == 0) {
                     *(volatile int *)&sh.cls[s] = !w_seen ? PA_HIDDEN : w_any ? PA_MIXED : PA_CLEAR;
                     pa_arrive(&sh.cfull[s]);
@@ -374,7 +376,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         const unsigned char *mrow = a.mask ? a.mask + (int64_t)tok * a.mask_nb1 : nullptr;
         for (int j = 0;; j++) {
             const int v = 2 * j + g;
-            if (!pa_wait(&sh.vfull[v % 8], (uint32_t)(v / 8) & 1u, abort_flag)) break;
+            if (!pa_wait(&sh.vfull[v % 8], (uint32_t)(v / 8) & 1u, abort_flag, a.wait_limit)) break;
             const int visit = *(volatile int *)&sh.visit[v % 8];
             __syncwarp();
             if (lane == 0) pa_arrive(&sh.vempty[v % 8]);
@@ -384,7 +386,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             uint32_t s[PA_N];
             float sc = a.scale_log2;
             if (!mixed) {
-                if (!pa_wait(&sh.sfull[g], (uint32_t)j & 1u, abort_flag)) break;
+                if (!pa_wait(&sh.sfull[g], (uint32_t)j & 1u, abort_flag, a.wait_limit)) break;
                 pa_fence_after();
 #pragma unroll
                 for (int c = 0; c < PA_N; c += 32) pa_ld32(s + c, t_s + (uint32_t)c);
@@ -426,7 +428,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
                         }
                     }
                 }
-                if (!pa_wait(&sh.sfull[g], (uint32_t)j & 1u, abort_flag)) break;
+                if (!pa_wait(&sh.sfull[g], (uint32_t)j & 1u, abort_flag, a.wait_limit)) break;
                 pa_fence_after();
                 sc = 1.0f;
 #pragma unroll
@@ -503,7 +505,7 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         }
         sh.ml[g][r][0] = m;
         sh.ml[g][r][1] = l;
-        const bool finished = !*abort_flag && pa_wait(&sh.done, 0, abort_flag);
+        const bool finished = __all_sync(0xffffffffu, pa_wait(&sh.done, 0, abort_flag, a.wait_limit) && !*abort_flag);
         pa_fence_after();
         asm volatile("bar.sync 1, 256;" ::: "memory");
         const float ma = sh.ml[0][r][0], mb = sh.ml[1][r][0], mm = fmaxf(ma, mb);
@@ -538,7 +540,11 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
     __syncthreads();
     pa_fence_after();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
-    if (tid == 0 && *abort_flag) atomicExch(a.err, PA_ERR_WAIT);
+    if (*abort_flag) {   // no row of this block is stored, by whichever CTA of the cluster: a maximum of NaN, which no row has otherwise, says so
+        if (tid == 0) atomicExch(a.err, PA_ERR_WAIT);
+        if (tid < PA_M) sh.ml[0][tid][0] = NAN;
+        __syncthreads();
+    }
     if (a.splits > 1) pa_cluster_sync();
     {
         // this CTA's share of the rows: a warp per row, the CTAs' partial outputs under their common maximum
@@ -550,11 +556,14 @@ fa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
             if (row >= a.rows) break;
             float2 st[PA_MAX_SPLITS];
             float top = -INFINITY;
+            bool whole = true;
 #pragma unroll
             for (int p = 0; p < PA_MAX_SPLITS; p++) {
                 st[p] = p < a.splits ? pa_ld_peer2(pa_mapa(ml + (uint32_t)r * 8, (uint32_t)p)) : make_float2(-INFINITY, 0.0f);
                 top = fmaxf(top, st[p].x);
+                whole = whole && st[p].x == st[p].x;
             }
+            if (!whole) continue;
             float sum = 0.0f, acc[D / 32];
 #pragma unroll
             for (int e = 0; e < D / 32; e++) acc[e] = 0.0f;
@@ -669,7 +678,19 @@ int launch(const CUtensorMap &km, const CUtensorMap &vm, PaArgs &p, int64_t bloc
     return launch_pdl_cluster(fa_prompt_kernel<D, SPLIT>, grid, dim3(PA_THREADS), (unsigned)p.splits, PaCfg<D>::SMEM, s, km, vm, p);
 }
 
+uint32_t g_attn_wait_limit = 0;
+int g_attn_mute = -1;
+
 }  // namespace
+
+void attn_debug_wait(int spin_limit, int mute_tile) {
+    g_attn_wait_limit = spin_limit > 0 ? (uint32_t)spin_limit : 0u;
+    g_attn_mute = mute_tile;
+}
+void attn_wait_hook(uint32_t *limit, int *mute) {
+    *limit = g_attn_wait_limit ? g_attn_wait_limit : PA_WAIT_LIMIT;
+    *mute = g_attn_wait_limit ? g_attn_mute : -1;
+}
 
 // true: the fast prompt kernel took the call (*rc is its status); false: not a shape it handles.  Which of 2 to 63 rows come here: flash_attn.cu
 bool flash_attn_fast_prompt(const b200_flash_attn_args *a, cudaStream_t s, int *rc) {
@@ -705,6 +726,7 @@ bool flash_attn_fast_prompt(const b200_flash_attn_args *a, cudaStream_t s, int *
     p.k_nb2 = a->k_nb2;
     p.v_nb1 = a->v_nb1;
     p.v_nb2 = a->v_nb2;
+    attn_wait_hook(&p.wait_limit, &p.mute);
     p.dst = a->dst;
     p.n_kv = a->n_kv;
     p.rows = rows;

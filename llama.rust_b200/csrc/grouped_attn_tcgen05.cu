@@ -12,7 +12,7 @@
 //   * a row whose output is not finite is computed again from the entries it sees alone (pa_row_again): the products multiply hidden ones by 0;
 //   * what a row sees is arithmetic: only tiles at an edge of it compare entries, with three thresholds of the row's.
 // What it takes, beside the other kernel: at grouped_tc_takes.
-// Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device error word.
+// Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device error word, and no row of its block is stored.
 #include "attn_tcgen05.cuh"
 #include "attn_tile.cuh"
 #include "dense.cuh"
@@ -48,7 +48,7 @@ struct GaEntries {
 
 template <typename Y, int D>
 __global__ void __launch_bounds__(GA_THREADS, 1)
-grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_constant__ CUtensorMap runs, const GroupedArgs a, int group, bool vec_q, int *err) {
+grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_constant__ CUtensorMap runs, const GroupedArgs a, int group, bool vec_q, int *err, uint32_t wait_limit, int mute) {
     using C = GaCfg<D>;
     extern __shared__ uint8_t ga_raw[];
     __shared__ GaShared sh;
@@ -106,7 +106,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
             int seq = 0;
             const uint64_t q_desc = pa_desc(q_s, 16), k_desc = pa_desc(kv_s, 16), v_desc = pa_desc(kv_s, GA_N * 128);
             auto wait_slot = [&](int q) {
-                const bool ok = pa_wait(&sh.full[q % C::SLOTS], (uint32_t)(q / C::SLOTS) & 1u, abort_flag);
+                const bool ok = pa_wait(&sh.full[q % C::SLOTS], (uint32_t)(q / C::SLOTS) & 1u, abort_flag, wait_limit);
                 pa_fence_after();
                 return ok;
             };
@@ -124,7 +124,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
                 }
                 seq++;
             };
-            bool ok = pa_wait(&sh.qready, 0, abort_flag);
+            bool ok = pa_wait(&sh.qready, 0, abort_flag, wait_limit);
             for (int g = 0; g < 2 && ok && g < tiles; g++) {
                 ok = wait_slot(seq);
                 if (ok) scores(g);
@@ -132,7 +132,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
             for (int v = 0; v < tiles && ok; v++) {
                 const int g = v & 1, j = v >> 1, s = seq % C::SLOTS;
                 const bool more = v + 2 < tiles;
-                ok = wait_slot(seq) && (!more || wait_slot(seq + 1)) && pa_wait(&sh.pready[g], (uint32_t)j & 1u, abort_flag);
+                ok = wait_slot(seq) && (!more || wait_slot(seq + 1)) && pa_wait(&sh.pready[g], (uint32_t)j & 1u, abort_flag, wait_limit);
                 if (!ok) break;
                 pa_fence_after();
                 if (leader) {
@@ -149,7 +149,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
             }
             if (leader) pa_commit(&sh.done);
             // the operands and tensor memory stay until the products are through, whatever the other roles do
-            for (uint32_t it = 0; it < PA_WAIT_LIMIT && !pa_try(&sh.done, 0); it++) {}
+            pa_drain(&sh.done, 0, wait_limit);
         } else if (warp == 0) {
             // keys of tile 0, keys of tile 1, then values of tile v and keys of tile v + 2, the order in which the products read them.  A lane brings four
             // entries' rows, whose cells it has looked up: a row that the lists do not have reads as zeros (and is reported)
@@ -177,14 +177,15 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
                 r.run = (__ballot_sync(0xffffffffu, mine) >> (lane & ~7) & 0xffu) == 0xffu;
                 return r;
             };
-            const auto load = [&](const Rows &rows, int from) {
+            const auto load = [&](const Rows &rows, int from, bool muted = false) {
                 const int s = seq % C::SLOTS;
-                if (!pa_wait(&sh.empty[s], ((uint32_t)(seq / C::SLOTS) & 1u) ^ 1u, abort_flag)) return false;
+                if (!pa_wait(&sh.empty[s], ((uint32_t)(seq / C::SLOTS) & 1u) ^ 1u, abort_flag, wait_limit)) return false;
                 if (lane == 0) pa_expect(&sh.full[s], C::TILE);
                 __syncwarp();
                 const uint32_t dst = kv_s + (uint32_t)(s * C::TILE + lane * 512), bar = pa_smem(&sh.full[s]);
 #pragma unroll
                 for (int c = 0; c < C::CHUNKS; c++) {
+                    if (muted) continue;
                     if (!rows.run)
                         asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst + c * (GA_N * 128)),
                                      "l"(&cells), "r"(from + 64 * c), "r"(rows.c[0]), "r"(rows.c[1]), "r"(rows.c[2]), "r"(rows.c[3]), "r"(bar)
@@ -199,17 +200,16 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
             };
             const int keys = hk * (a.dim + a.vdim), values = keys + a.dim;
             Rows r0s = find(0), r1s = find(1);
-            bool ok = load(r0s, keys) && (tiles < 2 || load(r1s, keys));
+            bool ok = tiles < 1 || (load(r0s, keys) && (tiles < 2 || load(r1s, keys)));
             for (int v = 0; v < tiles && ok; v++) {
                 const Rows next = find(v + 2);   // on their way while a slot is waited for
-                ok = load(r0s, values) && (v + 2 >= tiles || load(next, keys));
+                ok = load(r0s, values, v == mute && hk == 0 && r0 + tokens == sg[SEG_ROWS]) && (v + 2 >= tiles || load(next, keys));
                 r0s = r1s;
                 r1s = next;
             }
             // a CTA that gives up still waits (bounded) for the copies it has in flight
             if (*abort_flag)
-                for (int q = seq < C::SLOTS ? 0 : seq - C::SLOTS; q < seq; q++)
-                    for (uint32_t it = 0; it < PA_WAIT_LIMIT && !pa_try(&sh.full[q % C::SLOTS], (uint32_t)(q / C::SLOTS) & 1u); it++) {}
+                for (int q = seq < C::SLOTS ? 0 : seq - C::SLOTS; q < seq; q++) pa_drain(&sh.full[q % C::SLOTS], (uint32_t)(q / C::SLOTS) & 1u, wait_limit);
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");
@@ -277,7 +277,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
         float m = -INFINITY, l = 0.0f;
         for (int j = 0; 2 * j + g < tiles; j++) {
             const int k0 = (2 * j + g) * GA_N;
-            if (!pa_wait(&sh.sfull[g], (uint32_t)j & 1u, abort_flag)) break;
+            if (!pa_wait(&sh.sfull[g], (uint32_t)j & 1u, abort_flag, wait_limit)) break;
             pa_fence_after();
             uint32_t s[GA_N];
 #pragma unroll
@@ -345,7 +345,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
         }
         sh.ml[g][r][0] = m;
         sh.ml[g][r][1] = l;
-        const bool finished = !*abort_flag && pa_wait(&sh.done, 0, abort_flag);
+        const bool finished = __all_sync(0xffffffffu, pa_wait(&sh.done, 0, abort_flag, wait_limit) && !*abort_flag);
         pa_fence_after();
         asm volatile("bar.sync 1, 256;" ::: "memory");
         const float ma = sh.ml[0][r][0], mb = sh.ml[1][r][0], mm = fmaxf(ma, mb);
@@ -452,8 +452,11 @@ int launch(const GroupedArgs &a, int *err, cudaStream_t s) {
     if (rc != B200_STATUS_SUCCESS) return rc;
     rc = rows_map(&cells, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.cache, a.ldc, a.n_cells, a.ldc, 1);   // one row high: rows are gathered
     if (rc != B200_STATUS_SUCCESS) return rc;
+    uint32_t wait_limit;
+    int mute;
+    attn_wait_hook(&wait_limit, &mute);
     return launch_pdl(grouped_attn_tc_kernel<Y, D>, dim3((unsigned)((a.n + per - 1) / per + a.n_seg), (unsigned)a.kv_heads), dim3(GA_THREADS), GaCfg<D>::SMEM, s, cells, runs, a, group, vec_q,
-                      err);
+                      err, wait_limit, mute);
 }
 
 }  // namespace

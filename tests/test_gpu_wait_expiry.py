@@ -215,3 +215,70 @@ def test_few_rows_mat_mul_wait_expiry(n, ty, skip, row0, rows):
         assert bits_equal(out.download(np.float32, n * m).reshape(m, n), good)
     finally:
         dev.set_numerics(dev.EXACT)
+
+
+@pytest.mark.parametrize("T,H,Hkv,D,n_kv", [(64, 8, 2, 128, 2048), (512, 32, 8, 128, 512), (32, 16, 4, 128, 1024), (200, 8, 8, 64, 3000)], ids=str)
+def test_prompt_attention_wait_expiry(T, H, Hkv, D, n_kv):
+    """The values of a tile never come: the first CTA (alone or one of a cluster) gives up after 20000 polls, code 4 is reported, the rows of its block are
+    left unwritten, by the other CTAs of the cluster too; every other row is what an undisturbed launch gives, and so is the next launch."""
+    import ctypes as C
+
+    from test_gpu_flash_attn import synth_case
+    dev = b200.load()
+    dev.set_device(0)
+    q, k, v, mask = synth_case(H, Hkv, D, T, n_kv, seed=T + n_kv)
+    dq, dk, dv, dm = (dev.device_array(np.ascontiguousarray(x)) for x in (np.transpose(q, (1, 0, 2)), k, v, mask))
+    dst = dev.DeviceBuffer(4 * T * H * D)
+    a = dev.FlashAttnArgs()
+    a.dk, a.dv, a.n_tok, a.n_head, a.n_head_kv, a.n_kv = D, D, T, H, Hkv, n_kv
+    a.q, a.q_nb1, a.q_nb2 = dq.ptr, H * D * 4, D * 4
+    a.k, a.k_nb1, a.k_nb2 = dk.ptr, D * 2, n_kv * D * 2
+    a.v, a.v_nb1, a.v_nb2 = dv.ptr, D * 2, n_kv * D * 2
+    a.mask, a.mask_nb1 = dm.ptr, n_kv * 2
+    a.scale, a.dst, a.mode = D ** -0.5, dst.ptr, 1
+
+    def run():
+        dev.check(dev.lib.b200_memset(dst.ptr, 0xFF, 4 * T * H * D, None), "memset")
+        dev.check(dev.lib.b200_flash_attn_ext(C.byref(a), None), "flash_attn_ext")
+        dev.synchronize()
+        return dst.download(np.uint32, T * H * D).reshape(T, H, D)
+
+    good = run()
+    assert dev.kernel_error() == 0
+    dev.lib.b200_debug_attn_wait(20000, 0)
+    try:
+        got = run()           # returns: the wait gave up
+    finally:
+        dev.lib.b200_debug_attn_wait(0, -1)
+    assert dev.kernel_error() == 4
+    assert dev.kernel_error() == 0
+    group = H // Hkv
+    left = np.zeros((T, H), bool)   # the last block of 128 (token, head) rows of the first key head: launched first
+    rows = np.arange((T * group - 1) // 128 * 128, T * group)
+    left[rows // group, rows % group] = True
+    assert (got[left] == 0xFFFFFFFF).all(), "rows of a block that gave up must not be stored"
+    assert (got[~left] == good[~left]).all()
+    assert (run() == good).all() and dev.kernel_error() == 0
+
+
+def test_grouped_prompt_attention_wait_expiry():
+    """the same in the grouped attention of a long BF16 prompt: the step reports code 4, and a step of another context (captured launches keep the limit
+    that they were made with) is undisturbed"""
+    import importlib
+
+    import lenolix_models as M
+    from decoder_checks import feed, model
+    dev = b200.load()
+    dev.set_device(0)
+    ll = importlib.import_module("llama_rust_b200.llama")
+    cfg = M.config([M.layer(heads=8, kv_heads=2, dim=128, vdim=128, window=130, keep=9, rot=64)], width=64)
+    w, toks = M.weights(cfg, 7), M.tokens(cfg, 300, 8)
+    good = feed(model(ll, cfg, w, "bfloat16", n_ctx=1024), toks, 300)
+    dev.lib.b200_debug_attn_wait(20000, 0)
+    try:
+        with pytest.raises(dev.B200Error, match="error code 4"):
+            feed(model(ll, cfg, w, "bfloat16", n_ctx=1024), toks, 300)
+    finally:
+        dev.lib.b200_debug_attn_wait(0, -1)
+    assert dev.kernel_error() == 0
+    assert bits_equal(feed(model(ll, cfg, w, "bfloat16", n_ctx=1024), toks, 300), good)
