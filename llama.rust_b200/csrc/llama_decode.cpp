@@ -612,9 +612,11 @@ int b200_llama_decode_seqs(b200_llama *c, const int32_t *tokens, const int32_t *
     }
     if (argmax) c->backend->iface.get_tensor_async(c->backend, g->argmax, argmax, 0, (size_t)n_out * 4);
     c->backend->iface.synchronize(c->backend);
-    if (!back || code) {   // reading the word this way also clears it
+    if (!back || code) {   // reading the word this way also clears it; another context may have done so by now, but the code is this step's too
+        const int seen = code;
         rc = b200_kernel_error(&code);
         if (rc != B200_STATUS_SUCCESS) return rc;
+        if (code == 0) code = seen;
     }
     B200_REQUIRE(code == 0, "llama_decode: a kernel reported error code %d", code);
     return B200_STATUS_SUCCESS;
