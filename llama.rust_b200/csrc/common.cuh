@@ -172,7 +172,7 @@ constexpr int64_t FEW_ACT_GROUPS = 1ll << 24;   // it keeps 32-bit byte offsets 
 bool few_takes(int type, int route, int64_t n, int64_t k, int64_t m);
 bool few_takes_for(int type, int route, int64_t n, int64_t k, int64_t m, int sms);
 void gemm_few_debug_wait(int spin_limit, int skip_unit);   // test hook
-bool few_takes_experts(int type, int64_t k, int64_t act_rows, int64_t n_expert, int64_t pairs);
+bool few_takes_experts(int type, int64_t n, int64_t k, int64_t act_rows, int64_t n_expert, int64_t pairs);
 int launch_gemm_few(int type, int count, const int64_t *n, int64_t k, int64_t m, const uint8_t *const *tiles, ActView acts, float *const *dst, const int64_t *lddst, cudaStream_t s);
 int launch_gemm_tcgen05(int mode, int64_t n, int64_t k, int64_t m, const uint8_t *tiles, ActView acts, float *dst, int64_t lddst,
                         cudaStream_t s);

@@ -682,16 +682,25 @@ bool few_takes(int type, int route, int64_t n, int64_t k, int64_t m) {
     if (m >= GEMM_FAST_MIN_COLS && (type == B200_TYPE_Q4_K || type == B200_TYPE_Q6_K) && getenv("B200_GEMM_FAST")) return false;
     return few_takes_for(type, route, n, k, m, m < 32 ? 148 : sm_count());   // (of so few rows the number of SMs says nothing)
 }
-// MUL_MAT_ID, the pairs grouped by expert, by the pairs an expert has on average.  768 x 2048, us: Q4_K experts, whose alternative reads an expert's
-// weights once per pair: 128 experts, 512 pairs 68 -> 45, 4096 pairs 502 -> 135; 32 experts, 64 pairs 13 (20 here), 256 pairs 36 -> 23.
-// MXFP4 (Q4_0) against int8 tiles of 32 pairs: 128 experts, 128 pairs 83 -> 52 (64 -> 39), 512 pairs 121 -> 67 (92 -> 50), 1024 pairs 123 -> 80
-// (94 -> 62); 32 pairs an expert 174 -> 189 (137 -> 153)
-bool few_takes_experts(int type, int64_t k, int64_t act_rows, int64_t n_expert, int64_t pairs) {
+// MUL_MAT_ID, the pairs grouped by expert, by the pairs an expert has on average; us, the others / this kernel, even routing.
+//   * Q6_K, Q8_0: the alternative reads an expert's weights once per pair.  From 4 pairs an expert on; 128 experts of 768 x 2048, 512 pairs 0.35 and
+//     0.26 of its time.
+//   * Q4_K: the same, but its per-pair kernel is quicker on rows of few super-blocks, of which most of this one's warps have none: 128 experts of
+//     768 x 2048 on 512 pairs 68 / 45, 4096 pairs 502 / 135; 60 of 512 x 1024 on 256 pairs (4 each) 15 / 20, on 512 (8) 0.92; 256 x 512 2.1
+//     times as long with 4 each, 1.5 with 8.
+//   * MXFP4 and Q4_0 against int8 tiles of 128 rows x 32 pairs, up to 16 pairs an expert: 768 x 2048, 128 experts, 128 pairs 83 / 52 (64 / 39), 512 pairs
+//     121 / 67 (92 / 50), 2048 pairs 0.91; 32 pairs an expert 174 / 189 (137 / 153).  Not rows of less than four super-blocks (256 x 512 1.1 to 1.5
+//     times as long), with four to seven of them up to 4 pairs an expert only (512 x 1024, 60 experts of 8.5 pairs 1.0 to 1.08), and as few where
+//     the int8 tiles are one wave (8 experts of 2048 x 2048, 128 pairs 1.17).  Routing as uneven as 1 / rank gains as much; where 8 of 128 experts have all
+//     the pairs this kernel is up to a third slower, which the host cannot know.
+bool few_takes_experts(int type, int64_t n, int64_t k, int64_t act_rows, int64_t n_expert, int64_t pairs) {
     if (numerics_mode() != 1 || pairs < 64 || pairs >= 0x7fffffffLL / 32 || n_expert >= (1 << 20) || act_rows * (k / GROUP_K) >= FEW_ACT_GROUPS) return false;
     const char *e = getenv("B200_GEMM_FEW");
     if (e && e[0] == '0') return false;
-    const int64_t avg = pairs / (n_expert < pairs ? n_expert : pairs);
-    return type == B200_TYPE_MXFP4 || type == B200_TYPE_Q4_0 ? avg <= 16 : avg >= 4;
+    const int64_t experts = n_expert < pairs ? n_expert : pairs, avg = pairs / experts, nb = k / GROUP_K;
+    if (type == B200_TYPE_MXFP4 || type == B200_TYPE_Q4_0) return nb >= 4 && avg <= (nb < 8 || (n + 127) / 128 * experts <= sm_count() ? 4 : 16);
+    if (type == B200_TYPE_Q4_K) return nb >= 4 && avg >= 4 && avg * nb >= 32;
+    return avg >= 4;
 }
 
 // count matrices of one type and row length against the same m activation rows

@@ -536,7 +536,7 @@ size_t mmid_grouped_scratch_bytes(int64_t n_expert, int64_t n_pairs) {
 }
 int launch_mul_mat_id_grouped(int type, int64_t n, int64_t k, int64_t n_expert, int64_t ne11, int64_t n_tok, int64_t n_ids, const uint8_t *tiles,
                               ActView acts, const int32_t *ids, float *dst, void *lists, cudaStream_t s) {
-    const bool few = few_takes_experts(type, k, ne11 * n_tok, n_expert, n_tok * n_ids);
+    const bool few = few_takes_experts(type, n, k, ne11 * n_tok, n_expert, n_tok * n_ids);
     B200_REQUIRE(few || type == B200_TYPE_MXFP4 || type == B200_TYPE_Q4_0, "mul_mat_id grouped: type %d is not a 32-element-block type on the 8x8 route", type);
     const int64_t n_pairs = n_tok * n_ids;
     B200_REQUIRE(n_pairs < 0x7fffffffLL / TI_COLS && n_expert < (1 << 20), "mul_mat_id grouped: too many pairs or experts");

@@ -1047,7 +1047,7 @@ int launch_mul_mat_id(int type, int64_t n, int64_t k, int64_t n_expert, int64_t 
     const bool repack = n % 8 == 0;
     // enough pairs to fill tensor-core tiles: grouped by expert, every expert's weights read once (same per-block chain,
     // same bits as the per-pair kernels below)
-    if (((type != B200_TYPE_MXFP4 && type != B200_TYPE_Q4_0) || repack) && few_takes_experts(type, k, ne11 * n_tok, n_expert, pairs) && mmid_grouped_enabled())
+    if (((type != B200_TYPE_MXFP4 && type != B200_TYPE_Q4_0) || repack) && few_takes_experts(type, n, k, ne11 * n_tok, n_expert, pairs) && mmid_grouped_enabled())
         return launch_mul_mat_id_grouped(type, n, k, n_expert, ne11, n_tok, n_ids, tiles, acts, ids, dst, counts, s);
     if ((type == B200_TYPE_MXFP4 || type == B200_TYPE_Q4_0) && repack && pairs >= 64 && mmid_grouped_enabled() && gemm_tcgen05_enabled())
         return launch_mul_mat_id_grouped(type, n, k, n_expert, ne11, n_tok, n_ids, tiles, acts, ids, dst, counts, s);

@@ -103,11 +103,11 @@ def test_siblings_and_the_fused_add(dev, fast, ty):
 
 
 @pytest.mark.parametrize("ty", TYPES, ids=lambda t: orc.TYPE_NAMES[t])
-@pytest.mark.parametrize("experts,top,tokens,ne11", [(40, 2, 40, 1), (5, 3, 30, 3), (4, 4, 100, 1)], ids=str)
-def test_experts(dev, fast, ty, experts, top, tokens, ne11):
-    """blocks of 8 and 16 pairs, experts without any, items that are not full; ids out of range are skipped"""
-    n, k = 72, 768
-    W = synth.weights(ty, experts * n, k, seed=71).reshape(experts, n, -1)
+@pytest.mark.parametrize("experts,top,tokens,ne11,n,k", [(40, 2, 40, 1, 72, 2048), (5, 3, 30, 3, 72, 2304), (4, 4, 100, 1, 72, 1024), (60, 8, 60, 1, 400, 2048), (20, 2, 40, 1, 72, 1024)], ids=str)
+def test_experts(dev, fast, ty, experts, top, tokens, ne11, n, k):
+    """blocks of 8 and 16 pairs, experts without any, items that are not full; ids out of range are skipped.  (Which type takes the kernel where: MXFP4 and
+    Q4_0 the first and the last two, the K-quants and Q8_0 the second and third, and the fourth.)"""
+    W = synth.weights(ty, experts * n, k, seed=71, period=72 * 7 + 1).reshape(experts, n, -1)
     B = synth.activations(tokens * ne11, k, seed=72).reshape(tokens, ne11, k)
     ids = top_k_ids(tokens, experts, top, seed=73)
     if experts == 40:
