@@ -1,6 +1,6 @@
 // Grouped-query attention of a prompt's rows over BF16 cells on the tcgen05 tensor cores: the function of grouped_attn_mma_kernel
-// (grouped_attn.cu: window, kept first positions, sinks, rotated queries, entries that lead to cells), head sizes up to 128, for key heads that a
-// power of two of query heads shares.
+// (grouped_attn.cu: window, kept first positions, sinks, rotated queries, entries that lead to cells), for keys and values of 64 or 128 channels (D) and
+// key heads that a power of two of query heads shares.
 //
 // The frame is fa_prompt_kernel's (flash_attn_prompt.cu): 128 rows of one key head, a row being (token, query head), two groups of four softmax
 // warps that take turns at tiles of 128 entries, scores, weights and unnormalised outputs in tensor memory, a rescaling of the output only
@@ -198,7 +198,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
                 seq++;
                 return true;
             };
-            const int keys = hk * (a.dim + a.vdim), values = keys + a.dim;
+            const int keys = hk * 2 * D, values = keys + D;
             Rows r0s = find(0), r1s = find(1);
             bool ok = tiles < 1 || (load(r0s, keys) && (tiles < 2 || load(r1s, keys)));
             for (int v = 0; v < tiles && ok; v++) {
@@ -227,23 +227,23 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
 #pragma unroll
                 for (int u = 0; u < 8; u++) {
                     const int x = (warp - 8) * 16 + h + u, tok = min(x / group, tokens - 1);
-                    const float *q = a.proj + (row0 + tok) * a.ldp + (int64_t)(hk * group + x % group) * a.dim;
+                    const float *q = a.proj + (row0 + tok) * a.ldp + (int64_t)(hk * group + x % group) * D;
                     const float *rope = a.rope + (int64_t)(pos0 + tok) * a.rot_dims;
 #pragma unroll
                     for (int c = 0; c < C::CHUNKS; c++) {
                         const int j = 64 * c + 2 * lane, i = j < half ? j : j - half;
-                        const bool in = j < a.dim, rot = j < a.rot_dims;
-                        const int at = in ? j : 0, other = rot ? (j < half ? j + half : j - half) : at;
+                        const bool rot = j < a.rot_dims;
+                        const int other = rot ? (j < half ? j + half : j - half) : j;
                         w[u][c] = make_float4(1.0f, 0.0f, 1.0f, 0.0f);
                         if (vec_q) {
-                            f[u][c] = *(const float2 *)(q + at);
+                            f[u][c] = *(const float2 *)(q + j);
                             y[u][c] = *(const float2 *)(q + other);
                             if (a.rot_dims > 0) w[u][c] = *(const float4 *)(rope + (rot ? 2 * i : 0));
                         } else {   // of pairs that straddle an edge each channel on its own
                             float v[2];
                             for (int k = 0; k < 2; k++) {
                                 const int d = j + k, n = d < half ? d : d - half;
-                                v[k] = d >= a.dim ? 0.0f : q[d];
+                                v[k] = q[d];
                                 if (d < a.rot_dims) v[k] = d < half ? fmaf(v[k], rope[2 * n], -(q[d + half] * rope[2 * n + 1])) : fmaf(v[k], rope[2 * n], q[d - half] * rope[2 * n + 1]);
                             }
                             f[u][c] = make_float2(v[0], v[1]);
@@ -261,7 +261,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
                             const float s1 = j < half ? -1.0f : 1.0f;
                             v = make_float2(fmaf(v.x, w[u][c].x, s1 * (y[u][c].x * w[u][c].y)), fmaf(v.y, w[u][c].z, s1 * (y[u][c].y * w[u][c].w)));
                         }
-                        if (x / group >= tokens || j >= a.dim) v = make_float2(0.0f, 0.0f);
+                        if (x / group >= tokens) v = make_float2(0.0f, 0.0f);
                         *(uint32_t *)(q_g + c * (GA_M * 128) + (x >> 3) * 1024 + (x & 7) * 128 + ((((lane >> 2) ^ (x & 7)) << 4) | (lane & 3) * 4)) = bf16_pack(v.x, v.y);
                     }
                 }
@@ -395,15 +395,15 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
         const float m = sh.ml[0][x][0], lt = sh.ml[0][x][1];
         const float mf = fmaxf(m, sinks[i]), w = pa_ex2(m - mf), f = w / (lt * w + pa_ex2(sinks[i] - mf));
         const float *part = (const float *)(q_g + GA_M * D * 2) + (size_t)x * C::PITCH;
-        Y *y = (Y *)a.y + (row0 + tok) * a.ldy + (int64_t)head * a.vdim;
+        Y *y = (Y *)a.y + (row0 + tok) * a.ldy + (int64_t)head * D;
         bool fine = pa_finite(lt);
 #pragma unroll
         for (int c = 0; c < C::CHUNKS; c++) {
             const int j = 64 * c + 2 * lane;
             const float2 v = *(const float2 *)(part + j);
             fine = fine && pa_finite(v.x) && pa_finite(v.y);
-            if (j < a.vdim) y[j] = from_f32<Y>(v.x * f);
-            if (j + 1 < a.vdim) y[j + 1] = from_f32<Y>(v.y * f);
+            y[j] = from_f32<Y>(v.x * f);
+            y[j + 1] = from_f32<Y>(v.y * f);
         }
         if (!__all_sync(0xffffffffu, fine)) again |= 1u << i;
     }
@@ -411,7 +411,7 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
     for (; again; again &= again - 1) {
         const int x = warp + 16 * (__ffs(again) - 1), tok = x / group, head = hk * group + x - tok * group, p = pos0 + tok;
         const int h0 = min(en.kept - 1, p), l1 = max(en.kept, p - window - en.lo + en.kept + 1), h1 = min(en.total - 1, p - en.lo + en.kept);
-        const __nv_bfloat16 *const cache = (const __nv_bfloat16 *)a.cache + (int64_t)hk * (a.dim + a.vdim);
+        const __nv_bfloat16 *const cache = (const __nv_bfloat16 *)a.cache + (int64_t)hk * 2 * D;
         const int kept = sg[SEG_KEPT], key0 = sg[SEG_KEY0];
         const int64_t tab0 = sg[SEG_TAB0];
         float acc[D / 32], m, lt;
@@ -421,12 +421,12 @@ grouped_attn_tc_kernel(const __grid_constant__ CUtensorMap cells, const __grid_c
             const int64_t at = tab0 + (at_pos < kept ? at_pos : kept + at_pos - key0);
             if ((at_pos >= kept && at_pos < key0) || at < 0 || at >= a.n_tab || a.tab[at] < 0 || a.tab[at] >= a.n_cells) return false;   // reported above
             *key = (const uint8_t *)(cache + (int64_t)a.tab[at] * a.ldc);
-            *value = *key + 2 * a.dim;
+            *value = *key + 2 * D;
             return true;
         }, acc, &m, &lt);
         const float sink = a.sink ? a.sink[head] * 1.4426950408889634f : -INFINITY;
         const float mf = fmaxf(m, sink), w = pa_ex2(m - mf), f = w / (lt * w + pa_ex2(sink - mf));
-        Y *y = (Y *)a.y + (row0 + tok) * a.ldy + (int64_t)head * a.vdim;
+        Y *y = (Y *)a.y + (row0 + tok) * a.ldy + (int64_t)head * D;
 #pragma unroll
         for (int c = 0; c < C::CHUNKS; c++) {
             y[64 * c + 2 * lane] = from_f32<Y>(acc[2 * c] * f);
@@ -446,7 +446,7 @@ int launch(const GroupedArgs &a, int *err, cudaStream_t s) {
         attr_done[dev] = true;
     }
     const int group = a.heads / a.kv_heads, per = GA_M / group;
-    const bool vec_q = a.dim % 2 == 0 && a.ldp % 2 == 0 && a.rot_dims % 4 == 0 && (((uintptr_t)a.proj | (uintptr_t)a.rope) & 15) == 0;
+    const bool vec_q = a.ldp % 2 == 0 && a.rot_dims % 4 == 0 && (((uintptr_t)a.proj | (uintptr_t)a.rope) & 15) == 0;
     CUtensorMap cells, runs;
     int rc = rows_map(&runs, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.cache, a.ldc, a.n_cells, a.ldc, 32);
     if (rc != B200_STATUS_SUCCESS) return rc;
