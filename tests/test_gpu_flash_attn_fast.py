@@ -55,7 +55,7 @@ def run_fast(dev, q, k, v, mask, scale, **kw):
 
 
 def test_fast_policy_takes_rows_below_a_prompt_batch(dev, monkeypatch):
-    """under the fast numerics policy fewer than 64 query rows take the tensor-core decode kernel (not the CPU's bits,
+    """under the fast numerics policy fewer than 64 query rows take a tensor-core kernel (not the CPU's bits,
     within the tolerance of f64); with that kernel switched off a single row takes the f32 CUDA-core kernel and several
     rows keep the exact kernels"""
     scale = 1.0 / np.sqrt(128.0)
@@ -154,7 +154,7 @@ def test_unsupported_variants_fall_back_to_the_exact_kernels(dev):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
-# ---- prompt batches: the tensor-core kernel (csrc/flash_attn_prefill.cu) ---------------------------------------------
+# ---- prompt batches: the tensor-core kernel (csrc/flash_attn_prompt.cu; its edges: test_gpu_flash_attn_prompt.py) ------
 PREFILL = [
     # (H, Hkv, D, T, n_kv, causal)
     (8, 2, 128, 64, 64, True),        # one tile, one row block per KV head
@@ -167,16 +167,9 @@ PREFILL = [
 ]
 
 
-@pytest.mark.parametrize("kernel", ["tcgen05", "mma.sync"])
 @pytest.mark.parametrize("shape", PREFILL, ids=str)
-def test_prompt_batches(dev, shape, kernel, monkeypatch):
-    """the mma.sync kernel is the default; head size 128 with two or more heads per KV head also has a tcgen05 kernel,
-    taken when B200_FA_PREFILL_TC=1 (read per call)"""
+def test_prompt_batches(dev, shape):
     H, Hkv, D, T, n_kv, causal = shape
-    if kernel == "tcgen05":
-        if D != 128 or H == Hkv:
-            pytest.skip("no tcgen05 form for this shape")
-        monkeypatch.setenv("B200_FA_PREFILL_TC", "1")
     q, k, v, mask = synth_case(H, Hkv, D, T, n_kv, seed=sum(shape[:5]), causal=causal)
     scale = 1.0 / np.sqrt(float(D))
     want = ref64(q, k, v, mask, scale)
@@ -184,7 +177,7 @@ def test_prompt_batches(dev, shape, kernel, monkeypatch):
     d_g64 = row_rel(got, want)
     # the same function with q rounded to f16 first, as the CPU path (and this kernel) rounds it: flash_attn.rs:433
     d_g64q = row_rel(got, ref64(q.astype(np.float16).astype(np.float32), k, v, mask, scale))
-    line = f"prompt {shape} {kernel}: GPU-f64 {d_g64:.2e}  GPU-f64(q16) {d_g64q:.2e}"
+    line = f"prompt {shape}: GPU-f64 {d_g64:.2e}  GPU-f64(q16) {d_g64q:.2e}"
     if T * n_kv * H <= 8 * 100 * 1000:   # the CPU restatement is a scalar loop: small cases only
         cpu, _ = orc.flash_attn(q, k, v, mask, scale)
         d_gc, d_c64 = row_rel(got, cpu), row_rel(cpu, want)
