@@ -129,8 +129,8 @@ __device__ __forceinline__ float2 pa_ld_peer2(uint32_t addr) {
 // ---- rows whose output is not finite ------------------------------------------------------------------------------
 // The products run over whole tiles, so what a cell holds that a row does not see meets that row with weight 0: 0 * Inf and NaN scores spoil it.  A
 // row that ends with anything but finite numbers is therefore computed once more, by a warp, from the cells it sees alone: nothing where all is
-// finite, and the definition's Inf and NaN where they belong.  (4096 positions take a row a quarter of a millisecond; a NaN score, as of a query with
-// a NaN, ends it at the first 32.)
+// finite, and the definition's Inf and NaN where they belong.  (4096 positions take a row about a millisecond; a NaN score, as of a query with a NaN, ends
+// it at the first 32: 512 rows of 32 heads over 4096 positions, one query a NaN, 76 us.)
 __device__ __forceinline__ bool pa_finite(float x) { return fabsf(x) < INFINITY; }
 template <bool BF16>
 __device__ __forceinline__ float2 pa_two(uint32_t w) {

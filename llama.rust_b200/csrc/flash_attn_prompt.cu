@@ -7,7 +7,7 @@
 //     so that every K / V tile and every mask row is shared by the group.  Row r is lane r of tensor memory.
 //   * K and V come in tiles of 128 positions by TMA (128-byte swizzle; positions past the cache read as zeros), K a K-major and V an
 //     MN-major B operand: a cached row's value elements are contiguous along N, so neither tile is transposed.
-//   * The tiles that are visited alternate between two groups of four softmax warps.  Each has its own scores (128 columns of
+//   * (As published with FlashAttention-4:) the tiles that are visited alternate between two groups of four softmax warps.  Each has its own scores (128 columns of
 //     tensor memory), its own unnormalised output and its own running maximum and sum, so that one group's exponentials hide the
 //     other's products; the two are added at the end.  A thread owns a whole row: no exchange between threads.
 //   * The weights go back into tensor memory over the scores they came from, as the A operand of p v: shared memory carries K, V and q only.
@@ -25,8 +25,8 @@
 //     partial outputs meet in shared memory and every CTA finishes its share of the rows.
 // Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device error word, and no row of its block is stored.
 // What bounds it (512 rows of 32 heads over 4096 positions, 8 KV heads of 128: 50 us; the mma.sync kernel in its place before took 169, 0.19 of
-// the rate the products alone would allow): a tile of 128 x 128 costs about 1850 SM clocks, 1024 of them exponentials (16 a clock) and as many
-// products, which two groups overlap only in part; and about 10 us of a launch are its beginning (q, the first tiles) and end.  On the way: one
+// the rate the products alone would allow): a tile of 128 x 128 costs about 2000 SM clocks, 1024 of them exponentials (16 a clock) and as many
+// products, which two groups overlap only in part (tensor pipe busy 30 % of the time, exponentials' pipe 35 %, issue slots 44 %); and about 10 us of a launch are its beginning (q, the first tiles) and end.  On the way: one
 // lane that walked the tiles and issued the products with its descriptors in ordinary registers 67.8 us; the warp together, one elected
 // lane issuing 57.9; two floats per instruction around the exponentials 53.4; one warp that sorts the tiles for everyone 50.7.
 // Not handled here (the caller falls back to the exact kernels): sinks, ALiBi, softcap, dk != dv.

@@ -105,7 +105,6 @@ __device__ __forceinline__ uint64_t few_add2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-__device__ __forceinline__ float few_or_zero(float x) { return fabsf(x) < INFINITY ? x : 0.0f; }
 // the integers 0 .. 63 in two bytes of x as f16
 __device__ __forceinline__ uint32_t few_byte_f16x2(uint32_t x, uint32_t selector) {
     const uint32_t h = __byte_perm(x, 0x64646464u, selector);   // 1024 + byte
@@ -339,7 +338,6 @@ struct FewChunk {
         const int lane = threadIdx.x & 31, g8 = lane >> 2, t = lane & 3;
         uint32_t mn[2][2][2];
         float dw[2][2], dm[2][2];
-        uint64_t dr2[2][2];   // Q6_K: for what rounding a product leaves out, which is added first (an infinite scale has none)
 #pragma unroll
         for (int mt = 0; mt < 2; mt++)
 #pragma unroll
@@ -354,14 +352,22 @@ struct FewChunk {
                     mn[mt][r][1] = few_byte_f16x2(((x.w >> 4) & 0x0f0f0f0fu) | (((x.z >> 6) & 0x03030303u) << 4), sel);
                 } else {
                     dw[mt][r] = f16_bits_to_f32(*(const uint16_t *)(w + 6656 + row * 2));
-                    dr2[mt][r] = few_pair(few_or_zero(dw[mt][r]), few_or_zero(dw[mt][r]));
                 }
             }
+        // Q6_K: what rounding a product leaves out is added first, where there is such a thing (asked for the warp: two selects a scale and activation
+        // row took a 128256 x 4096 head on 16 rows from 143 to 159 us)
+        bool finite = true;
+        if (TYPE == B200_TYPE_Q6_K) {
+            float far = fmaxf(fmaxf(fabsf(dw[0][0]), fabsf(dw[0][1])), fmaxf(fabsf(dw[1][0]), fabsf(dw[1][1])));
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) far = fmaxf(far, fabsf(dx[nt]));
+            finite = !__any_sync(0xffffffffu, far == INFINITY);
+        }
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) {
             if (GROUPED && nt >= nt_live) continue;
             const float d0 = __shfl_sync(0xffffffffu, dx[nt], 8 * t), d1 = __shfl_sync(0xffffffffu, dx[nt], 8 * t + 4);   // of columns 2 t and 2 t + 1
-            const uint64_t dx2 = few_pair(d0, d1), dxr2 = few_pair(few_or_zero(d0), few_or_zero(d1));
+            const uint64_t dx2 = few_pair(d0, d1);
             uint32_t b0 = 0, b1 = 0;
             if (TYPE == B200_TYPE_Q4_K) {
                 b0 = few_short_f16x2(bs[nt][0]);
@@ -377,7 +383,7 @@ struct FewChunk {
                     const uint64_t i2f = few_pair((float)i2[0], (float)i2[1]), d2 = few_pair(dw[mt][r], dw[mt][r]);
                     uint64_t v = few_mul2(i2f, d2);
                     if (TYPE == B200_TYPE_Q4_K) v = few_fma2(few_pair(mg[2 * r], mg[2 * r + 1]), few_pair(dm[mt][r], dm[mt][r]), v);
-                    else acc[mt][nt][r] = few_fma2(few_fma2(i2f, dr2[mt][r], few_mul2(i2f, dr2[mt][r]) ^ 0x8000000080000000ull), dxr2, acc[mt][nt][r]);
+                    else if (finite) acc[mt][nt][r] = few_fma2(few_fma2(i2f, d2, v ^ 0x8000000080000000ull), dx2, acc[mt][nt][r]);
                     acc[mt][nt][r] = few_fma2(v, dx2, acc[mt][nt][r]);
                 }
             }
@@ -629,21 +635,21 @@ void gemm_few_debug_wait(int spin_limit, int skip_unit) {
 }
 
 // Whether m activation rows are few, on a GPU of sms SMs.  us, weights from HBM, the others / this kernel:
-//   * Up to 31 rows: 14336 x 4096 on 8 and 16 rows Q4_K 25 / 13 and 27 / 18, Q6_K 24 / 17 and 28 / 25, Q8_0 24 / 14 and 25 / 17, Q4_0 23 / 13 and
-//     24 / 17, MXFP4 29 / 20 and 30 / 24; 4096 x 14336 Q8_0 67 / 14 and 70 / 17, on 2 and 4 rows 36 / 13 and 71 / 13.  But not Q6_K on 9 to 31 rows
+//   * Up to 31 rows: 14336 x 4096 on 8 and 16 rows Q4_K 25 / 13 and 26 / 18, Q6_K 24 / 17 and 28 / 26, Q8_0 26 / 16 and 28 / 23, Q4_0 25 / 13 and
+//     26 / 17, MXFP4 33 / 20 and 34 / 24; 4096 x 14336 Q8_0 73 / 18 and 75 / 22, on 4 rows 82 / 17.  But not Q6_K on 9 to 31 rows
 //     where the exact kernel (gemm_mma.cu) is as quick or quicker: up to 8 super-blocks (6144 x 2048 on 20 12.4 / 14.4, 14336 x 2048 20 / 23), and
 //     up to 16 of small matrices (4096 x 4096 on 12 9.9 / 10.9, 2048 x 4096 on 24 9.9 / 10.6, but 4096 x 4096 on 24 15.8 / 13.6; 14336 x 4096 25.8 / 25.4, on 16 27.5 / 25.4, 128256 x 4096 on 16
 //     158 / 145).  Otherwise one rule for every n: a matrix alone and one among its siblings take the same kernel.
-//   * K-quants up to 63 rows: 14336 x 4096 on 48 Q4_K 65 / 38, Q6_K 70 / 53, 1000 x 2048 on 32 29 / 8.
-//   * Above that by estimates, in microseconds, x = 10^6 weights, b = blocks of 16 rows: here 8 + c x b (instructions, 50 to 60 % of what a SM
-//     issues: the weights are unpacked again for every block; more with less than 8 super-blocks, where warps have none), against
+//   * K-quants up to 63 rows: 14336 x 4096 on 48 Q4_K 66 / 39, Q6_K 69 / 54, 1000 x 2048 on 32 29 / 8.
+//   * Above that by estimates, in microseconds, x = 10^6 weights, b = blocks of 16 rows: here 8 + c x b (instructions and waits for weights: a SM
+//     issues in 38 to 44 % of its slots on 16 rows, and the weights are unpacked again for every block; more with less than 8 super-blocks, where warps have none), against
 //       K-quants on the fast tcgen05 kernel (2048 weight rows and up, its rows in one block of 256): by its weights or, in few tiles, by its
 //       latency a super-block, whichever says less;
 //       K-quants of fewer weight rows, on the exact kernels: a latency a super-block too (one wave);
 //       the others on int8 tiles of 128 x 32: 5 + 1.5 a wave and super-block, MXFP4 1.9, where the f16 kernel is not the better one.
 //     The estimates are a little high for this kernel and low for the others: over 1190 products (n 512 to 32000, k 1024 to 14336, 32 to 512
 //     rows, the five types) one that is taken is more than 3 % slower (6144 x 2048 Q4_K on 112 rows 23.6 / 24.5).  4096 x 14336 on 32 rows: Q4_K
-//     113 / 24, Q6_K 143 / 35, Q8_0 91 / 24; 4096 x 4096 on 64: Q4_K 28 / 19, Q8_0 31 / 17; 1024 x 4096 Q6_K on 512 55 / 43.
+//     118 / 24, Q6_K 189 / 35, Q8_0 95 / 28; 4096 x 4096 on 64: Q4_K 29 / 18, Q8_0 32 / 19; 1024 x 4096 Q6_K on 512 55 / 43.
 bool few_takes_for(int type, int route, int64_t n, int64_t k, int64_t m, int sms) {
     if (m < 2 || n <= 0 || m * (k / GROUP_K) >= FEW_ACT_GROUPS) return false;   // 32-bit byte offsets into the activations
     const bool q6 = type == B200_TYPE_Q6_K, kq = type == B200_TYPE_Q4_K || q6;
