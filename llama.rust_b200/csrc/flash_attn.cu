@@ -668,24 +668,31 @@ extern "C" int b200_flash_attn_ext(const struct b200_flash_attn_args *args, void
     // than it (measured on 16 sequences over 10240 cells).
     const bool policy = args->mode == 0 && numerics_mode() == 1;
     if ((args->mode == 1 || policy) && args->n_tok < 64) {
-        // What the decode kernel does not take (heads in groups that do not divide 16, mask rows off 4 bytes) keeps the kernels below, which read
-        // q and the weights in F32, or as the CPU does, and no position that a row does not see.
         if (fa_decode_mma_enabled() && flash_attn_decode_mma_takes(args)) {
-            // The prompt kernel computes 128 rows at a time with its positions over a cluster, the decode kernel 16 rows (whole tokens) that skip what
-            // none of them sees; the host does not know whether the rows are a prompt's or sequences', each with a stretch of its own.  Measured on
-            // both, on rows of unequal stretches and on alternating cells, in ten groupings of heads; us, decode / prompt kernel, 32 heads of 128 on
-            // 8 KV heads, 16 rows: 512 positions 15.3 / 11.6 (sequences 14.6 / 11.7), 2048 20.5 / 13.2 (17.7 / 13.2), 4096 25 / 16 (20 / 16).
-            //   * Fewer than 12 rows leave most of the 128 empty (32 heads on 32, 8 rows over 4096: 26 / 29 where one row has most cells).
-            //   * Small launches lose to the cluster's beginning and end: 8 heads on 2, 16 rows over 512 positions 10.6 / 11.7, 48 over 256 11.2 / 16.
-            //   * Above 4096 positions sequences are the decode kernel's, which walks each one's tiles alone: 32 of them over 8192 20 / 23, over
-            //     32768 50 / 69 (16 heads on 4: 29 / 67), although a prompt's rows would be quicker here (56 / 23, 180 / 56).  With about 2000
-            //     (row, head) pairs either is quicker here: 63 rows of 32 heads over 8192 21 / 21 (95 / 27), over 32768 65 / 57 (342 / 71).
-            //   * With heads of 64 the decode kernel has half as much to do and this one the same exponentials: 8 heads on 1, 24 rows over 512
-            //     positions 8.6 / 11.2, 48 sequences over 1536 with 8 heads on 2 10.6 / 11.7, 63 over 4096 on one key head 18 / 21.
-            const int64_t pairs = args->n_tok * args->n_head;
-            const bool wide = args->dk == 128 && args->n_tok >= 12 && args->n_kv >= 512 && (args->n_kv <= 4096 ? pairs * args->n_kv >= 12 * 8 * 1024 : pairs >= 2000);
+            // Two to 63 rows.  The prompt kernel computes 128 (row, head) pairs of a key head at a time with its positions over a cluster, the decode kernel
+            // 16 of whole tokens that skip what none of them sees; the host does not know whether the rows are a prompt's or sequences', each with a
+            // stretch of its own.  Measured: 2 to 63 rows, ten groupings of heads, 256 to 32768 positions, causal masks, equal and unequal
+            // stretches, alternating cells.  us, decode / prompt kernel, 32 heads of 128 on 8, 16 rows of a prompt (sequences): 512 positions 15.3 / 11.6
+            // (14.6 / 11.7), 2048 20.5 / 13.2 (17.7 / 13.2), 4096 25 / 16 (20 / 16), 8192 36 / 22 (20 / 22).
+            //   * Up to 4096 positions the prompt kernel, but for small launches, which lose to the cluster's beginning and end (8 heads on 2, 16
+            //     rows over 512 10.6 / 11.7; 8 on 4, 4 over 1024 9.2 / 10.2; 4 on 4, 2 over 2048 equal): pairs times positions squared says which.  And but
+            //     for few pairs of many key heads (32 on 32, 8 rows over 4096 26 / 29): a key head's 128 stand mostly empty.
+            //   * Up to 8192 where each key head has 12 pairs: a prompt's rows win by half to two thirds, equal sequences lose by up to a fifth (63 of 8 heads
+            //     on 4 20 / 24; with heads of 64, which the decode kernel has half as much to do with, 16 / 23).
+            //   * Above, what each loses on the other's kernel decides: 48 rows over 32768, 32 heads on 8, a prompt 259 / 69, sequences 56 / 67; 8 on 2 74 / 52
+            //     and 25 / 47.
+            const int64_t pairs = args->n_tok * args->n_head, n = args->n_kv;
+            const bool filled = pairs >= 12 * args->n_head_kv;
+            const bool wide = args->n_tok > 1 && (n <= 8192 ? n >= (args->dk == 128 ? 512 : 1024) && pairs * n * n >= (args->dk == 128 ? 48ll << 20 : 96ll << 20) &&
+                                                                  (filled || (n <= 4096 && args->n_head_kv <= 8 && args->dk == 128))
+                                                            : args->n_tok >= 32 && pairs >= 640);
             if (wide && flash_attn_fast_prompt(args, (cudaStream_t)stream, &rc)) return rc;
             if (flash_attn_decode_mma(args, (cudaStream_t)stream, &rc)) return rc;
+        } else if (fa_decode_mma_enabled() && policy && args->n_tok > 1) {
+            // What the decode kernel does not take (heads in groups that do not divide 16, mask rows off 4 bytes): under the policy the prompt kernel,
+            // whose alternative has the CPU's f16 sums (16 rows over 1023 positions 164 us and 4e-3 from float64, 13 us and 1e-6 here); a call that
+            // asks for mode 1 has the kernel below, with q and the weights in F32
+            if (flash_attn_fast_prompt(args, (cudaStream_t)stream, &rc)) return rc;
         }
         if ((args->mode == 1 || args->n_tok == 1) && flash_attn_fast_rows(args, (cudaStream_t)stream, &rc)) return rc;
     }

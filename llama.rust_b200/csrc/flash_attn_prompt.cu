@@ -695,7 +695,7 @@ void attn_wait_hook(uint32_t *limit, int *mute) {
 // true: the fast prompt kernel took the call (*rc is its status); false: not a shape it handles.  Which of 2 to 63 rows come here: flash_attn.cu
 bool flash_attn_fast_prompt(const b200_flash_attn_args *a, cudaStream_t s, int *rc) {
     *rc = B200_STATUS_SUCCESS;
-    if (a->sinks || a->max_bias != 0.0f || a->logit_softcap != 0.0f || a->dk != a->dv || (a->dk != 64 && a->dk != 128) || a->n_kv == 0 || a->n_tok == 0 || (a->dk == 64 && a->n_tok < 64))
+    if (a->sinks || a->max_bias != 0.0f || a->logit_softcap != 0.0f || a->dk != a->dv || (a->dk != 64 && a->dk != 128) || a->n_kv == 0 || a->n_tok == 0)
         return false;
     if (a->q_nb1 % 8 || a->q_nb2 % 8 || ((uintptr_t)a->q & 7) || ((uintptr_t)a->dst & 7) || a->n_head % a->n_head_kv) return false;
     if (a->k_nb1 % 16 || a->v_nb1 % 16 || a->k_nb2 % 16 || a->v_nb2 % 16 || ((uintptr_t)a->k & 15) || ((uintptr_t)a->v & 15)) return false;
@@ -737,10 +737,9 @@ bool flash_attn_fast_prompt(const b200_flash_attn_args *a, cudaStream_t s, int *
     // a row's maximum is taken before the scale, which must then not be negative: its sign goes to q
     p.scale_log2 = fabsf(a->scale) * PA_LOG2E;
     p.q_sign = a->scale < 0.0f ? -1.0f : 1.0f;
-    // two-part weights where the decode kernel's are the measure (the caller sends it heads of 128 only with fewer than 64 rows)
-    if (D == 64) *rc = launch<64, false>(km, vm, p, blocks, a->n_head_kv, dev, s);
-    else if (a->n_tok < 64) *rc = launch<128, true>(km, vm, p, blocks, a->n_head_kv, dev, s);
-    else *rc = launch<128, false>(km, vm, p, blocks, a->n_head_kv, dev, s);
+    // two-part weights where the decode kernel's are the measure
+    if (a->n_tok < 64) *rc = D == 128 ? launch<128, true>(km, vm, p, blocks, a->n_head_kv, dev, s) : launch<64, true>(km, vm, p, blocks, a->n_head_kv, dev, s);
+    else *rc = D == 128 ? launch<128, false>(km, vm, p, blocks, a->n_head_kv, dev, s) : launch<64, false>(km, vm, p, blocks, a->n_head_kv, dev, s);
     return true;
 }
 
