@@ -637,9 +637,9 @@ void gemm_few_debug_wait(int spin_limit, int skip_unit) {
 // Whether m activation rows are few, on a GPU of sms SMs.  us, weights from HBM, the others / this kernel:
 //   * Up to 31 rows: 14336 x 4096 on 8 and 16 rows Q4_K 25 / 13 and 26 / 18, Q6_K 24 / 17 and 28 / 26, Q8_0 26 / 16 and 28 / 23, Q4_0 25 / 13 and
 //     26 / 17, MXFP4 33 / 20 and 34 / 24; 4096 x 14336 Q8_0 73 / 18 and 75 / 22, on 4 rows 82 / 17.  But not Q6_K on 9 to 31 rows
-//     where the exact kernel (gemm_mma.cu) is as quick or quicker: up to 8 super-blocks (6144 x 2048 on 20 12.4 / 14.4, 14336 x 2048 20 / 23), and
-//     up to 16 of small matrices (4096 x 4096 on 12 9.9 / 10.9, 2048 x 4096 on 24 9.9 / 10.6, but 4096 x 4096 on 24 15.8 / 13.6; 14336 x 4096 25.8 / 25.4, on 16 27.5 / 25.4, 128256 x 4096 on 16
-//     158 / 145).  Otherwise one rule for every n: a matrix alone and one among its siblings take the same kernel.
+//     of up to 8 super-blocks, where the exact kernel (gemm_mma.cu) is as quick or quicker: 6144 x 2048 on 20 12.4 / 14.4, 14336 x 2048 20 / 23.  (Of 16
+//     it is a tenth quicker in small matrices, 4096 x 4096 on 12 rows 9.9 / 10.9, and slower in large ones, 128256 x 4096 on 16 158 / 145; 7.8e-8
+//     from float64, 6.1e-8 here.)  One rule for every n: a matrix alone and one among its siblings take the same kernel.
 //   * K-quants up to 63 rows: 14336 x 4096 on 48 Q4_K 66 / 39, Q6_K 69 / 54, 1000 x 2048 on 32 29 / 8.
 //   * Above that by estimates, in microseconds, x = 10^6 weights, b = blocks of 16 rows: here 8 + c x b (instructions and waits for weights: a SM
 //     issues in 38 to 44 % of its slots on 16 rows, and the weights are unpacked again for every block; more with less than 8 super-blocks, where warps have none), against
@@ -667,7 +667,7 @@ bool few_takes_for(int type, int route, int64_t n, int64_t k, int64_t m, int sms
             break;
         default: return false;
     }
-    if (q6 && route == B200_ROUTE_TILED && m > 8 && m < 32 && (k <= 8 * GROUP_K || (k <= 16 * GROUP_K && n < (m <= 16 ? 14336 : 4096)))) return false;
+    if (q6 && route == B200_ROUTE_TILED && m > 8 && m < 32 && k <= 8 * GROUP_K) return false;
     if (m < 32 || (kq && m < GEMM_FAST_MIN_COLS)) return true;
     if (m > (kq && n >= 2048 ? 256 : 512)) return false;
     const double x = (double)n * (double)k * 1e-6 * 148 / sms, nb = (double)(k / GROUP_K), blocks = (double)((m + 15) / 16);   // per SM as on 148

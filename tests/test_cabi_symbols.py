@@ -163,9 +163,8 @@ def test_few_rows_kernel_choice():
         assert f(ty, 14336, 14336, 16, 148) == 1 and f(ty, 14336, 4096, 513, 148) == 0
         assert f(ty, 8, (1 << 24) // 16 * 256, 16, 148) == 0 and f(ty, 8, (1 << 24) // 16 * 256 - 256, 16, 148) == 1
         assert f(ty, 4096, 4096, 16, 0) == -1 and f(ty, 4096, 100, 16, 148) == -1
-    # the exact kernel's: Q6_K, 9 to 31 rows of up to 8 super-blocks, up to 16 in small matrices
+    # the exact kernel's: Q6_K, 9 to 31 rows of up to 8 super-blocks
     assert [f(mod.Q6_K, 6144, k, m, 148) for k, m in ((2048, 8), (2048, 9), (2048, 31), (2304, 31), (2048, 32))] == [1, 0, 0, 1, 1]
-    assert [f(mod.Q6_K, n, k, m, 148) for n, k, m in ((4096, 4096, 16), (14336, 4096, 16), (2048, 4096, 17), (4096, 4096, 17), (4096, 4352, 16))] == [0, 1, 0, 1, 1]
     # the tcgen05 kernels': K-quants of short rows, batches past its block of 256 rows
     assert [f(mod.Q6_K, 6144, 2048, m, 148) for m in (64, 80, 112)] == [1, 1, 0]
     assert [f(mod.Q4_K, 8192, 2048, m, 148) for m in (64, 80, 112)] == [1, 1, 0]
